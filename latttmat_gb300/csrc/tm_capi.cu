@@ -124,6 +124,7 @@ template <class T>
 double matvec_bfly(const Op& op, const T* x, T* y, bool scaled, cudaStream_t s);
 template <class T>
 void matvec_eo(const Op& op, const T* x, T* y, bool scaled32, cudaStream_t s);
+void matvec_eo_ref(const Op& op, const void* x, void* y, tm_dtype dt, cudaStream_t s);
 double eo_scale32(const Op& op);
 template <class T>
 double matvec_aux(const Op& op, const T* x, T* y, bool scaled, cudaStream_t s);
@@ -217,15 +218,10 @@ void matvec_ref_order(const Op& op, const void* x, void* y, tm_dtype dt, cudaStr
     if (dt != TM_F64) fail(TM_ERR_UNSUPPORTED, "two-layer operators run in FP64 only");
     matvec_two_layer(op, (const double*)x, (double*)y, s);
   } else if (dt == TM_F64_DF && !base.has_pi) {
-    if (base.eo.active)
-      matvec_eo_df(base, (const double*)x, (double*)y, s);
-    else
-      matvec_aux_df(op, (const double*)x, (double*)y, s);
+    matvec_aux_df(op, (const double*)x, (double*)y, s);
   } else if (!base.has_pi) {
     if (dt == TM_F64) {
-      if (base.eo.active) {
-        matvec_eo<double>(base, (const double*)x, (double*)y, false, s);
-      } else if (bfly_core(base.kind)) {
+      if (bfly_core(base.kind)) {
         matvec_bfly<double>(base, (const double*)x, (double*)y, false, s);
       } else {
         matvec_aux<double>(op, (const double*)x, (double*)y, false, s);
@@ -237,19 +233,7 @@ void matvec_ref_order(const Op& op, const void* x, void* y, tm_dtype dt, cudaStr
         matvec_aux<float>(op, (const float*)x, (float*)y, false, s);
     }
   } else {
-    const uint32_t* pi = base.pi.as<uint32_t>();
-    if (dt != TM_F32) {
-      gather_f64((const double*)x, pi, base.xp.as<double>(), n, s);
-      if (dt == TM_F64_DF)
-        matvec_eo_df(base, base.xp.as<double>(), base.yp.as<double>(), s);
-      else
-        matvec_eo<double>(base, base.xp.as<double>(), base.yp.as<double>(), false, s);
-      scatter_f64(base.yp.as<double>(), pi, (double*)y, n, s);
-    } else {
-      gather_f32((const float*)x, pi, base.xp.as<float>(), n, s);
-      matvec_eo<float>(base, base.xp.as<float>(), base.yp.as<float>(), false, s);
-      scatter_f32(base.yp.as<float>(), pi, (float*)y, n, s);
-    }
+    matvec_eo_ref(base, x, y, dt, s);
   }
   const_cast<Op&>(op).matvecs++;
 }
@@ -342,7 +326,6 @@ static void build_op(Op& op) {
       op.eo.w1_32.alloc(((size_t)op.eo.n_orep << op.eo.m) * 4);
       op.eo.w1_64.alloc(((size_t)op.eo.n_orep << op.eo.m) * 8);
       if (const size_t xb = eo_xchg_bytes(op.eo)) op.eo.xchg.alloc(xb);
-      op.xp.alloc((size_t)op.n * 8);
       op.yp.alloc((size_t)op.n * 8);
     } else {
       if (op.L > 30) fail(TM_ERR_LIMIT, "generic reduced path supports L <= 30");

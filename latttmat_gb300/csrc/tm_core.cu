@@ -232,13 +232,4 @@ void scatter_f64(const double* src, const uint32_t* idx, double* dst, int64_t n,
   scatter_kernel<double><<<grid_for(n), 256, 0, s>>>(src, idx, dst, n);
   TM_CKK("scatter");
 }
-void gather_f32(const float* src, const uint32_t* idx, float* dst, int64_t n, cudaStream_t s) {
-  gather_kernel<float><<<grid_for(n), 256, 0, s>>>(src, idx, dst, n);
-  TM_CKK("gather");
-}
-void scatter_f32(const float* src, const uint32_t* idx, float* dst, int64_t n, cudaStream_t s) {
-  scatter_kernel<float><<<grid_for(n), 256, 0, s>>>(src, idx, dst, n);
-  TM_CKK("scatter");
-}
-
 }  // namespace ltm

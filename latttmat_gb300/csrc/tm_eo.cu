@@ -627,8 +627,33 @@ __global__ void __launch_bounds__(1024, 1) eo_pass1(EOArgs A, const InT* __restr
 }
 
 // Output modes of pass 2: y = val * sout32 (FP32), val * sout64 * post
-// (FP64), or val * soutdf in double-float (double-float storage).
-enum { kOutF32 = 0, kOutF64 = 1, kOutDF = 2 };
+// (FP64), val * soutdf in double-float (double-float storage), or an FP32
+// val * soutdf * post formed in double-float and rounded once (kOutF32S).
+enum { kOutF32 = 0, kOutF64 = 1, kOutDF = 2, kOutF32S = 3 };
+
+// Output factor of kOutF32S: two * hl, two a power of two near its square
+// root, so that the partial products stay near the result's exponent range.
+struct EoPost {
+  double f64;
+  float two;
+  dfloat hl;
+};
+
+// (v * sc) * post rounded to FP32 once: the products' rounding errors are
+// carried along (TwoProduct by FMA), so the result is the FP64 path's to
+// within the last rounding.  Two FP64 multiplies and three conversions per
+// output took 0.44 ms of pass 2's 1.22 ms at L = 32 (two FP64 lanes per
+// clock and SM); this takes 0.79 ms in all.
+__device__ __forceinline__ float scale_round(float v, dfloat sc, const EoPost& post) {
+  const float a = v * post.two;  // exact
+  const float p = a * sc.hi;
+  // zeros, infinities, NaN and products near the ends of the exponent range
+  // (where the error terms would be lost) take the FP64 form
+  if (!(fabsf(p) > 1e-24f && fabsf(p) < 1e24f)) return (float)((double)v * (double)sc * post.f64);
+  const float e = fmaf(a, sc.lo, fmaf(a, sc.hi, -p));
+  const float q = p * post.hl.hi;
+  return q + fmaf(e, post.hl.hi, fmaf(p, post.hl.lo, fmaf(p, post.hl.hi, -q)));
+}
 
 // pass 2: z[(e_rep, o)] = (Th_O w)[(e_rep, o)]; emit designated outputs.
 // The w value at (e_rep, o) is the pass-1 value at the H-image
@@ -646,7 +671,7 @@ __global__ void __launch_bounds__(1024, 1) eo_pass2(EOArgs A, const T* __restric
                                                     const uint16_t* __restrict__ out_o,
                                                     const double* __restrict__ sout64,
                                                     const float* __restrict__ sout32,
-                                                    const dfloat* __restrict__ soutdf, double post,
+                                                    const dfloat* __restrict__ soutdf, EoPost post,
                                                     OutT* __restrict__ y, float4* __restrict__ xchg) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* sm = reinterpret_cast<T*>(smem_raw);
@@ -696,9 +721,10 @@ __global__ void __launch_bounds__(1024, 1) eo_pass2(EOArgs A, const T* __restric
   const uint32_t k0 = out_off[g0], k1 = out_off[g0 + (1 << (A.ct - A.c))];
   // the output scales are loaded with the o indices, a batch at a time, so
   // their loads are in flight together
-  using Scale = typename std::conditional<OSC == kOutDF, dfloat, typename std::conditional<OSC == kOutF64, double, float>::type>::type;
+  constexpr bool kScaleDF = (OSC == kOutDF || OSC == kOutF32S);
+  using Scale = typename std::conditional<kScaleDF, dfloat, typename std::conditional<OSC == kOutF64, double, float>::type>::type;
   const Scale* __restrict__ scale = [&] {
-    if constexpr (OSC == kOutDF) return soutdf;
+    if constexpr (kScaleDF) return soutdf;
     else if constexpr (OSC == kOutF64) return sout64;
     else return sout32;
   }();
@@ -721,8 +747,10 @@ __global__ void __launch_bounds__(1024, 1) eo_pass2(EOArgs A, const T* __restric
         const T val = sm[spad(ov[q] & lmask)];
         if constexpr (OSC == kOutDF)
           y[k] = val * sc[q];
+        else if constexpr (OSC == kOutF32S)
+          y[k] = scale_round(val, sc[q], post);
         else if constexpr (OSC == kOutF64)
-          y[k] = (OutT)((double)val * sc[q] * post);
+          y[k] = (OutT)((double)val * sc[q] * post.f64);
         else
           y[k] = (OutT)(val * T(sc[q]));
       }
@@ -1203,6 +1231,8 @@ void build_eo_plan(Op& op, const EOHostTables* Hp) {
 }
 
 // ------------------------------------------------------------------ launch
+double eo_scale32(const Op& op);
+
 namespace {
 
 // u = x * sin * gin.  gin = (1 + r)^-L keeps the magnitudes of the
@@ -1219,6 +1249,85 @@ __global__ void eo_scale_in(const T* __restrict__ x, const double* __restrict__ 
     else
       u[i] = x[i] * ((T)s32[i] * gin32);
   }
+}
+
+// The same from a vector in the reference's order: u[k] = x[pi[k]] * sin[k] *
+// gin, the permutation and the scaling in one pass, four gathers in flight per
+// thread.  Bound by the gathers (one 32-byte sector of x each).  At L = 32 in
+// FP32 (67 M rows) separate gather and scaling kernels took 0.61 ms.
+template <class T>
+__global__ void __launch_bounds__(256) eo_gather_scale(const T* __restrict__ x, const uint32_t* __restrict__ pi,
+                                                       const double* __restrict__ s64,
+                                                       const float* __restrict__ s32, T* __restrict__ u, int64_t n,
+                                                       double gin) {
+  const float gin32 = (float)gin;
+  for (int64_t i0 = ((int64_t)blockIdx.x * 256) * 4 + threadIdx.x; i0 < n; i0 += (int64_t)gridDim.x * 1024) {
+    uint32_t at[4];
+    T v[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (i0 + q * 256 < n) at[q] = __ldcs(pi + i0 + q * 256);
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (i0 + q * 256 < n) v[q] = __ldg(x + at[q]);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int64_t i = i0 + q * 256;
+      if (i < n) {
+        if constexpr (sizeof(T) == 8)
+          u[i] = (T)((double)v[q] * __ldcs(s64 + i) * gin);
+        else
+          u[i] = v[q] * ((T)__ldcs(s32 + i) * gin32);
+      }
+    }
+  }
+}
+
+// y[i] = yp[pinv[i]]: the way back to the reference's order, by a gather.
+// The scatter y[pi[k]] = yp[k] writes partial sectors, 1.35 ms at L = 32 in
+// FP32 against 0.49 ms for the opposite gather.
+template <class T>
+__global__ void __launch_bounds__(256) eo_gather_out(const T* __restrict__ yp, const uint32_t* __restrict__ pinv,
+                                                     T* __restrict__ y, int64_t n) {
+  for (int64_t i0 = ((int64_t)blockIdx.x * 256) * 4 + threadIdx.x; i0 < n; i0 += (int64_t)gridDim.x * 1024) {
+    uint32_t at[4];
+    T v[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (i0 + q * 256 < n) at[q] = __ldcs(pinv + i0 + q * 256);
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (i0 + q * 256 < n) v[q] = __ldg(yp + at[q]);
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (i0 + q * 256 < n) __stcs(y + i0 + q * 256, v[q]);
+  }
+}
+
+// blocks for the four-per-thread gathers
+int grid_gather(int64_t n) {
+  return (int)std::max<int64_t>(1, std::min<int64_t>((n + 1023) / 1024, (int64_t)num_sms() * 32));
+}
+
+// Whether kOutF32S may stand in for the FP64 output scaling: the scales
+// dup * Tvec and (e^K + e^-K)^L have to stay well inside the FP32 exponent
+// range (e^60 of e^87), from the largest exponent genTvec can reach.
+bool eo_scale_fits32(const Op& op) {
+  const double hb = 0.5 * std::fabs(op.mp.betaJ);
+  const double bz = hb * (op.L * (1.0 + std::fabs(op.mp.kappa) + std::fabs(op.mp.h)) + std::fabs(op.nfexp));
+  const double lnS = op.L * std::log(std::exp(op.mp.betaJ) + std::exp(-op.mp.betaJ));
+  return bz < 60.0 && lnS < 60.0;
+}
+
+EoPost eo_post(double S) {
+  EoPost p{S, 1.f, dfloat(1.0)};
+  int e = 0;
+  std::frexp(S, &e);
+  if (std::isfinite(S) && S > 0 && e < 120) {
+    p.two = std::ldexp(1.f, e / 2);
+    p.hl = dfloat(S / (double)p.two);
+  }
+  return p;
 }
 
 // input factor of the unnormalised butterflies: (1 + r)^-L, r = e^-2|K|
@@ -1277,7 +1386,7 @@ void launch_pass1(const EOArgs& A, int ntiles, const typename EoIO<T>::In* u, co
 
 template <class T, int KB, int OSC, class OutT = typename EoIO<T>::Out>
 void launch_pass2(const EOArgs& A, int ntiles, const T* w1, const EOPlan& P, const double* sout64,
-                  const float* sout32, const dfloat* soutdf, double post, OutT* y, cudaStream_t s) {
+                  const float* sout32, const dfloat* soutdf, EoPost post, OutT* y, cudaStream_t s) {
   size_t shm = (size_t)((1 << A.n) + (1 << A.n) / 32 + 1) * sizeof(T);
   auto kfn = (A.c > 0) ? eo_pass2<T, KB, OSC, OutT, true> : eo_pass2<T, KB, OSC, OutT, false>;
   raise_smem_limit((const void*)kfn, shm);
@@ -1320,47 +1429,64 @@ EOArgs make_args(const Op& op, int c) {
   return A;
 }
 
+// ref: x and y in the reference's order (the pi-ordered result passes through yp)
 template <class T, int KB>
 void eo_dispatch(const Op& op, const EOArgs& A, const typename EoIO<T>::In* x, typename EoIO<T>::Out* y,
-                 bool scaled32, cudaStream_t s) {
+                 bool scaled32, bool ref, cudaStream_t s) {
   using In = typename EoIO<T>::In;
   const EOPlan& P = op.eo;
   const int64_t R = op.n;
   In* u = static_cast<In*>(op.ws_c.p);
   T* w1 = (sizeof(T) == 8) ? static_cast<T*>(P.w1_64.p) : static_cast<T*>(P.w1_32.p);
   if (P.prof_on) TM_CK(cudaEventRecord(P.prof_ev[0], s));
-  eo_scale_in<In><<<grid_for(R), 256, 0, s>>>(x, op.sin64.as<double>(), op.sin32.as<float>(), u, R,
-                                               eo_gin(op));
+  if (ref)
+    eo_gather_scale<In><<<grid_gather(R), 256, 0, s>>>(x, op.pi.as<uint32_t>(), op.sin64.as<double>(),
+                                                       op.sin32.as<float>(), u, R, eo_gin(op));
+  else
+    eo_scale_in<In><<<grid_for(R), 256, 0, s>>>(x, op.sin64.as<double>(), op.sin32.as<float>(), u, R,
+                                                 eo_gin(op));
   TM_CKK("eo_scale_in");
   if (P.prof_on) TM_CK(cudaEventRecord(P.prof_ev[1], s));
   launch_pass1<T, KB>(A, P.n_orep, u, P, w1, s);
   TM_CKK("eo_pass1");
   if (P.prof_on) TM_CK(cudaEventRecord(P.prof_ev[2], s));
-  const double S = std::pow(std::exp(op.mp.betaJ) + std::exp(-op.mp.betaJ), (double)op.L);
-  if (scaled32)
-    launch_pass2<T, KB, kOutF32>(A, P.n_erep, w1, P, op.sout64.as<double>(), op.sout32.as<float>(), nullptr, 1.0,
-                                 y, s);
-  else
-    launch_pass2<T, KB, kOutF64>(A, P.n_erep, w1, P, op.sout64.as<double>(), op.sout32.as<float>(), nullptr, S, y,
-                                 s);
+  const EoPost post = eo_post(scaled32 ? 1.0 : eo_scale32(op));
+  using Out = typename EoIO<T>::Out;
+  Out* yo = ref ? op.yp.as<Out>() : y;
+  const double* so64 = op.sout64.as<double>();
+  const float* so32 = op.sout32.as<float>();
+  if (scaled32) {
+    launch_pass2<T, KB, kOutF32>(A, P.n_erep, w1, P, so64, so32, nullptr, post, yo, s);
+  } else {
+    bool f32s = false;
+    if constexpr (std::is_same<T, float>::value) {
+      f32s = eo_scale_fits32(op);
+      if (f32s) launch_pass2<T, KB, kOutF32S>(A, P.n_erep, w1, P, so64, so32, op.soutdf.as<dfloat>(), post, yo, s);
+    }
+    if (!f32s) launch_pass2<T, KB, kOutF64>(A, P.n_erep, w1, P, so64, so32, nullptr, post, yo, s);
+  }
   TM_CKK("eo_pass2");
   if (P.prof_on) TM_CK(cudaEventRecord(P.prof_ev[3], s));
+  if (ref) {
+    eo_gather_out<Out><<<grid_gather(R), 256, 0, s>>>(yo, op.pinv.as<uint32_t>(), y, R);
+    TM_CKK("eo_gather_out");
+  }
 }
 
 template <class T>
 void matvec_eo_engine(const Op& op, const typename EoIO<T>::In* x, typename EoIO<T>::Out* y, bool scaled32,
-                      cudaStream_t s) {
+                      bool ref, cudaStream_t s) {
   const int c = (sizeof(T) == 8) ? op.eo.c64 : op.eo.c32;
   EOArgs A = make_args<T>(op, c);
   int kb = A.n - A.p;
   switch (kb) {
-    case 1: eo_dispatch<T, 1>(op, A, x, y, scaled32, s); break;
-    case 2: eo_dispatch<T, 2>(op, A, x, y, scaled32, s); break;
-    case 3: eo_dispatch<T, 3>(op, A, x, y, scaled32, s); break;
-    case 4: eo_dispatch<T, 4>(op, A, x, y, scaled32, s); break;
+    case 1: eo_dispatch<T, 1>(op, A, x, y, scaled32, ref, s); break;
+    case 2: eo_dispatch<T, 2>(op, A, x, y, scaled32, ref, s); break;
+    case 3: eo_dispatch<T, 3>(op, A, x, y, scaled32, ref, s); break;
+    case 4: eo_dispatch<T, 4>(op, A, x, y, scaled32, ref, s); break;
     default:
       if constexpr (sizeof(T) == 4)
-        eo_dispatch<T, 5>(op, A, x, y, scaled32, s);
+        eo_dispatch<T, 5>(op, A, x, y, scaled32, ref, s);
       else
         fail(TM_ERR_LIMIT, "even/odd tile too large for the 8-byte engines");
       break;
@@ -1373,7 +1499,7 @@ void matvec_eo_engine(const Op& op, const typename EoIO<T>::In* x, typename EoIO
 // solver applies that factor in FP64).
 template <class T>
 void matvec_eo(const Op& op, const T* x, T* y, bool scaled32, cudaStream_t s) {
-  matvec_eo_engine<T>(op, x, y, scaled32, s);
+  matvec_eo_engine<T>(op, x, y, scaled32, false, s);
 }
 
 template void matvec_eo<float>(const Op&, const float*, float*, bool, cudaStream_t);
@@ -1381,7 +1507,18 @@ template void matvec_eo<double>(const Op&, const double*, double*, bool, cudaStr
 
 // FP64 in/out, double-float arithmetic (the solver's refinement products)
 void matvec_eo_df(const Op& op, const double* x, double* y, cudaStream_t s) {
-  matvec_eo_engine<dfloat>(op, x, y, false, s);
+  matvec_eo_engine<dfloat>(op, x, y, false, false, s);
+}
+
+// The three engines on vectors in the reference's order.  x is read by the
+// first kernel and y written by the last, so y may be x.
+void matvec_eo_ref(const Op& op, const void* x, void* y, tm_dtype dt, cudaStream_t s) {
+  if (dt == TM_F32)
+    matvec_eo_engine<float>(op, (const float*)x, (float*)y, false, true, s);
+  else if (dt == TM_F64_DF)
+    matvec_eo_engine<dfloat>(op, (const double*)x, (double*)y, false, true, s);
+  else
+    matvec_eo_engine<double>(op, (const double*)x, (double*)y, false, true, s);
 }
 
 namespace {
@@ -1418,7 +1555,7 @@ void eo_dispatch_dd(const Op& op, const EOArgs& A, const dfloat* x, dfloat* y, c
                            P.wout.as<uint2>(), w1, eo_xchg<dfloat>(A, P, P.n_orep)));
   TM_CKK("eo_pass1_dd");
   launch_pass2<dfloat, KB, kOutDF, dfloat>(A, P.n_erep, w1, P, op.sout64.as<double>(), op.sout32.as<float>(),
-                                           op.soutdf.as<dfloat>(), 1.0, y, s);
+                                           op.soutdf.as<dfloat>(), eo_post(1.0), y, s);
   TM_CKK("eo_pass2_dd");
 }
 }  // namespace
@@ -1447,14 +1584,14 @@ void matvec_eo_f64_into(const Op& op, const double* x, double* y, double* u, dou
   eo_scale_in<double><<<grid_for(R), 256, 0, s>>>(x, op.sin64.as<double>(), op.sin32.as<float>(), u, R,
                                                    eo_gin(op));
   TM_CKK("eo_scale_in");
-  const double S = std::pow(std::exp(op.mp.betaJ) + std::exp(-op.mp.betaJ), (double)op.L);
+  const EoPost post = eo_post(eo_scale32(op));
   switch (A.n - A.p) {
 #define TM_EO_INTO(KBV)                                                                                      \
   case KBV:                                                                                                  \
     launch_pass1<double, KBV>(A, P.n_orep, u, P, w1, s);                                                     \
     TM_CKK("eo_pass1");                                                                                      \
     launch_pass2<double, KBV, kOutF64>(A, P.n_erep, w1, P, op.sout64.as<double>(), op.sout32.as<float>(),   \
-                                       nullptr, S, y, s);                                                    \
+                                       nullptr, post, y, s);                                                 \
     TM_CKK("eo_pass2");                                                                                      \
     break;
     TM_EO_INTO(1)

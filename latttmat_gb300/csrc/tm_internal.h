@@ -152,7 +152,8 @@ struct Op {
   // workspace
   DBuf ws_a, ws_b, ws_c;  // full-space scratch
   DBuf hx, hy;            // device copies for host-vector matvecs
-  DBuf xp, yp;            // permuted vectors for the reference-order entry
+  DBuf xp;                // full-space result of the aux-bit products before contraction
+  DBuf yp;                // pi-ordered result of the even/odd reference-order product
   double scale32 = 1.0;   // FP32 matvec output scale (applied in FP64)
 
   // two-layer operators
@@ -201,8 +202,6 @@ void gather_f64(const double* src, const uint32_t* idx, double* dst, int64_t n, 
 void gather_cols_f64(const double* src, int64_t lds, const uint32_t* idx, double* dst, int64_t n, int nvec,
                      cudaStream_t s);
 void scatter_f64(const double* src, const uint32_t* idx, double* dst, int64_t n, cudaStream_t s);
-void gather_f32(const float* src, const uint32_t* idx, float* dst, int64_t n, cudaStream_t s);
-void scatter_f32(const float* src, const uint32_t* idx, float* dst, int64_t n, cudaStream_t s);
 
 }  // namespace ltm
 
