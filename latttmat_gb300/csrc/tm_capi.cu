@@ -333,12 +333,13 @@ static void build_op(Op& op) {
       op.ws_a.release();
       op.ws_b.release();
       op.ws_c.alloc((size_t)op.n * 8);
-      if (bfly_core(op.kind)) op.ws_a.alloc((size_t)op.nstate * 8);
+      if (bfly_core(op.kind)) build_bfly(op);
     }
   } else {
     if (op.L > 30) fail(TM_ERR_LIMIT, "full operators support L <= 30");
     op.n = op.nstate;
     build_tvec(op);
+    if (bfly_core(op.kind)) build_bfly(op);
   }
   if (!bfly_core(op.kind)) build_aux(op);
 }

@@ -1,21 +1,27 @@
 // Full-space transfer-matrix cores and the generic reduced-basis path.
 //
-// Kronecker sweep (x-ANNNI perpendicular TM, 3D ANNNI): the inter-layer
+// Kronecker factor (x-ANNNI perpendicular TM, 3D ANNNI): the inter-layer
 // factor Th = (x)_{i<L} t with t = [[e^K, e^-K], [e^-K, e^K]]
 // (TMat/tmat.cpp:79-93, the L in-place butterflies of XATMatVecProd2D and of
-// permute_mult_TL).  Here the butterflies run in shared-memory tiles: a pass
-// takes up to NB bits at once, so L bits cost ceil(L/NB) passes over HBM
-// instead of L.  The coefficients are normalised, a' = e^K/(e^K+e^-K), so
-// intermediates stay bounded in FP32; (e^K+e^-K)^L is folded into the FP64
-// output scale.  The Boltzmann-weight scaling (Tv^(1/2) x) is fused into the
-// first pass's load and nf*Tv^(1/2) into the last pass's store.
+// permute_mult_TL), applied as x0 + r x1 (tm_bfly.cuh).  FP64 products are
+// bound by the FP64 pipe (two lanes per clock and SM on sm_103a: every FMA
+// and conversion counts, memory does not), FP32 products by memory.
 //
-// Generic reduced path (any reduced operator): expand the representative
-// vector to the full space through the state->rank map, run the full core,
-// then gather the representatives (TMat/tmatreduce.cpp:406-529 restated as
-// y = D^(1/2) Tv^(1/2) Th Tv^(1/2) P D^(-1/2) x evaluated at representatives).
+// Full operators: shared-memory tile passes of up to 10 bits
+// (kron_tile_kernel), Tv^(1/2) fused into the first load and nf Tv^(1/2) into
+// the last store.
+//
+// Reduced operators evaluate y = D^(1/2) Tv^(1/2) Th Tv^(1/2) P D^(-1/2) x
+// (TMat/tmatreduce.cpp:406-529) at the representatives.  With a translation
+// group the output bits are built from the top down and only prefixes that
+// lead to a representative are kept (tm_tree.cu, kron_tree_kernel): about a
+// third of the multiply-adds at L = 25.  Groups without translations (open
+// boundary) expand to the full space, run the full passes and gather.
+#include <algorithm>
 #include <cmath>
+#include <vector>
 
+#include "tm_bfly.cuh"
 #include "tm_internal.h"
 
 namespace ltm {
@@ -23,113 +29,329 @@ namespace ltm {
 namespace {
 
 template <class T>
-struct Coef {
-  T a, b;
+struct Kron {
+  T r;       // min(a, b) / max(a, b)
+  int swap;  // b > a
 };
 
-// smem index with one pad word every 32 elements (bank-conflict relief for
-// strided butterfly partners)
-__device__ __forceinline__ int spad(int e) { return e + (e >> 5); }
-
-// One sweep pass.  Elements handled by a CTA: 2^nb butterfly positions (bits
-// [lo, lo+nb)) times 2^cb contiguous positions (bits [0, cb), only when lo>0),
-// for one value of the remaining "outer" bits.
-//   load_mode 0: v = x[i]; 1: v = x[i]*pre[i]; 2: v = x[map[i]]
-//   store_mode 0: out[i] = v; 1: out[i] = v*post*scale[i] (FP64 product)
 template <class T>
-__global__ void __launch_bounds__(512) sweep_kernel(const T* __restrict__ x, T* __restrict__ out,
-                                                    int L, int lo, int nb, int cb, Coef<T> c,
-                                                    int load_mode, const double* __restrict__ pre,
-                                                    const uint32_t* __restrict__ map,
-                                                    int store_mode, const double* __restrict__ scale,
-                                                    double post) {
-  extern __shared__ unsigned char smem_raw[];
+Kron<T> kron_of(const Op& op) {
+  return Kron<T>{(T)std::exp(-2.0 * std::fabs(op.mp.betaJ)), op.mp.betaJ < 0 ? 1 : 0};
+}
+
+// ------------------------------------------------------------------ tile passes
+// One butterfly round on tile bits [G0, G0 + GS) of every row (a row is the
+// 2^nb mixed positions of one chunk position).
+template <class T, int G0, int GS>
+__device__ __forceinline__ void tile_round(T* sm, int nb, int cb, int pitch, const Kron<T>& c) {
+  const int fb = nb - GS;
+  for (int f = threadIdx.x; f < (1 << (fb + cb)); f += blockDim.x) {
+    const int g = f & ((1 << fb) - 1);
+    T* b = sm + (f >> fb) * pitch + spad((g & ((1 << G0) - 1)) | ((g >> G0) << (G0 + GS)));
+    T v[1 << GS];
+#pragma unroll
+    for (int i = 0; i < (1 << GS); ++i) v[i] = b[spad(i << G0)];
+    reg_bfly<T, GS>(v, c.r, c.swap);
+#pragma unroll
+    for (int i = 0; i < (1 << GS); ++i) b[spad(i << G0)] = v[i];
+  }
+  __syncthreads();
+}
+
+constexpr int kTileMix = 11;  // most mixed bits of a tile
+
+template <class T, int KB, int R = 0>
+__device__ __forceinline__ void tile_rounds(T* sm, int nb, int cb, int pitch, const Kron<T>& c) {
+  constexpr int G0 = R * KB;
+  const int left = nb - G0;
+  if (left <= 0) return;
+  if (left >= KB) {
+    tile_round<T, G0, KB>(sm, nb, cb, pitch, c);
+  } else {
+    if constexpr (KB > 3)
+      if (left == 3) tile_round<T, G0, 3>(sm, nb, cb, pitch, c);
+    if constexpr (KB > 2)
+      if (left == 2) tile_round<T, G0, 2>(sm, nb, cb, pitch, c);
+    if constexpr (KB > 1)
+      if (left == 1) tile_round<T, G0, 1>(sm, nb, cb, pitch, c);
+    return;
+  }
+  if constexpr ((R + 1) * KB < kTileMix) tile_rounds<T, KB, R + 1>(sm, nb, cb, pitch, c);
+}
+
+// x * pre * fac (load) and v * sc * fac (store) in the vector's type
+__device__ __forceinline__ double weigh(double v, double t, const ScaleF& f) { return v * t * f.f64; }
+__device__ __forceinline__ float weigh(float v, double t, const ScaleF& f) { return scale_round(v, t, f); }
+
+// One pass: 2^nb positions of bits [lo, lo + nb) times 2^cb contiguous
+// positions of bits [0, cb) (only when lo > 0), for one value of the other
+// bits per block.
+//   load_mode 0: v = x[i]; 1: v = x[i]*pre[i]*fin; 2: v = x[map[i]]
+//   store_mode 0: out[i] = v; 1: out[i] = v*scale[i]*fout
+template <class T, int KB>
+__global__ void __launch_bounds__(512) kron_tile_kernel(const T* __restrict__ x, T* __restrict__ out, int lo, int nb,
+                                                        int cb, Kron<T> c, int load_mode,
+                                                        const double* __restrict__ pre, ScaleF fin,
+                                                        const uint32_t* __restrict__ map, int store_mode,
+                                                        const double* __restrict__ scale, ScaleF fout) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
   T* sm = reinterpret_cast<T*>(smem_raw);
-  const int tile_bits = nb + cb;
-  const int tile = 1 << tile_bits;
-  // outer index -> the bits not in [0,cb) U [lo,lo+nb)
+  const int tile = 1 << (nb + cb);
+  const int pitch = spad(1 << nb) | 1;  // odd: chunk neighbours fall into different banks
+  // block index -> the bits not in [0, cb) U [lo, lo + nb)
   const uint64_t outer = blockIdx.x;
-  const uint64_t low_outer_bits = (uint64_t)(lo - cb);  // bits [cb, lo)
-  const uint64_t o_lo = outer & ((1ull << low_outer_bits) - 1);
-  const uint64_t o_hi = outer >> low_outer_bits;
-  const uint64_t base = (o_lo << cb) | (o_hi << (lo + nb));
-  auto gidx = [&](int e) -> uint64_t {
-    uint64_t k = (uint64_t)(e & ((1 << cb) - 1));
-    uint64_t j = (uint64_t)(e >> cb);
-    return base | k | (j << lo);
-  };
+  const int low_outer = lo - cb;
+  const uint64_t base = ((outer & ((1ull << low_outer) - 1)) << cb) | ((outer >> low_outer) << (lo + nb));
+  const int kmask = (1 << cb) - 1;
   for (int e = threadIdx.x; e < tile; e += blockDim.x) {
-    uint64_t i = gidx(e);
+    const uint64_t i = base | (uint64_t)(e & kmask) | ((uint64_t)(e >> cb) << lo);
     T v;
     if (load_mode == 0)
       v = x[i];
     else if (load_mode == 1)
-      v = (T)((double)x[i] * pre[i]);
+      v = weigh(x[i], pre[i], fin);
     else
       v = x[map[i]];
-    sm[spad(e)] = v;
+    sm[(e & kmask) * pitch + spad(e >> cb)] = v;
   }
   __syncthreads();
-  const int npair = tile >> 1;
-  for (int b = 0; b < nb; ++b) {
-    const int bit = cb + b;  // position inside the tile index
-    for (int p = threadIdx.x; p < npair; p += blockDim.x) {
-      int lowm = (1 << bit) - 1;
-      int e0 = ((p & ~lowm) << 1) | (p & lowm);
-      int e1 = e0 | (1 << bit);
-      T v0 = sm[spad(e0)], v1 = sm[spad(e1)];
-      sm[spad(e0)] = c.a * v0 + c.b * v1;
-      sm[spad(e1)] = c.b * v0 + c.a * v1;
-    }
-    __syncthreads();
-  }
+  tile_rounds<T, KB>(sm, nb, cb, pitch, c);
   for (int e = threadIdx.x; e < tile; e += blockDim.x) {
-    uint64_t i = gidx(e);
-    T v = sm[spad(e)];
-    if (store_mode == 1) v = (T)((double)v * post * scale[i]);
+    const uint64_t i = base | (uint64_t)(e & kmask) | ((uint64_t)(e >> cb) << lo);
+    T v = sm[(e & kmask) * pitch + spad(e >> cb)];
+    if (store_mode == 1) v = weigh(v, scale[i], fout);
     out[i] = v;
   }
 }
 
+template <class T, int KB>
+void launch_tile(int64_t nblocks, int threads, size_t shm, cudaStream_t s, const T* x, T* out, int lo, int nb, int cb,
+                 const Kron<T>& c, int load_mode, const double* pre, const ScaleF& fin, const uint32_t* map,
+                 int store_mode, const double* scale, const ScaleF& fout) {
+  if (shm > 48 * 1024) raise_smem_limit((const void*)kron_tile_kernel<T, KB>, shm);
+  kron_tile_kernel<T, KB><<<(unsigned)nblocks, threads, shm, s>>>(x, out, lo, nb, cb, c, load_mode, pre, fin, map,
+                                                                  store_mode, scale, fout);
+  TM_CKK("kron_tile");
+}
+
+// The passes of a full-space product.  Up to 9 bits go in one pass (one
+// block; a second launch would cost more than its 9 levels), else the bits
+// are spread over ceil(L / 9) (FP64) or ceil(L / 10) passes.  A block takes
+// up to 16 contiguous positions beside the mixed ones, fewer where that would
+// leave SMs without a block: at small L the FP64 pipe of one SM is the limit
+// (L = 12 in one 4096-element block took 38 us).  Threads: 16 elements each
+// (one round of four levels in registers) in large tiles, 2 or 4 in small
+// ones, so that all four schedulers of an SM have a warp.
 template <class T>
-void run_sweep(const Op& op, const T* x, T* out, int L, int load_mode, const double* pre,
-               const uint32_t* map, int store_mode, const double* scale, double post,
-               cudaStream_t s) {
-  const double K = op.mp.betaJ;
-  const double ea = std::exp(K), eb = std::exp(-K);
-  Coef<T> c;
-  c.a = (T)(ea / (ea + eb));
-  c.b = (T)(eb / (ea + eb));
-  const int NB = (sizeof(T) == 8) ? 12 : 13;  // tile bits (32 KB per tile either way)
-  const int CB = (sizeof(T) == 8) ? 4 : 5;
+void run_sweep(const Op& op, const T* x, T* out, int load_mode, const double* pre, double fin, const uint32_t* map,
+               int store_mode, const double* scale, double fout, cudaStream_t s) {
+  const int L = op.L;
+  const Kron<T> c = kron_of<T>(op);
+  const int most = (sizeof(T) == 8) ? 9 : 10;
+  const int npass = (L <= 9) ? 1 : std::max(2, (L + most - 1) / most);
+  const ScaleF fi = scale_factor(fin), fo = scale_factor(fout);
   int lo = 0;
-  bool first = true;
   const T* src = x;
-  while (lo < L) {
-    int cb = (lo == 0) ? 0 : std::min(CB, lo);
-    int nb = std::min(L - lo, NB - cb);
-    bool last = (lo + nb >= L);
-    int tile = 1 << (nb + cb);
-    int64_t nblocks = (int64_t)1 << (L - nb - cb);
-    int threads = std::min(512, std::max(32, tile / 2));
-    size_t shm = (size_t)(tile + tile / 32 + 1) * sizeof(T);
-    sweep_kernel<T><<<(unsigned)nblocks, threads, shm, s>>>(
-        src, out, L, lo, nb, cb, c, first ? load_mode : 0, pre, map, last ? store_mode : 0, scale,
-        post);
-    TM_CKK("sweep");
+  for (int p = 0; p < npass; ++p) {
+    const int nb = (L - lo + npass - p - 1) / (npass - p);
+    const int cb = std::min(std::min(4, lo), std::max(0, L - nb - 7));
+    const int tb = nb + cb;
+    const int kb = (tb >= 11) ? 4 : (tb >= 9 ? 2 : 1);
+    const int threads = std::min(512, std::max(32, (1 << tb) >> kb));
+    const size_t shm = ((size_t)(((1 << nb) + (1 << nb) / 32) | 1) << cb) * sizeof(T);
+    const bool first = (p == 0), last = (p == npass - 1);
+    const int64_t nblocks = (int64_t)1 << (L - tb);
+    auto go = [&](auto k) {
+      launch_tile<T, decltype(k)::value>(nblocks, threads, shm, s, src, out, lo, nb, cb, c, first ? load_mode : 0, pre,
+                                         fi, map, last ? store_mode : 0, scale, fo);
+    };
+    if (kb == 4)
+      go(std::integral_constant<int, 4>());
+    else if (kb == 2)
+      go(std::integral_constant<int, 2>());
+    else
+      go(std::integral_constant<int, 1>());
     src = out;
-    first = false;
     lo += nb;
   }
 }
 
+// ------------------------------------------------------------------ prefix-tree passes
+// The butterflies (x0 + r x1, x1 + r x0) on a thread's 2^KB values, top bit
+// first, forming output blocks below which the mask has a child.  The mask is
+// the same for the whole warp and each block of outputs is one branch: a
+// predicated or selected FMA would take its slot on the FP64 pipe all the
+// same.  The last two levels of a block of four outputs go together.
+template <class T, int KB, int B = KB - 1, int H = 0>
+__device__ __forceinline__ void tree_bfly(T (&v)[1 << KB], uint32_t mask, T r) {
+  constexpr uint32_t kSub = (1u << (1 << B)) - 1u;  // the 2^B leaves of one output block
+  constexpr int J0 = (2 * H) << B, J1 = (2 * H + 1) << B;
+  const bool a0 = (mask >> J0) & kSub, a1 = (mask >> J1) & kSub;
+  if (B <= 1 ? (a0 || a1) : (a0 && a1)) {
+#pragma unroll
+    for (int i = 0; i < (1 << B); ++i) {
+      const T x0 = v[J0 + i], x1 = v[J1 + i];
+      v[J0 + i] = fma_t(r, x1, x0);
+      v[J1 + i] = fma_t(r, x0, x1);
+    }
+    if constexpr (B > 0) {
+      tree_bfly<T, KB, B - 1, 2 * H>(v, B == 1 ? 3u << J0 : mask, r);
+      tree_bfly<T, KB, B - 1, 2 * H + 1>(v, B == 1 ? 3u << J1 : mask, r);
+    }
+  } else if constexpr (B > 1) {
+    if (a0) {
+#pragma unroll
+      for (int i = 0; i < (1 << B); ++i) v[J0 + i] = fma_t(r, v[J1 + i], v[J0 + i]);
+      tree_bfly<T, KB, B - 1, 2 * H>(v, mask, r);
+    } else if (a1) {
+#pragma unroll
+      for (int i = 0; i < (1 << B); ++i) v[J1 + i] = fma_t(r, v[J0 + i], v[J1 + i]);
+      tree_bfly<T, KB, B - 1, 2 * H + 1>(v, mask, r);
+    }
+  }
+}
+
+// One level of a reduced product: the KB next output bits.  Element (node,
+// low): value of the vector whose top bits are the node's prefix (new bits)
+// and whose low bits (`rest` of them, plus the KB mixed here) are still old.
+// A thread holds the 2^KB values of one (node, low), mixes them and stores
+// the node's children at (child, low).
+//   FIRST: one node, values gathered from u through the state -> rank map,
+//          at the complement of every state for K < 0 (t with a and b
+//          exchanged is t after a spin flip, and the flip commutes with t);
+//          with the input scaling (u = x tvec gin) folded in where tv is given
+//          (few enough rows that gathering the weights too costs less than a
+//          launch);
+//   LAST:  the children are the representatives: y = post dup tvec value.
+// Bound by the FP64 pipe in FP64 (78% busy in the first level at L = 25), by
+// the map gather in FP32.  FP64 products against three full-space tile passes
+// with two FP64 operations per element and bit: x-ANNNI at L = 25 without
+// flip 3.17 -> 0.465 ms, the 5x5 layer with flip 3.16 -> 0.142 ms.
+template <class T, int KB, bool FIRST, bool LAST>
+__global__ void __launch_bounds__(256) kron_tree_kernel(const T* __restrict__ src, const uint32_t* __restrict__ smap,
+                                                        const uint2* __restrict__ nodes, int64_t nnode, int rest,
+                                                        Kron<T> c, T* __restrict__ dst,
+                                                        const uint16_t* __restrict__ dup,
+                                                        const double* __restrict__ tv, double post) {
+  const int64_t total = nnode << rest;
+  const int64_t span = (total + 31) & ~(int64_t)31;  // whole warps (the mask is combined over the warp)
+  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < span; t += (int64_t)gridDim.x * blockDim.x) {
+    const bool on = t < total;
+    const int64_t node = on ? (t >> rest) : 0;
+    const int64_t low = on ? (t & (((int64_t)1 << rest) - 1)) : 0;
+    const uint2 nd = on ? __ldg(nodes + node) : make_uint2(0u, 0u);
+    T v[1 << KB];
+    if constexpr (FIRST) {
+      uint32_t at[1 << KB];
+#pragma unroll
+      for (int j = 0; j < (1 << KB); ++j) {
+        const int64_t i = ((int64_t)j << rest) | low;
+        at[j] = __ldcs(smap + (c.swap ? ((int64_t)1 << (rest + KB)) - 1 - i : i));
+      }
+#pragma unroll
+      for (int j = 0; j < (1 << KB); ++j) v[j] = __ldg(src + at[j]);
+      if (tv) {
+#pragma unroll
+        for (int j = 0; j < (1 << KB); ++j) v[j] = (T)((double)v[j] * tv[at[j]] * post);
+      }
+    } else {
+      const T* p = src + (node << (rest + KB)) + low;
+#pragma unroll
+      for (int j = 0; j < (1 << KB); ++j) v[j] = p[(int64_t)j << rest];
+    }
+    tree_bfly<T, KB>(v, __reduce_or_sync(0xffffffffu, nd.y), c.r);
+    int64_t child = nd.x;
+#pragma unroll
+    for (int j = 0; j < (1 << KB); ++j) {
+      if ((nd.y >> j) & 1u) {
+        if constexpr (LAST)
+          dst[child] = (T)((double)v[j] * post * (double)dup[child] * tv[child]);
+        else
+          dst[(child << rest) | low] = v[j];
+        ++child;
+      }
+    }
+  }
+}
+
+int grid_for(int64_t n, int threads = 256) {
+  int64_t b = (n + threads - 1) / threads;
+  int64_t cap = (int64_t)num_sms() * 16;
+  return (int)std::max<int64_t>(1, std::min(b, cap));
+}
+
+template <class T, bool FIRST, bool LAST>
+void launch_tree(int kb, const T* src, const uint32_t* smap, const uint2* nodes, int64_t nnode, int rest,
+                 const Kron<T>& c, T* dst, const uint16_t* dup, const double* tv, double post, cudaStream_t s) {
+  const int grid = (int)std::min<int64_t>(((nnode << rest) + 255) / 256, (int64_t)num_sms() * 64);
+  auto go = [&](auto k) {
+    kron_tree_kernel<T, decltype(k)::value, FIRST, LAST><<<grid, 256, 0, s>>>(src, smap, nodes, nnode, rest, c, dst,
+                                                                              dup, tv, post);
+  };
+  switch (kb) {
+    case 4: go(std::integral_constant<int, 4>()); break;
+    case 3: go(std::integral_constant<int, 3>()); break;
+    case 2: go(std::integral_constant<int, 2>()); break;
+    default: go(std::integral_constant<int, 1>()); break;
+  }
+  TM_CKK("kron_tree");
+}
+
+// y = post dup tvec (Th u) at the representatives; fold: u is x, to be
+// scaled by tvec gin on the way in
+template <class T>
+void run_tree(const Op& op, const T* u, T* y, bool fold, double gin, double post, cudaStream_t s) {
+  const PrefixTree& t = op.tree;
+  const Kron<T> c = kron_of<T>(op);
+  T* buf[2] = {op.ws_a.as<T>(), op.ws_b.as<T>()};
+  const T* src = u;
+  const uint16_t* dup = op.dup.as<uint16_t>();
+  const double* tv = op.tvec.as<double>();
+  for (int i = 0; i < t.nlev; ++i) {
+    const int kb = t.b[i + 1] - t.b[i], rest = op.L - t.b[i + 1];
+    const bool first = (i == 0), last = (i == t.nlev - 1);
+    T* dst = last ? y : buf[i & 1];
+    const uint32_t* smap = op.smap.as<uint32_t>();
+    if (first)
+      launch_tree<T, true, false>(kb, src, smap, t.level(i), t.n[i], rest, c, dst, dup, fold ? tv : nullptr, gin, s);
+    else if (!last)
+      launch_tree<T, false, false>(kb, src, smap, t.level(i), t.n[i], rest, c, dst, dup, tv, post, s);
+    else
+      launch_tree<T, false, true>(kb, src, smap, t.level(i), t.n[i], rest, c, dst, dup, tv, post, s);
+    src = dst;
+  }
+}
+
+// ------------------------------------------------------------------ small operators
+// A whole reduced product of up to 2^11 states in one block: expand, mix,
+// contract (y may be x: every read of x precedes the first barrier).  Launches are what a small product costs (about 2.5 us each
+// against 1.1 us of FP64 work at L = 9): from L = 12 on one SM's FP64 pipe
+// would take longer than the tree's launches.
+constexpr int kSmallBits = 11;
+template <class T>
+__global__ void __launch_bounds__(512) kron_small_kernel(const T* x, const uint32_t* __restrict__ smap,
+                                                         const uint32_t* __restrict__ idx,
+                                                         const uint16_t* __restrict__ dup,
+                                                         const double* __restrict__ tv, int L, Kron<T> c, double gin,
+                                                         double post, T* y, int n) {
+  __shared__ T sm[(1 << kSmallBits) + (1 << kSmallBits) / 32 + 1];
+  for (int i = threadIdx.x; i < (1 << L); i += blockDim.x) {
+    const uint32_t q = smap[i];
+    sm[spad(i)] = (T)((double)x[q] * tv[q] * gin);
+  }
+  __syncthreads();
+  tile_rounds<T, 2>(sm, L, 0, 0, c);
+  for (int i = threadIdx.x; i < n; i += blockDim.x)
+    y[i] = (T)((double)sm[spad((int)idx[i])] * post * (double)dup[i] * tv[i]);
+}
+
 // ---- generic reduced path kernels
 template <class T>
-__global__ void scale_in_kernel(const T* __restrict__ x, const double* __restrict__ tv, T* __restrict__ u,
+__global__ void scale_in_kernel(const T* __restrict__ x, const double* __restrict__ tv, double gin, T* __restrict__ u,
                                 int64_t n) {
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   int64_t st = (int64_t)gridDim.x * blockDim.x;
-  for (; i < n; i += st) u[i] = (T)((double)x[i] * tv[i]);
+  for (; i < n; i += st) u[i] = (T)((double)x[i] * tv[i] * gin);
 }
 
 // y[r] = post * dup[r] * tv[r] * z[idx[r]]
@@ -142,38 +364,85 @@ __global__ void contract_kernel(const T* __restrict__ z, const uint32_t* __restr
   for (; i < n; i += st) y[i] = (T)((double)z[idx[i]] * post * (double)dup[i] * tv[i]);
 }
 
-int grid_for(int64_t n, int threads = 256) {
-  int64_t b = (n + threads - 1) / threads;
-  int64_t cap = (int64_t)num_sms() * 16;
-  return (int)std::max<int64_t>(1, std::min(b, cap));
-}
-
 }  // namespace
 
+// Constants of a Kronecker-core operator, and the workspace of its generic
+// reduced product: the prefix tree of the translation groups with its two
+// level buffers, or the full-space vector.
+void build_bfly(Op& op) {
+  const double K = op.mp.betaJ, aK = std::fabs(K);
+  KronConst& kc = op.kron;
+  kc.S = std::pow(std::exp(K) + std::exp(-K), (double)op.L);
+  // gin keeps the magnitudes of the unnormalised butterflies those of the
+  // normalised factor, (max(a, b) / (a + b))^L = (1 + r)^-L; out undoes it
+  // (its rounding cancels) and applies max(a, b)^L = e^{|K| L}, with the
+  // factor that the rounding of r adds to a constant vector taken out: all L
+  // levels share that rounding, which would grow as L
+  const long double rl = std::exp(-2.0L * (long double)aK), n = (long double)op.L;
+  kc.gin = std::pow(1.0 + (double)rl, -(double)op.L);
+  const long double emax = std::exp((long double)aK * n) / kc.gin;
+  kc.out64 = (double)(emax * std::pow((1.0L + rl) / (1.0L + (long double)kron_of<double>(op).r), n));
+  kc.out32 = (double)(emax * std::pow((1.0L + rl) / (1.0L + (long double)kron_of<float>(op).r), n));
+  if (op.kind == K_XAT) return;
+  const bool shifts = (op.kind == K_XAM && op.grp.periodic) || op.kind == K_XAM3;
+  if (op.L <= kSmallBits) return;
+  if (!shifts) {
+    op.ws_a.alloc((size_t)op.nstate * 8);
+    return;
+  }
+  // four bits per level, the odd ones out in threes at the end
+  std::vector<int> steps;
+  const int nlev = (op.L + 3) / 4;
+  for (int i = 0, b = 0; i < nlev; ++i) {
+    steps.push_back((op.L - b + nlev - i - 1) / (nlev - i));
+    b += steps.back();
+  }
+  build_prefix_tree(op, op.L, steps, op.tree);
+  int64_t most[2] = {1, 1};
+  for (int i = 0; i + 1 < nlev; ++i)
+    most[i & 1] = std::max(most[i & 1], op.tree.n[i + 1] << (op.L - op.tree.b[i + 1]));
+  op.ws_a.alloc((size_t)most[0] * 8);
+  op.ws_b.alloc((size_t)most[1] * 8);
+}
+
 // y = T x on the full space (K_XAT) or on the reduced basis through the full
-// space (reduced kinds whose core is the Kronecker sweep).  scaled=true:
+// space (reduced kinds whose core is the Kronecker factor).  scaled=true:
 // the result is divided by S = (e^K+e^-K)^L and S is returned.
 template <class T>
 double matvec_bfly(const Op& op, const T* x, T* y, bool scaled, cudaStream_t s) {
-  const double K = op.mp.betaJ;
-  const double S = std::pow(std::exp(K) + std::exp(-K), (double)op.L);
-  const double sf = scaled ? 1.0 : S;
+  const KronConst& kc = op.kron;
+  const double sf = ((sizeof(T) == 8) ? kc.out64 : kc.out32) / (scaled ? kc.S : 1.0);
+  const double ret = scaled ? kc.S : 1.0;
+  const double* tv = op.tvec.as<double>();
   if (op.kind == K_XAT) {
     // y = nf * Tv^(1/2) * Th * Tv^(1/2) * x   (TMat/tmat.cpp:71-102)
-    run_sweep<T>(op, x, y, op.L, 1, op.tvec.as<double>(), nullptr, 1, op.tvec.as<double>(),
-                 op.normfactor * sf, s);
-    return scaled ? S : 1.0;
+    run_sweep<T>(op, x, y, 1, tv, kc.gin, nullptr, 1, tv, op.normfactor * sf, s);
+    return ret;
   }
+  const uint32_t* smap = op.smap.as<uint32_t>();
+  const uint32_t* idx = op.idx.as<uint32_t>();
+  const uint16_t* dup = op.dup.as<uint16_t>();
   // reduced: u = Tvec .* x ; v = P u ; z = Th v ; y = dup .* Tvec .* z[idx]
+  if (op.L <= kSmallBits) {
+    kron_small_kernel<T><<<1, 512, 0, s>>>(x, smap, idx, dup, tv, op.L, kron_of<T>(op), kc.gin, sf, y, (int)op.n);
+    TM_CKK("kron_small");
+    return ret;
+  }
+  const bool fold = op.tree.nlev && op.L <= 16;
   T* u = static_cast<T*>(op.ws_c.p);
+  if (!fold) {
+    scale_in_kernel<T><<<grid_for(op.n), 256, 0, s>>>(x, tv, kc.gin, u, op.n);
+    TM_CKK("scale_in");
+  }
+  if (op.tree.nlev) {
+    run_tree<T>(op, fold ? x : u, y, fold, kc.gin, sf, s);
+    return ret;
+  }
   T* full = static_cast<T*>(op.ws_a.p);
-  scale_in_kernel<T><<<grid_for(op.n), 256, 0, s>>>(x, op.tvec.as<double>(), u, op.n);
-  TM_CKK("scale_in");
-  run_sweep<T>(op, u, full, op.L, 2, nullptr, op.smap.as<uint32_t>(), 0, nullptr, 1.0, s);
-  contract_kernel<T><<<grid_for(op.n), 256, 0, s>>>(full, op.idx.as<uint32_t>(), op.dup.as<uint16_t>(),
-                                                    op.tvec.as<double>(), sf, y, op.n);
+  run_sweep<T>(op, u, full, 2, nullptr, 1.0, smap, 0, nullptr, 1.0, s);
+  contract_kernel<T><<<grid_for(op.n), 256, 0, s>>>(full, idx, dup, tv, sf, y, op.n);
   TM_CKK("contract");
-  return scaled ? S : 1.0;
+  return ret;
 }
 
 template double matvec_bfly<float>(const Op&, const float*, float*, bool, cudaStream_t);

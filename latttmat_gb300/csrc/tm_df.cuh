@@ -9,6 +9,9 @@
 // native FP64 one several times over, at relative error ~1e-14 per sweep.
 #pragma once
 #include <cuda_runtime.h>
+#include <stdint.h>
+
+#include <cmath>
 
 namespace ltm {
 
@@ -84,6 +87,54 @@ __device__ __forceinline__ dfloat& operator+=(dfloat& a, dfloat b) {
 __device__ __forceinline__ dfloat& operator*=(dfloat& a, dfloat b) {
   a = a * b;
   return a;
+}
+
+// A constant factor of a result rounded to FP32 once (scale_round): f64, and
+// the same as two * hl with `two` a power of two near its square root, so
+// that partial products stay near the result's exponent range.
+struct ScaleF {
+  double f64;
+  float two;
+  dfloat hl;
+};
+inline ScaleF scale_factor(double S) {
+  ScaleF p{S, 1.f, dfloat(1.0)};
+  int e = 0;
+  std::frexp(S, &e);
+  if (std::isfinite(S) && S > 0 && e > -120 && e < 120) {
+    p.two = std::ldexp(1.f, e / 2);
+    p.hl = dfloat(S / (double)p.two);
+  }
+  return p;
+}
+
+// (v * sc) * post rounded to FP32 once: the products' rounding errors are
+// carried along (TwoProduct by FMA), so the result is that of FP64 arithmetic
+// to within the last rounding, without the FP64 pipe (two lanes per clock and
+// SM, conversions included).  Zeros, infinities, NaN and products near the
+// ends of the exponent range, where the error terms would be lost, take the
+// FP64 form.
+__device__ __forceinline__ float scale_round(float v, dfloat sc, const ScaleF& post) {
+  const float a = v * post.two;  // exact
+  const float p = a * sc.hi;
+  if (!(fabsf(p) > 1e-24f && fabsf(p) < 1e24f)) return (float)((double)v * (double)sc * post.f64);
+  const float e = fmaf(a, sc.lo, fmaf(a, sc.hi, -p));
+  const float q = p * post.hl.hi;
+  return q + fmaf(e, post.hl.hi, fmaf(p, post.hl.lo, fmaf(p, post.hl.hi, -q)));
+}
+
+// v * t * post for an FP64 weight t: t is split into a double-float by
+// integer operations (the hi word truncated to 24 bits, the lo word the 29
+// bits below), so nothing runs on the FP64 pipe but the rare cases.
+__device__ __forceinline__ float scale_round(float v, double t, const ScaleF& post) {
+  const uint32_t up = (uint32_t)__double2hiint(t), dn = (uint32_t)__double2loint(t);
+  const int e = (int)((up >> 20) & 0x7ffu) - 1023;
+  if (e < -70 || e > 90) return (float)((double)v * t * post.f64);
+  const uint32_t sign = up & 0x80000000u;
+  const uint32_t m23 = ((up & 0xfffffu) << 3) | (dn >> 29);
+  const float hi = __uint_as_float(sign | ((uint32_t)(e + 127) << 23) | m23);
+  const float lo = __uint2float_rn(dn & 0x1fffffffu) * __uint_as_float(sign | ((uint32_t)(e - 52 + 127) << 23));
+  return scale_round(v, dfloat(hi, lo), post);
 }
 
 // Forward-mode tangent pair (value, derivative with respect to one

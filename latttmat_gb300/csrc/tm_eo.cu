@@ -52,6 +52,7 @@
 #include <type_traits>
 #include <vector>
 
+#include "tm_bfly.cuh"
 #include "tm_df.cuh"
 #include "tm_group.cuh"
 #include "tm_internal.h"
@@ -124,8 +125,6 @@ struct EOArgs {
   int swap;
 };
 
-__device__ __forceinline__ int spad(int e) { return e + (e >> 5); }
-
 template <class T>
 __device__ __forceinline__ T coef_r(const EOArgs& A);
 template <>
@@ -134,39 +133,6 @@ template <>
 __device__ __forceinline__ double coef_r<double>(const EOArgs& A) { return A.r64; }
 template <>
 __device__ __forceinline__ dfloat coef_r<dfloat>(const EOArgs& A) { return dfloat(A.r64); }
-
-// r * x + y in the engine's arithmetic
-__device__ __forceinline__ float fma_t(float r, float x, float y) { return fmaf(r, x, y); }
-__device__ __forceinline__ double fma_t(double r, double x, double y) { return fma(r, x, y); }
-__device__ __forceinline__ dfloat fma_t(dfloat r, dfloat x, dfloat y) { return df_fma_unnorm(r, x, y); }
-
-// In-register butterflies on all NB levels of the 2^NB elements held by one
-// thread.  Output pair of level lv: (x0 + r x1, x1 + r x0), or exchanged
-// (swap).
-template <class T, int NB>
-__device__ __forceinline__ void reg_bfly(T (&v)[1 << NB], T r, int swap) {
-  if (!swap) {
-#pragma unroll
-    for (int lv = 0; lv < NB; ++lv)
-#pragma unroll
-      for (int i = 0; i < (1 << NB); ++i)
-        if (!(i & (1 << lv))) {
-          const T x0 = v[i], x1 = v[i | (1 << lv)];
-          v[i] = fma_t(r, x1, x0);
-          v[i | (1 << lv)] = fma_t(r, x0, x1);
-        }
-  } else {
-#pragma unroll
-    for (int lv = 0; lv < NB; ++lv)
-#pragma unroll
-      for (int i = 0; i < (1 << NB); ++i)
-        if (!(i & (1 << lv))) {
-          const T x0 = v[i], x1 = v[i | (1 << lv)];
-          v[i] = fma_t(r, x0, x1);
-          v[i | (1 << lv)] = fma_t(r, x1, x0);
-        }
-  }
-}
 
 // The FP32 butterflies with the elements held in pairs (v[k] = elements 2k,
 // 2k + 1): level 0 pairs the two halves of one register pair (two scalar
@@ -629,31 +595,9 @@ __global__ void __launch_bounds__(1024, 1) eo_pass1(EOArgs A, const InT* __restr
 // Output modes of pass 2: y = val * sout32 (FP32), val * sout64 * post
 // (FP64), val * soutdf in double-float (double-float storage), or an FP32
 // val * soutdf * post formed in double-float and rounded once (kOutF32S).
+// Two FP64 multiplies and three conversions per output in place of the last
+// took 0.44 ms of pass 2's 1.22 ms at L = 32; it takes 0.79 ms in all.
 enum { kOutF32 = 0, kOutF64 = 1, kOutDF = 2, kOutF32S = 3 };
-
-// Output factor of kOutF32S: two * hl, two a power of two near its square
-// root, so that the partial products stay near the result's exponent range.
-struct EoPost {
-  double f64;
-  float two;
-  dfloat hl;
-};
-
-// (v * sc) * post rounded to FP32 once: the products' rounding errors are
-// carried along (TwoProduct by FMA), so the result is the FP64 path's to
-// within the last rounding.  Two FP64 multiplies and three conversions per
-// output took 0.44 ms of pass 2's 1.22 ms at L = 32 (two FP64 lanes per
-// clock and SM); this takes 0.79 ms in all.
-__device__ __forceinline__ float scale_round(float v, dfloat sc, const EoPost& post) {
-  const float a = v * post.two;  // exact
-  const float p = a * sc.hi;
-  // zeros, infinities, NaN and products near the ends of the exponent range
-  // (where the error terms would be lost) take the FP64 form
-  if (!(fabsf(p) > 1e-24f && fabsf(p) < 1e24f)) return (float)((double)v * (double)sc * post.f64);
-  const float e = fmaf(a, sc.lo, fmaf(a, sc.hi, -p));
-  const float q = p * post.hl.hi;
-  return q + fmaf(e, post.hl.hi, fmaf(p, post.hl.lo, fmaf(p, post.hl.hi, -q)));
-}
 
 // pass 2: z[(e_rep, o)] = (Th_O w)[(e_rep, o)]; emit designated outputs.
 // The w value at (e_rep, o) is the pass-1 value at the H-image
@@ -671,7 +615,7 @@ __global__ void __launch_bounds__(1024, 1) eo_pass2(EOArgs A, const T* __restric
                                                     const uint16_t* __restrict__ out_o,
                                                     const double* __restrict__ sout64,
                                                     const float* __restrict__ sout32,
-                                                    const dfloat* __restrict__ soutdf, EoPost post,
+                                                    const dfloat* __restrict__ soutdf, ScaleF post,
                                                     OutT* __restrict__ y, float4* __restrict__ xchg) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* sm = reinterpret_cast<T*>(smem_raw);
@@ -1319,17 +1263,6 @@ bool eo_scale_fits32(const Op& op) {
   return bz < 60.0 && lnS < 60.0;
 }
 
-EoPost eo_post(double S) {
-  EoPost p{S, 1.f, dfloat(1.0)};
-  int e = 0;
-  std::frexp(S, &e);
-  if (std::isfinite(S) && S > 0 && e < 120) {
-    p.two = std::ldexp(1.f, e / 2);
-    p.hl = dfloat(S / (double)p.two);
-  }
-  return p;
-}
-
 // input factor of the unnormalised butterflies: (1 + r)^-L, r = e^-2|K|
 double eo_gin(const Op& op) {
   return std::pow(1.0 + std::exp(-2.0 * std::fabs(op.mp.betaJ)), -(double)op.L);
@@ -1386,7 +1319,7 @@ void launch_pass1(const EOArgs& A, int ntiles, const typename EoIO<T>::In* u, co
 
 template <class T, int KB, int OSC, class OutT = typename EoIO<T>::Out>
 void launch_pass2(const EOArgs& A, int ntiles, const T* w1, const EOPlan& P, const double* sout64,
-                  const float* sout32, const dfloat* soutdf, EoPost post, OutT* y, cudaStream_t s) {
+                  const float* sout32, const dfloat* soutdf, ScaleF post, OutT* y, cudaStream_t s) {
   size_t shm = (size_t)((1 << A.n) + (1 << A.n) / 32 + 1) * sizeof(T);
   auto kfn = (A.c > 0) ? eo_pass2<T, KB, OSC, OutT, true> : eo_pass2<T, KB, OSC, OutT, false>;
   raise_smem_limit((const void*)kfn, shm);
@@ -1450,7 +1383,7 @@ void eo_dispatch(const Op& op, const EOArgs& A, const typename EoIO<T>::In* x, t
   launch_pass1<T, KB>(A, P.n_orep, u, P, w1, s);
   TM_CKK("eo_pass1");
   if (P.prof_on) TM_CK(cudaEventRecord(P.prof_ev[2], s));
-  const EoPost post = eo_post(scaled32 ? 1.0 : eo_scale32(op));
+  const ScaleF post = scale_factor(scaled32 ? 1.0 : eo_scale32(op));
   using Out = typename EoIO<T>::Out;
   Out* yo = ref ? op.yp.as<Out>() : y;
   const double* so64 = op.sout64.as<double>();
@@ -1555,7 +1488,7 @@ void eo_dispatch_dd(const Op& op, const EOArgs& A, const dfloat* x, dfloat* y, c
                            P.wout.as<uint2>(), w1, eo_xchg<dfloat>(A, P, P.n_orep)));
   TM_CKK("eo_pass1_dd");
   launch_pass2<dfloat, KB, kOutDF, dfloat>(A, P.n_erep, w1, P, op.sout64.as<double>(), op.sout32.as<float>(),
-                                           op.soutdf.as<dfloat>(), eo_post(1.0), y, s);
+                                           op.soutdf.as<dfloat>(), scale_factor(1.0), y, s);
   TM_CKK("eo_pass2_dd");
 }
 }  // namespace
@@ -1584,7 +1517,7 @@ void matvec_eo_f64_into(const Op& op, const double* x, double* y, double* u, dou
   eo_scale_in<double><<<grid_for(R), 256, 0, s>>>(x, op.sin64.as<double>(), op.sin32.as<float>(), u, R,
                                                    eo_gin(op));
   TM_CKK("eo_scale_in");
-  const EoPost post = eo_post(eo_scale32(op));
+  const ScaleF post = scale_factor(eo_scale32(op));
   switch (A.n - A.p) {
 #define TM_EO_INTO(KBV)                                                                                      \
   case KBV:                                                                                                  \

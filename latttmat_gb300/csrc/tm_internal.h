@@ -112,6 +112,26 @@ struct EOPlan {
   bool prof_on = false;
 };
 
+// Prefix tree of a reduced operator's representatives (tm_tree.cu): level i
+// holds the distinct b[i]-bit prefixes, a node {first child, mask of the
+// children's step bits}; level nlev is the representatives themselves.
+constexpr int kTreeMaxLevels = 32;
+struct PrefixTree {
+  int nlev = 0;                      // 0: no tree
+  int b[kTreeMaxLevels + 1] = {0};   // prefix length per level
+  int64_t n[kTreeMaxLevels + 1] = {0};
+  int64_t off[kTreeMaxLevels + 1] = {0};
+  DBuf nodes;                        // uint2, level i at off[i]
+  uint2* level(int i) const { return nodes.as<uint2>() + off[i]; }
+};
+
+// Host constants of the Kronecker-core products (set once per operator).
+struct KronConst {
+  double S = 1.0;               // (e^K + e^-K)^L
+  double gin = 1.0;             // input factor (1 + r)^-L
+  double out64 = 1.0, out32 = 1.0;  // output factors of the FP64 / FP32 butterflies
+};
+
 struct Op {
   // identity
   char model = 'A';
@@ -141,6 +161,8 @@ struct Op {
   DBuf tvec;       // f64 [n or nstate]: the operator's Tvec (Tv^(1/2) [* nf^(1/2)] / sqrt(dup))
   // generic reduced path: state -> rank map
   DBuf smap;       // u32 [nstate]
+  KronConst kron;
+  PrefixTree tree; // translation groups: output prefixes that lead to a representative
   // pi order (internal vector order): pi[k] = reference index; identity if empty
   bool has_pi = false;
   DBuf pi, pinv;   // u32 [n]
@@ -168,6 +190,8 @@ void build_group(Op& op);
 void build_orbit_table(Op& op);          // idx, dup (reference order)
 void build_tvec(Op& op);                 // Tvec for the operator
 void build_state_map(Op& op);            // smap for the generic reduced path
+void build_prefix_tree(const Op& op, int nbits, const std::vector<int>& steps, PrefixTree& out);
+void build_bfly(Op& op);                 // constants, tree and workspace of the Kronecker-core products
 struct EOHostTables;                     // host-side even/odd plan tables (tm_eo.cu)
 std::shared_ptr<EOHostTables> eo_host_tables(int m, int flip);
 void build_eo_plan(Op& op, const EOHostTables* host = nullptr);  // even/odd plan for K_XAM
