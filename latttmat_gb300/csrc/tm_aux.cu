@@ -8,22 +8,27 @@
 // sites per step with two carried bits; its transpose swaps the roles of the
 // coupling factors (optdirection = 1).
 //
-// The reference rotates the state by one (two) sites after every step, so the
-// sites a step touches are always the low ones.  Undoing the rotation (a
-// fixed frame: after L/KS steps the rotation is the identity) shows that step
-// t is a local gate: it rewrites the aux bits and the KS sites at positions
-// KS*t .. KS*t+KS-1 from the same 2^(NA+KS) values, with weights that depend on
-// the next KS sites (or, at the last step, on the lastbit pass).  Here a pass
-// gathers tiles of 2^12 (FP64) or 2^13 (FP32) elements whose index bits are the
-// aux bits, a few contiguous low sites (coalescing) and the sites of several
-// consecutive steps, applies those steps in shared memory and writes the tile
-// back in place: ceil(steps / steps-per-pass) sweeps over HBM instead of one
-// per step.  The first pass builds its tiles from x (the reference's sparse
-// initial vector), the last pass folds aux bits and lastbit passes into y.
-// Arithmetic per element is the reference's, in its order.  FP32 steps are
-// scaled by the inverse of their largest row sum; the product of the scales
-// is applied in FP64.  Reduced operators (XDM, ZBM) gather x through the
-// state->rank map and contract the full-space result at the representatives.
+// Undoing the reference's rotation of the state after every step leaves local
+// gates in a fixed frame: step t rewrites the carried letter and the letter
+// (one or two sites) at its position, with weights that depend on the next old
+// letter (at the end of the ring, on the first one: everything runs once per
+// value of it, the "lastbit").  Here the ring is walked from the top of the state
+// down, so that
+//   - a prefix of the new state is known after every step, and a reduced
+//     operator keeps only the prefixes that lead to an orbit's smallest state
+//     (tm_tree.cu): at L = 24 (BNNNI) a third of the elements are left after
+//     four of the twelve steps and a sixth after seven;
+//   - the remaining old bits stay contiguous, whatever the prefixes are.
+// A pass keeps a tile of 2^10..2^14 elements (some letters, a contiguous chunk
+// of the bits below them, the carried letter) in shared memory for several
+// steps; the first pass builds its tiles from x with the first step already
+// applied (the carried letter has one value per state there), the last holds
+// all lastbit values of a node, sums them and the carried letters and writes
+// y.  A step takes two
+// multiply-adds and one multiply per output (BNNNI; one and one for DNNI)
+// through factored tables (ChainTab).  FP32 and double-float steps are scaled
+// by the inverse of their largest row sum; the product of the scales is
+// applied at the output.
 #include <algorithm>
 #include <cmath>
 #include <mutex>
@@ -43,479 +48,797 @@ int grid_for(int64_t n) {
   return (int)std::max<int64_t>(1, std::min<int64_t>(b, (int64_t)num_sms() * 32));
 }
 
-__device__ __forceinline__ int spad(int e) { return e + (e >> 5); }
+// x + rho y in the chain's arithmetic (double-float: renormalised by the
+// multiply that follows)
+__device__ __forceinline__ float xpry(float rho, float y, float x) { return fmaf(rho, y, x); }
+__device__ __forceinline__ double xpry(double rho, double y, double x) { return fma(rho, y, x); }
+__device__ __forceinline__ dfloat xpry(dfloat rho, dfloat y, dfloat x) { return df_fma_unnorm(rho, y, x); }
+__device__ __forceinline__ tangent xpry(tangent rho, tangent y, tangent x) { return x + rho * y; }
 
-__device__ __forceinline__ int64_t chain_pass_blocks_dev(const ChainPass& cp);
+// element type of the pre-scaled input vector u (tangent: its value)
+template <class T>
+struct ChainIn {
+  using U = T;
+};
+template <>
+struct ChainIn<tangent> {
+  using U = dfloat;
+};
+__device__ __forceinline__ void to_elem(float u, float& v) { v = u; }
+__device__ __forceinline__ void to_elem(double u, double& v) { v = u; }
+__device__ __forceinline__ void to_elem(dfloat u, dfloat& v) { v = u; }
+__device__ __forceinline__ void to_elem(dfloat u, tangent& v) { v = tangent(u, dfloat(0.f, 0.f)); }
 
-// the part of a tile value the fold sums: the value, or for a tangent pair
-// its derivative (the tangent product's output)
-__device__ __forceinline__ double fold_part(float x) { return (double)x; }
-__device__ __forceinline__ double fold_part(double x) { return x; }
-__device__ __forceinline__ double fold_part(dfloat x) { return (double)x; }
-__device__ __forceinline__ double fold_part(tangent x) { return (double)x.d; }
+// x times its FP64 weight in the chain's arithmetic
+__device__ __forceinline__ void weigh_in(float x, double t, float& v) { v = scale_round(x, t, ScaleF{1.0, 1.f, dfloat(1.f, 0.f)}); }
+__device__ __forceinline__ void weigh_in(double x, double t, float& v) { v = (float)(x * t); }
+__device__ __forceinline__ void weigh_in(double x, double t, double& v) { v = x * t; }
+__device__ __forceinline__ void weigh_in(double x, double t, dfloat& v) { v = dfloat(x * t); }
+__device__ __forceinline__ void weigh_in(double x, double t, tangent& v) { v = tangent(x * t); }
 
-// acc + a b in the chain's arithmetic: one renormalisation for double-float
-// (df_fma) instead of one per multiply and add
-__device__ __forceinline__ float mad_t(float a, float b, float acc) { return fmaf(a, b, acc); }
-__device__ __forceinline__ double mad_t(double a, double b, double acc) { return fma(a, b, acc); }
-__device__ __forceinline__ dfloat mad_t(dfloat a, dfloat b, dfloat acc) { return df_fma(a, b, acc); }
-__device__ __forceinline__ tangent mad_t(tangent a, tangent b, tangent acc) { return acc + a * b; }
+// fold: sums of the carried letters and lastbit passes, without the FP64 pipe
+// except in FP64 (double-float keeps 48 bits; FP32 values sum exactly enough)
+template <class T>
+struct FoldAcc {
+  using A = dfloat;
+};
+template <>
+struct FoldAcc<double> {
+  using A = double;
+};
+__device__ __forceinline__ dfloat fold_add(dfloat a, float x) { return a + dfloat(x, 0.f); }
+__device__ __forceinline__ double fold_add(double a, double x) { return a + x; }
+__device__ __forceinline__ dfloat fold_add(dfloat a, dfloat x) { return a + x; }
+__device__ __forceinline__ dfloat fold_add(dfloat a, tangent x) { return a + x.d; }
 
-// Double-float values two to a lane pair (hi words in one float2, lo words
-// in another), for the double-float BNNNI steps on the packed FP32 pipes.
-// Each is the scalar double-float operation of tm_df.cuh lane by lane, in
-// the same operation order; differences are fma(b, -1, a), and -p comes from
-// the weight's negated hi word, so no operand needs a separate negation.
-__device__ __forceinline__ float2 dsub2(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }
-// x * w (operator*): w = (wh, wl) with wn = -wh
-__device__ __forceinline__ void df2_mul(float2 xh, float2 xl, float2 wh, float2 wl, float2 wn, float2& oh,
-                                       float2& ol) {
-  const float2 np = __fmul2_rn(xh, wn);  // -p
-  float2 e = __ffma2_rn(xh, wh, np);
-  e = __ffma2_rn(xh, wl, e);
-  e = __ffma2_rn(xl, wh, e);
-  oh = dsub2(e, np);                        // p + e
-  ol = dsub2(e, __fadd2_rn(oh, np));        // e - (h - p)
+// ------------------------------------------------------------------ tile slots
+// A slot holds the S values of the carried letter.  It is kept as 16-byte (8
+// for DNNI in FP32) vectors, each in a plane of its own: neighbouring slots
+// are then neighbouring vectors, where whole 32-byte slots would use half the
+// banks per access (the first BNNNI pass's shared-memory pipe was 73% busy
+// that way, its FP32 pipe 45%).  Vector i of a plane sits at i + i / 8 (8-byte
+// vectors: i + i / 16), one pad per 128 bytes, so that strided letters spread
+// over the banks, and planes are 64 bytes apart modulo 128.  Double-float
+// slots are planar (hi words, then lo words), the order the packed FP32 lanes
+// take them in.
+template <class T, int S>
+struct SlotT {
+  static constexpr int kBytes = S * (int)sizeof(T);
+  using V = typename std::conditional<kBytes == 8, uint2, uint4>::type;
+  static constexpr int kVecs = kBytes / (int)sizeof(V);
+  static constexpr int kShift = (kBytes == 8) ? 4 : 3;
+};
+
+__host__ __device__ __forceinline__ int slot_plane(int slots, int slot_bytes) {
+  const int n = slots + (slots >> (slot_bytes == 8 ? 4 : 3));
+  return slot_bytes <= 16 ? n : ((n + 7) & ~7) + 4;
 }
-// x * w + y (df_fma)
-__device__ __forceinline__ void df2_fma(float2 xh, float2 xl, float2 wh, float2 wl, float2 wn, float2 yh, float2 yl,
-                                       float2& oh, float2& ol) {
-  const float2 np = __fmul2_rn(xh, wn);  // -p
-  float2 pe = __ffma2_rn(xh, wh, np);
-  pe = __ffma2_rn(xh, wl, pe);
-  pe = __ffma2_rn(xl, wh, pe);
-  const float2 sm = dsub2(yh, np);                     // p + y.hi
-  const float2 bb = __fadd2_rn(sm, np);                // s - p
-  const float2 e2 = dsub2(yh, bb);                     // y.hi - bb
-  float2 se = dsub2(e2, __fadd2_rn(np, dsub2(sm, bb)));  // (p - (s - bb)) + (y.hi - bb)
-  se = __fadd2_rn(se, __fadd2_rn(pe, yl));
-  oh = __fadd2_rn(sm, se);
-  ol = dsub2(se, dsub2(oh, sm));
+
+// vector k of slot i
+template <class T, int S>
+__device__ __forceinline__ typename SlotT<T, S>::V* slot_vec(unsigned char* sm, int plane, int i, int k) {
+  return reinterpret_cast<typename SlotT<T, S>::V*>(sm) + k * plane + i + (i >> SlotT<T, S>::kShift);
 }
 
-// byte offset of the fold accumulators in chain_kernel's shared memory
-__host__ __device__ __forceinline__ size_t chain_acc_offset(int tile, size_t elem) {
-  return (((size_t)(tile + tile / 32 + 1) * elem) + 15) & ~(size_t)15;
-}
-
-// tile state index -> state bits: the tile's state bits are the contiguous
-// runs [0, cb) and [lo, lo + nst - cb)
-__device__ __forceinline__ uint64_t tile_state(uint64_t v, int cb, int lo) {
-  return (v & ((1ull << cb) - 1)) | ((v >> cb) << lo);
-}
-
-__device__ __forceinline__ uint64_t dep(uint64_t v, const int* pos, int nb) {
-  uint64_t g = 0;
-  for (int k = 0; k < nb; ++k) g |= ((v >> k) & 1ull) << pos[k];
-  return g;
-}
-
-// Initial (lastbit pass lb) value of element (aux, r): TMat/tmat.cpp:392-457
-// (DNNI: aux = copy of the top site, site 0 = lb; boundary cases 5 and 9) and
-// :604-612 (BNNNI: aux = copy of the two top sites, sites 0-1 = lb).
-template <class T, int ZB, class IO>
-__device__ __forceinline__ T chain_init(const IO* __restrict__ x, const double* __restrict__ pre,
-                                        const uint32_t* __restrict__ smap, int L, int bc, uint64_t r, int aux, int lb,
-                                        const AuxCoefT<T>& c) {
-  auto u = [&]() -> T {
-    if (smap) {
-      const uint32_t q = smap[r];
-      return (T)((double)x[q] * pre[q]);
-    }
-    return pre ? (T)((double)x[r] * pre[r]) : (T)x[r];
-  };
-  if (ZB) {
-    if ((int)(r >> (L - 2)) == aux && (int)(r & 3) == lb) return u();
-    return (T)0;
+// a slot in a pass buffer (its vectors are consecutive there)
+template <class T, int S>
+__device__ __forceinline__ void vec_to_slot(const typename SlotT<T, S>::V (&raw)[SlotT<T, S>::kVecs], T (&v)[S]) {
+  if constexpr (std::is_same<T, dfloat>::value) {
+    const float* f = reinterpret_cast<const float*>(raw);
+#pragma unroll
+    for (int q = 0; q < S; ++q) v[q] = dfloat(f[q], f[S + q]);
+  } else {
+    const T* e = reinterpret_cast<const T*>(raw);
+#pragma unroll
+    for (int q = 0; q < S; ++q) v[q] = e[q];
   }
-  if (bc == 0) {
-    if ((int)(r >> (L - 1)) == aux && (int)(r & 1) == lb) return u();
-    return (T)0;
-  }
-  if (bc == 5) return aux == 0 ? u() * c.b2[r & 1] * c.b2[r >> (L - 1)] : (T)0;
-  return aux == 1 ? u() * c.b2[(r & 1) ^ 1] * c.b2[r >> (L - 1)] : (T)0;  // bc 9
 }
-
-// One pass of steps over tiles in shared memory.
-//   ZB = 0: DNNI, NA = 1 aux bit, one site per step (permute_mult_T1 /
-//           _last, TMat/tmat.cpp:344-376); L steps.
-//   ZB = 1: diagonal BNNNI, NA = 2, two sites per step (TMat/tmat.cpp:521-588,
-//           dir = optdirection); L/2 steps.
-// P: the nlb*2^L*2^NA buffer (in place).  first: tiles built from x; last:
-// y[r] = postc * post[r] * sum_{lb, aux} (one CTA loops the lastbit passes).
-// (the body of one block: `blk` is its index within the pass's grid)
-template <class T, int ZB, class IO>
-__device__ __forceinline__ void chain_block(T* __restrict__ P, const IO* __restrict__ x,
-                                            const double* __restrict__ pre, const uint32_t* __restrict__ smap,
-                                            IO* __restrict__ y, const double* __restrict__ post, double postc, int L,
-                                            int bc, int dir, const AuxCoefT<T>& c, const ChainPass& cp, uint64_t blk) {
-  constexpr int NA = ZB ? 2 : 1, KS = ZB ? 2 : 1, GB = NA + KS;  // group bits
-  extern __shared__ unsigned char smraw[];
-  T* sm = reinterpret_cast<T*>(smraw);
-  const int tile = 1 << (NA + cp.nst);
-  const int nsteps = ZB ? L / 2 : L;
-  // FP64 fold accumulators after the padded tile, at a 16-byte boundary
-  // (the FP32 tile's padded size is not a multiple of 8 bytes)
-  double* acc = reinterpret_cast<double*>(smraw + chain_acc_offset(tile, sizeof(T)));
-  // Step coefficients, functions of the control bits only.  The step's
-  // matrix factorises as out(a', s') = z_f[s'] u[a'][s'] sum_q w[s'][q]
-  // in(q, a'): w and u (the step normalisation folded into u) are the same
-  // for every group and sit in shared memory, read as broadcast rows; only
-  // z depends on the group's control bits f and is formed in registers.
-  //   BNNNI dir 0: w = b1[sr^al] b2[sr^ar] b2[sl^al], u = b1[sr^pl] b3[sr^pr] b3[sl^pl],
-  //                z = b2[sr^fr] b2[sl^fl];
-  //   BNNNI dir 1: w = b2[sr^ar] b2[sl^al], u = b1[sl^pr] b3[sr^pr] b3[sl^pl],
-  //                z = b1[sl^fr] b2[sr^fr] b2[sl^fl];
-  //   DNNI:        w = b2[s^q], u = b1[s^a], z = b2[nb^s].
-  // (TMat/tmat.cpp:344-376 and 521-588 form the same products per element.)
-  constexpr int NS = 1 << KS;
-  __shared__ __align__(16) T wrow[16];  // [s'][q]
-  __shared__ __align__(16) T urow[16];  // [s'][a']
-  if (ZB) {
-    for (int k = threadIdx.x; k < 16; k += blockDim.x) {
-      const int sv = k >> 2, q = k & 3, sl = sv >> 1, sr = sv & 1, al = q >> 1, ar = q & 1;
-      wrow[k] = !dir ? c.b1[sr ^ al] * c.b2[sr ^ ar] * c.b2[sl ^ al] : c.b2[sr ^ ar] * c.b2[sl ^ al];
-      const int pl = q >> 1, pr = q & 1;  // here q is a' = (pl, pr)
-      urow[k] = (!dir ? c.b1[sr ^ pl] * c.b3[sr ^ pr] * c.b3[sl ^ pl] : c.b1[sl ^ pr] * c.b3[sr ^ pr] * c.b3[sl ^ pl]) *
-                c.g;
+template <class T, int S>
+__device__ __forceinline__ void slot_to_vec(const T (&v)[S], typename SlotT<T, S>::V (&raw)[SlotT<T, S>::kVecs]) {
+  if constexpr (std::is_same<T, dfloat>::value) {
+    float* f = reinterpret_cast<float*>(raw);
+#pragma unroll
+    for (int q = 0; q < S; ++q) {
+      f[q] = v[q].hi;
+      f[S + q] = v[q].lo;
     }
   } else {
-    for (int k = threadIdx.x; k < 4; k += blockDim.x) {
-      const int sv = k >> 1, q = k & 1;
-      wrow[k] = c.b2[sv ^ q];
-      urow[k] = c.b1[sv ^ q] * c.g;  // q is a here
-    }
-  }
-  // native FP64 (bound by the FP64 pipe): z_f[s'] u[a'][s'] for all four f
-  // from a table, one multiply per output fewer
-  constexpr bool kZuTable = ZB && std::is_same<T, double>::value;
-  __shared__ __align__(16) T zutab[kZuTable ? 64 : 1];
-  if constexpr (kZuTable) {
-    for (int k = threadIdx.x; k < 64; k += blockDim.x) {
-      const int f = k >> 4, sv = (k >> 2) & 3, aux = k & 3;
-      const int fl = f >> 1, fr = f & 1, sl = sv >> 1, sr = sv & 1, pl = aux >> 1, pr = aux & 1;
-      T z = c.b2[sr ^ fr] * c.b2[sl ^ fl];
-      if (dir) z = z * c.b1[sl ^ fr];
-      const T u = (!dir ? c.b1[sr ^ pl] * c.b3[sr ^ pr] * c.b3[sl ^ pl] : c.b1[sl ^ pr] * c.b3[sr ^ pr] * c.b3[sl ^ pl]) * c.g;
-      zutab[k] = z * u;
-    }
-  }
-  // double-float BNNNI: the steps run on packed lanes (aux pairs); z_f u
-  // for all four f and the weights, split into hi / lo planes (the weights
-  // duplicated across the two lanes, with the negated hi word)
-  constexpr bool kPacked = ZB && std::is_same<T, dfloat>::value;
-  __shared__ __align__(16) float zuh[kPacked ? 64 : 1], zul[kPacked ? 64 : 1];
-  __shared__ __align__(16) float2 wph[kPacked ? 16 : 1], wpl[kPacked ? 16 : 1], wpn[kPacked ? 16 : 1];
-  if constexpr (kPacked) {
-    // (from the coefficients, as urow and wrow are formed: those rows are
-    // written by other threads and read only after the tile barrier)
-    for (int k = threadIdx.x; k < 64; k += blockDim.x) {
-      const int f = k >> 4, sv = (k >> 2) & 3, aux = k & 3;
-      const int fl = f >> 1, fr = f & 1, sl = sv >> 1, sr = sv & 1, pl = aux >> 1, pr = aux & 1;
-      const T u = (!dir ? c.b1[sr ^ pl] * c.b3[sr ^ pr] * c.b3[sl ^ pl] : c.b1[sl ^ pr] * c.b3[sr ^ pr] * c.b3[sl ^ pl]) *
-                  c.g;
-      T z = c.b2[sr ^ fr] * c.b2[sl ^ fl];
-      if (dir) z = z * c.b1[sl ^ fr];
-      const T zu = u * z;
-      zuh[k] = zu.hi;
-      zul[k] = zu.lo;
-    }
-    for (int k = threadIdx.x; k < 16; k += blockDim.x) {
-      const int sv = k >> 2, q = k & 3, sl = sv >> 1, sr = sv & 1, al = q >> 1, ar = q & 1;
-      const T w = !dir ? c.b1[sr ^ al] * c.b2[sr ^ ar] * c.b2[sl ^ al] : c.b2[sr ^ ar] * c.b2[sl ^ al];
-      wph[k] = make_float2(w.hi, w.hi);
-      wpl[k] = make_float2(w.lo, w.lo);
-      wpn[k] = make_float2(-w.hi, -w.hi);
-    }
-  }
-  // the factors z selects from, in registers (no indexed access)
-  const T b1_0 = c.b1[0], b1_1 = c.b1[1], b2_0 = c.b2[0], b2_1 = c.b2[1];
-  // outer index: state bits, then (unless last) the lastbit pass
-  const uint64_t ob = blk & ((1ull << cp.no) - 1);
-  const int lb_outer = (int)(blk >> cp.no);
-  const uint64_t rbase = dep(ob, cp.opos, cp.no);
-  const int site0 = KS * cp.t0;  // lowest site of the pass's steps
-  const int nloop = cp.last ? cp.nlb : 1;
-  if (cp.last)
-    for (int e = threadIdx.x; e < (tile >> NA); e += blockDim.x) acc[e] = 0.0;
-  // The aux bits and the cb low sites are contiguous in HBM, so a pass with
-  // 2^(NA + cb) >= VEC elements per run moves whole 16-byte chunks (VEC
-  // consecutive tile elements sit in consecutive padded slots: VEC divides 32).
-  constexpr int VEC = 16 / (int)sizeof(T);
-  const bool vec_io = (1 << (NA + cp.jbit0)) >= VEC;
-  for (int li = 0; li < nloop; ++li) {
-    const int lb = cp.last ? li : lb_outer;
-    // load / build the tile
-    if (!cp.first && vec_io) {
-      for (int e = threadIdx.x * VEC; e < tile; e += blockDim.x * VEC) {
-        const uint64_t r = rbase | tile_state((uint64_t)(e >> NA), cp.jbit0, site0);
-        const uint64_t at = (((uint64_t)lb << L | r) << NA) | (uint64_t)(e & ((1 << NA) - 1));
-        const uint4 raw = __ldcs(reinterpret_cast<const uint4*>(P + at));
-        const T* v = reinterpret_cast<const T*>(&raw);
-        T* dst = sm + spad(e);
+    T* e = reinterpret_cast<T*>(raw);
 #pragma unroll
-        for (int k = 0; k < VEC; ++k) dst[k] = v[k];
+    for (int q = 0; q < S; ++q) e[q] = v[q];
+  }
+}
+
+template <class T, int S>
+__device__ __forceinline__ void slot_ld(unsigned char* sm, int plane, int i, T (&v)[S]) {
+  typename SlotT<T, S>::V raw[SlotT<T, S>::kVecs];
+#pragma unroll
+  for (int k = 0; k < SlotT<T, S>::kVecs; ++k) raw[k] = *slot_vec<T, S>(sm, plane, i, k);
+  vec_to_slot<T, S>(raw, v);
+}
+
+template <class T, int S>
+__device__ __forceinline__ void slot_st(unsigned char* sm, int plane, int i, const T (&v)[S]) {
+  typename SlotT<T, S>::V raw[SlotT<T, S>::kVecs];
+  slot_to_vec<T, S>(v, raw);
+#pragma unroll
+  for (int k = 0; k < SlotT<T, S>::kVecs; ++k) *slot_vec<T, S>(sm, plane, i, k) = raw[k];
+}
+
+// ------------------------------------------------------------------ steps
+// DNNI: RL consecutive letters (top first) of a thread's 2^RL slots.  The
+// letter after each is the next one of the group, or `ctl` after the last.
+template <class T, int RL>
+__device__ __forceinline__ void dnni_steps(T (&v)[1 << RL][2], const ChainTab<T>& tab, int ctl) {
+  const T rho = tab.rho1;
+#pragma unroll
+  for (int j = 0; j < RL; ++j) {
+    const int bit = 1 << (RL - 1 - j);
+#pragma unroll
+    for (int w = 0; w < (1 << RL); ++w) {
+      if (w & bit) continue;
+      const int c = (j < RL - 1) ? ((w >> (RL - 2 - j)) & 1) : ctl;
+      const T* z = tab.zu + c * 4;
+      T in[2][2];
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        in[0][q] = v[w][q];
+        in[1][q] = v[w | bit][q];
       }
-    } else {
-      for (int e = threadIdx.x; e < tile; e += blockDim.x) {
-        const int aux = e & ((1 << NA) - 1);
-        const uint64_t r = rbase | tile_state((uint64_t)(e >> NA), cp.jbit0, site0);
-        T v;
-        if (cp.first)
-          v = chain_init<T, ZB, IO>(x, pre, smap, L, bc, r, aux, lb, c);
-        else
-          v = P[(((uint64_t)lb << L | r) << NA) | (uint64_t)aux];
-        sm[spad(e)] = v;
+#pragma unroll
+      for (int a = 0; a < 2; ++a) {
+        v[w][a] = z[a] * xpry(rho, in[a][1], in[a][0]);
+        v[w | bit][a] = z[2 + a] * xpry(rho, in[a][0], in[a][1]);
       }
     }
-    __syncthreads();
-    for (int j = 0; j < cp.T; ++j) {
-      const int t = cp.t0 + j;
-      const int sb = NA + cp.jbit0 + KS * j;  // tile bit of the step's lowest site
-      const bool lastst = (t == nsteps - 1);
-      const int groups = tile >> GB;
-      // Slot of (group base, aux q, step sites sp): spad(ebase) + q +
-      // spad(sp << sb), since spad(a | b) = spad(a) + spad(b) for disjoint
-      // a, b and q < 4 never reaches bit 5 of an aux-aligned base.
-      const int o1 = spad(1 << sb), o2 = ZB ? spad(2 << sb) : 0, o3 = ZB ? spad(3 << sb) : 0;
-      // The control sites (the next step's sites) are tile bits [sb + KS,
-      // sb + 2 KS) unless this is the pass's last step; then they are outer
-      // bits of the block, or the lastbit pass at the product's last step.
-      const bool ctl_in_tile = (j + 1 < cp.T);
-      const int ctl_outer = lastst ? (ZB ? lb : (bc == 0 ? lb : 0))
-                                   : (int)((rbase >> (KS * t + KS)) & (uint64_t)((1 << KS) - 1));
-      for (int gi = threadIdx.x; gi < groups; gi += blockDim.x) {
-        // tile index of the group base: insert zeros at [0, NA) and [sb, sb+KS)
-        const int lo = gi & ((1 << (sb - NA)) - 1);
-        const int hi = gi >> (sb - NA);
-        const int ebase = (hi << (sb + KS)) | (lo << NA);
-        const int ctl = ctl_in_tile ? ((ebase >> (sb + KS)) & ((1 << KS) - 1)) : ctl_outer;
-        T* b0 = sm + spad(ebase);
-        // an offset the compiler cannot see through: the coefficient rows are
-        // re-read (broadcast) per group instead of held in registers across
-        // the loop, which would leave too few for the group's values
-        int z0 = 0;
-        asm volatile("" : "+r"(z0));
-        const T* wr = wrow + z0;
-        const T* ur = urow + z0;
-        if (!ZB) {
-          // DNNI: out(a, s) = b1[s^a] b2[nb^s] (b2[s] in(0, a) + b2[s^1] in(1, a)),
-          // in(q, s') = value with aux q and site t = s'
-          const int nb = ctl;
-          T* b1p = b0 + o1;
-          T in[2][2];
+  }
+}
+
+// BNNNI: one letter; v[a'][q] in, v[s'][a'] out
+template <class T>
+__device__ __forceinline__ void bnnni_step(T (&v)[4][4], const ChainTab<T>& tab, int ctl) {
+  T out[4][4];
 #pragma unroll
-          for (int q = 0; q < 2; ++q) {
-            in[q][0] = b0[q];
-            in[q][1] = b1p[q];
-          }
+  for (int a = 0; a < 4; ++a) {
+    const T* z = tab.zu + ctl * 16 + a * 4;
+    T t[2][2];
 #pragma unroll
-          for (int sv = 0; sv < 2; ++sv) {
-            const T z = (nb ^ sv) ? b2_1 : b2_0;
-            const T w0 = wr[sv * 2], w1 = wr[sv * 2 + 1];
-            T* bo = sv ? b1p : b0;
+    for (int qr = 0; qr < 2; ++qr) {
+      t[0][qr] = xpry(tab.rho1, v[a][2 + qr], v[a][qr]);
+      t[1][qr] = xpry(tab.rho1, v[a][qr], v[a][2 + qr]);
+    }
 #pragma unroll
-            for (int a = 0; a < 2; ++a) bo[a] = (ur[sv * 2 + a] * z) * mad_t(w1, in[1][a], w0 * in[0][a]);
-          }
+    for (int sv = 0; sv < 4; ++sv) out[sv][a] = z[sv] * xpry(tab.rho2[sv], t[sv >> 1][1], t[sv >> 1][0]);
+  }
+#pragma unroll
+  for (int sv = 0; sv < 4; ++sv)
+#pragma unroll
+    for (int a = 0; a < 4; ++a) v[sv][a] = out[sv][a];
+}
+
+// Shared-memory step tables of a block: the ChainTab, and for double-float
+// BNNNI also its planar form for the packed lanes.
+template <class T>
+struct ChainSh {
+  ChainTab<T> tab;
+  T two[64];  // first pass: zu[c][s', a'] w1[s'][lb] of the second step, [c][s'][a']
+};
+struct ChainShDF {
+  ChainTab<dfloat> tab;
+  dfloat two[64];
+  float2 zh[32], zl[32];  // [c][a'][s' pair]
+  float2 r2h[2], r2l[2];  // [sl]: (sr = 0, 1)
+};
+
+// bnnni_step on the packed FP32 lanes: the two-term sums over ql pair the
+// values of qr, those over qr pair the results of sr.  31 packed operations
+// per output pair, as the scalar sequence would take per output.
+__device__ __forceinline__ void bnnni_step_df(float4 (&h)[4], float4 (&l)[4], const ChainShDF& sh, int ctl) {
+  const dfloat r1 = sh.tab.rho1;
+  const float2 rh = make_float2(r1.hi, r1.hi), rl = make_float2(r1.lo, r1.lo), rn = make_float2(-r1.hi, -r1.hi);
+  float oh[4][4], ol[4][4];  // [s'][a']
+#pragma unroll
+  for (int a = 0; a < 4; ++a) {
+    const float2 h0 = make_float2(h[a].x, h[a].y), h1 = make_float2(h[a].z, h[a].w);
+    const float2 l0 = make_float2(l[a].x, l[a].y), l1 = make_float2(l[a].z, l[a].w);
+    float2 th[2], tl[2];
+    df2_fma_unnorm(rh, rl, rn, h1, l1, h0, l0, th[0], tl[0]);
+    df2_fma_unnorm(rh, rl, rn, h0, l0, h1, l1, th[1], tl[1]);
+#pragma unroll
+    for (int sl = 0; sl < 2; ++sl) {
+      const float2 qh = sh.r2h[sl], ql = sh.r2l[sl];
+      float2 dh, dl;
+      df2_fma_unnorm(qh, ql, make_float2(-qh.x, -qh.y), make_float2(th[sl].y, th[sl].y),
+                     make_float2(tl[sl].y, tl[sl].y), make_float2(th[sl].x, th[sl].x),
+                     make_float2(tl[sl].x, tl[sl].x), dh, dl);
+      const int k = ctl * 8 + a * 2 + sl;
+      float2 ph, pl;
+      df2_mul(dh, dl, sh.zh[k], sh.zl[k], ph, pl);
+      oh[2 * sl][a] = ph.x;
+      oh[2 * sl + 1][a] = ph.y;
+      ol[2 * sl][a] = pl.x;
+      ol[2 * sl + 1][a] = pl.y;
+    }
+  }
+#pragma unroll
+  for (int sv = 0; sv < 4; ++sv) {
+    h[sv] = make_float4(oh[sv][0], oh[sv][1], oh[sv][2], oh[sv][3]);
+    l[sv] = make_float4(ol[sv][0], ol[sv][1], ol[sv][2], ol[sv][3]);
+  }
+}
+
+template <class T, int KS>
+using ChainShared = typename std::conditional<std::is_same<T, dfloat>::value && KS == 2, ChainShDF, ChainSh<T>>::type;
+
+// the block's step tables from global (or parameter) memory
+template <class T, int KS>
+__device__ __forceinline__ void chain_tables(ChainShared<T, KS>& sh, const ChainTab<T>& tab) {
+  constexpr int n = (int)(sizeof(ChainTab<T>) / 4);
+  for (int k = threadIdx.x; k < n; k += blockDim.x)
+    reinterpret_cast<uint32_t*>(&sh.tab)[k] = reinterpret_cast<const uint32_t*>(&tab)[k];
+  if constexpr (std::is_same<T, dfloat>::value && KS == 2) {
+    for (int k = threadIdx.x; k < 32; k += blockDim.x) {
+      const dfloat a = tab.zu[2 * k], b = tab.zu[2 * k + 1];
+      sh.zh[k] = make_float2(a.hi, b.hi);
+      sh.zl[k] = make_float2(a.lo, b.lo);
+    }
+    for (int k = threadIdx.x; k < 2; k += blockDim.x) {
+      const dfloat a = tab.rho2[2 * k], b = tab.rho2[2 * k + 1];
+      sh.r2h[k] = make_float2(a.hi, b.hi);
+      sh.r2l[k] = make_float2(a.lo, b.lo);
+    }
+  }
+}
+
+// Buffers of one product.
+template <class T, class IO>
+struct ChainIO {
+  const T* src;        // previous pass's output
+  T* dst;              // this pass's output
+  const typename ChainIn<T>::U* u;  // first pass: input times Tvec, or null:
+  const IO* x;         //   x[r] * pre[r]
+  const double* pre;
+  const uint32_t* smap;  // reduced: state -> row of u
+  IO* y;               // last pass
+  const double* tv;    //   y = sum * tv [* dup] * post
+  const uint16_t* dup;
+  ScaleF post;
+};
+
+// letters per round held in registers
+template <class T, int KS>
+struct RoundLetters {
+  static constexpr int value = (KS == 2) ? 1 : (sizeof(T) == 4 ? 3 : (sizeof(T) == 8 ? 2 : 1));
+};
+
+// What a round needs beside the tile.
+template <class T, class IO>
+struct RoundArgs {
+  const ChainIO<T, IO>* io;
+  uint64_t src0, dst0;   // slots: (lb, node) base of the source (lb: last passes add it) and destination
+  uint64_t src_lb;       // slots per lastbit value in the source (last passes)
+  uint64_t out0;         // first child node of the tile (full operators)
+  uint64_t low0;         // the block's outer old bits
+  int end_ctl;           // letter after the product's last one (-1: the lastbit value)
+  const uint2* nodes;    // tree: the round's nodes (children known), or null
+};
+
+enum { kRoundIn = 1, kRoundOut = 2 };
+
+// One round on RL letters from depth d of the pass; the words of depth d are
+// nodes [0, cnt) from `words` (full operators: 0 .. cnt - 1).  IN: the slots
+// come straight from the previous pass's buffer; OUT: they go straight to this
+// pass's buffer; otherwise both stay in the shared-memory tile.  A pass's
+// first and last rounds skip it that way: one write and one read of the
+// traffic through shared memory, which with the instructions that move it
+// bounds the FP32 passes, are saved at each end (the second DNNI pass at
+// L = 26 took 0.61 ms with the tile at both ends, 0.53 ms so).  The last pass
+// keeps the tile for its sums: summed in registers and over lanes, with
+// strided outputs, it took 1.03 ms against 0.86 ms.
+template <class T, int KS, int RL, int IOF, class IO>
+__device__ __forceinline__ void chain_round(unsigned char* sm, int plane, const ChainShared<T, KS>& sh,
+                                            const ChainPass& cp, int d, const uint16_t* __restrict__ words, int cnt,
+                                            const RoundArgs<T, IO>& A) {
+  constexpr int S = 1 << KS, W = 1 << (KS * RL);
+  using V = typename SlotT<T, S>::V;
+  constexpr int kVecs = SlotT<T, S>::kVecs;
+  constexpr bool kPacked = std::is_same<T, dfloat>::value && KS == 2;
+  const int bl = KS * (cp.T - d - RL) + cp.tb;  // tile bits below the round's letters
+  const int wmask = (1 << (KS * d)) - 1, tmask = (1 << cp.tb) - 1;
+  const bool inside = d + RL < cp.T;
+  const int total = cnt << bl;
+  // (whole lastbit groups stay together: total is a multiple of 2^tb)
+  for (int gi = threadIdx.x; gi < total; gi += blockDim.x) {
+    const int pi = gi >> bl, lo = gi & ((1 << bl) - 1);
+    const int p = words ? ((int)__ldg(words + pi) & wmask) : pi;
+    const int base = (p << (KS * RL + bl)) | lo;
+    int ctl;
+    if (inside)
+      ctl = (lo >> (bl - KS)) & (S - 1);
+    else if (cp.last)
+      ctl = A.end_ctl < 0 ? lo & (S - 1) : A.end_ctl;
+    else
+      ctl = (int)((A.low0 | (uint64_t)(lo & tmask)) >> (cp.rest - KS)) & (S - 1);
+    T v[W][S];
+    float4 h[4], l[4];
+    if constexpr ((IOF & kRoundIn) != 0) {
+      const uint64_t at = A.src0 + ((uint64_t)(lo >> cp.tb) << cp.rest) +
+                          (cp.last ? (uint64_t)(lo & tmask) * A.src_lb : (uint64_t)(lo & tmask));
+      const V* src = reinterpret_cast<const V*>(A.io->src) + at * kVecs;
+      const int sh_w = KS * (cp.T - RL) + cp.rest;  // (d = 0)
+#pragma unroll
+      for (int w = 0; w < W; ++w) {
+        const V* q = src + (((uint64_t)w << sh_w) * kVecs);
+        if constexpr (kPacked) {
+          h[w] = *reinterpret_cast<const float4*>(q);
+          l[w] = *reinterpret_cast<const float4*>(q + 1);
         } else {
-          // BNNNI: out((pl,pr), (sl,sr)) = z_f[s'] u[a'][s'] sum_q w[s'][q] in(q, a')
-          const int fl = ctl >> 1, fr = ctl & 1;
-          T* const bp[4] = {b0, b0 + o1, b0 + o2, b0 + o3};
-          if constexpr (kPacked) {
-            // lanes: a' = 2 pp and 2 pp + 1
-            float2 ih[4][2], il[4][2];
+          V raw[kVecs];
 #pragma unroll
-            for (int q = 0; q < 4; ++q)
-#pragma unroll
-              for (int pp = 0; pp < 2; ++pp) {
-                const float* e0 = reinterpret_cast<const float*>(bp[2 * pp] + q);
-                const float* e1 = reinterpret_cast<const float*>(bp[2 * pp + 1] + q);
-                ih[q][pp] = make_float2(e0[0], e1[0]);
-                il[q][pp] = make_float2(e0[1], e1[1]);
-              }
-#pragma unroll
-            for (int sv = 0; sv < NS; ++sv) {
-              const int kw = sv * 4 + z0;
-#pragma unroll
-              for (int pp = 0; pp < 2; ++pp) {
-                float2 dh, dl;
-                df2_mul(ih[0][pp], il[0][pp], wph[kw], wpl[kw], wpn[kw], dh, dl);
-#pragma unroll
-                for (int q = 1; q < 4; ++q)
-                  df2_fma(ih[q][pp], il[q][pp], wph[kw + q], wpl[kw + q], wpn[kw + q], dh, dl, dh, dl);
-                const int kz = ctl * 16 + sv * 4 + 2 * pp + z0;
-                const float2 zh = *reinterpret_cast<const float2*>(zuh + kz);
-                const float2 zl = *reinterpret_cast<const float2*>(zul + kz);
-                // zu * d (operator* with zu first): the d operand is the one negated
-                float2 oh, ol;
-                df2_mul(zh, zl, dh, dl, make_float2(-dh.x, -dh.y), oh, ol);
-                float* o0 = reinterpret_cast<float*>(bp[sv] + 2 * pp);
-                o0[0] = oh.x;
-                o0[1] = ol.x;
-                o0[2] = oh.y;
-                o0[3] = ol.y;
-              }
-            }
-            continue;
-          }
-          T in[4][4];
-#pragma unroll
-          for (int q = 0; q < 4; ++q)
-#pragma unroll
-            for (int sp = 0; sp < 4; ++sp) in[q][sp] = bp[sp][q];
-          // every input is read before any output is written, so each output
-          // is stored as soon as it is formed (fewer live registers)
-#pragma unroll
-          for (int sv = 0; sv < NS; ++sv) {
-            const int sl = sv >> 1, sr = sv & 1;
-            const T w0 = wr[sv * 4], w1 = wr[sv * 4 + 1], w2 = wr[sv * 4 + 2], w3 = wr[sv * 4 + 3];
-            if constexpr (kZuTable) {
-              const T* zu = zutab + ctl * 16 + sv * 4 + z0;
-#pragma unroll
-              for (int aux = 0; aux < 4; ++aux) {
-                T d = in[0][aux] * w0;
-                d = mad_t(in[1][aux], w1, d);
-                d = mad_t(in[2][aux], w2, d);
-                d = mad_t(in[3][aux], w3, d);
-                bp[sv][aux] = zu[aux] * d;
-              }
-            } else {
-              T z = ((sr ^ fr) ? b2_1 : b2_0) * ((sl ^ fl) ? b2_1 : b2_0);
-              if (dir) z = z * ((sl ^ fr) ? b1_1 : b1_0);
-#pragma unroll
-              for (int aux = 0; aux < 4; ++aux) {
-                T d = in[0][aux] * w0;
-                d = mad_t(in[1][aux], w1, d);
-                d = mad_t(in[2][aux], w2, d);
-                d = mad_t(in[3][aux], w3, d);
-                bp[sv][aux] = (ur[sv * 4 + aux] * z) * d;
-              }
-            }
-          }
+          for (int k = 0; k < kVecs; ++k) raw[k] = q[k];
+          vec_to_slot<T, S>(raw, v[w]);
         }
       }
-      __syncthreads();
-    }
-    if (cp.last) {
-      for (int e = threadIdx.x; e < (tile >> NA); e += blockDim.x) {
-        double a = acc[e];
+    } else {
 #pragma unroll
-        for (int aux = 0; aux < (1 << NA); ++aux) a += fold_part(sm[spad((e << NA) | aux)]);
-        acc[e] = a;
+      for (int w = 0; w < W; ++w) {
+        if constexpr (kPacked) {
+          h[w] = *reinterpret_cast<const float4*>(slot_vec<T, 4>(sm, plane, base | (w << bl), 0));
+          l[w] = *reinterpret_cast<const float4*>(slot_vec<T, 4>(sm, plane, base | (w << bl), 1));
+        } else {
+          slot_ld<T, S>(sm, plane, base | (w << bl), v[w]);
+        }
       }
-    } else if (vec_io) {
-      for (int e = threadIdx.x * VEC; e < tile; e += blockDim.x * VEC) {
-        const uint64_t r = rbase | tile_state((uint64_t)(e >> NA), cp.jbit0, site0);
-        uint4 raw;
-        T* v = reinterpret_cast<T*>(&raw);
-        const T* src = sm + spad(e);
+    }
+    if constexpr (kPacked)
+      bnnni_step_df(h, l, sh, ctl);
+    else if constexpr (KS == 1)
+      dnni_steps<T, RL>(v, sh.tab, ctl);
+    else
+      bnnni_step<T>(v, sh.tab, ctl);
+    if constexpr ((IOF & kRoundOut) != 0) {
+      // bl = tb here; the children of word p: consecutive in a full operator,
+      // those of its mask in a tree (one letter per round)
+      uint2 nd = make_uint2(0u, ~0u);
+      if (A.nodes) nd = __ldg(A.nodes + pi);
+      const uint64_t first = A.nodes ? (uint64_t)nd.x : A.out0 + ((uint64_t)p << (KS * RL));
 #pragma unroll
-        for (int k = 0; k < VEC; ++k) v[k] = src[k];
-        const uint64_t at = (((uint64_t)lb << L | r) << NA) | (uint64_t)(e & ((1 << NA) - 1));
-        __stcs(reinterpret_cast<uint4*>(P + at), raw);
+      for (int w = 0; w < W; ++w) {
+        if (!((nd.y >> w) & 1u)) continue;
+        const uint64_t child = first + (A.nodes ? (uint64_t)__popc(nd.y & ((1u << w) - 1u)) : (uint64_t)w);
+        V* q = reinterpret_cast<V*>(A.io->dst) + (A.dst0 + (child << cp.rest) + (uint64_t)(lo & tmask)) * kVecs;
+        if constexpr (kPacked) {
+          *reinterpret_cast<float4*>(q) = h[w];
+          *reinterpret_cast<float4*>(q + 1) = l[w];
+        } else {
+          V raw[kVecs];
+          slot_to_vec<T, S>(v[w], raw);
+#pragma unroll
+          for (int k = 0; k < kVecs; ++k) q[k] = raw[k];
+        }
       }
     } else {
-      for (int e = threadIdx.x; e < tile; e += blockDim.x) {
-        const uint64_t r = rbase | tile_state((uint64_t)(e >> NA), cp.jbit0, site0);
-        P[(((uint64_t)lb << L | r) << NA) | (uint64_t)(e & ((1 << NA) - 1))] = sm[spad(e)];
+#pragma unroll
+      for (int w = 0; w < W; ++w) {
+        if constexpr (kPacked) {
+          *reinterpret_cast<float4*>(slot_vec<T, 4>(sm, plane, base | (w << bl), 0)) = h[w];
+          *reinterpret_cast<float4*>(slot_vec<T, 4>(sm, plane, base | (w << bl), 1)) = l[w];
+        } else {
+          slot_st<T, S>(sm, plane, base | (w << bl), v[w]);
+        }
       }
     }
-    __syncthreads();
   }
-  if (cp.last) {
-    for (int e = threadIdx.x; e < (tile >> NA); e += blockDim.x) {
-      const uint64_t r = rbase | tile_state((uint64_t)e, cp.jbit0, site0);
-      double v = acc[e];
-      if (post) v *= post[r];
-      y[r] = (IO)(v * postc);
+  if constexpr ((IOF & kRoundOut) == 0) __syncthreads();
+}
+
+// a round of RL letters or the fewer that are left, by where its slots are
+template <class T, int KS, int RL, class IO>
+__device__ __forceinline__ void chain_round_n(int n, int iof, unsigned char* sm, int plane,
+                                              const ChainShared<T, KS>& sh, const ChainPass& cp, int d,
+                                              const uint16_t* words, int cnt, const RoundArgs<T, IO>& A) {
+  if constexpr (RL > 1) {
+    if (n < RL) {
+      chain_round_n<T, KS, RL - 1, IO>(n, iof, sm, plane, sh, cp, d, words, cnt, A);
+      return;
+    }
+  }
+  switch (iof) {
+    case 0: chain_round<T, KS, RL, 0, IO>(sm, plane, sh, cp, d, words, cnt, A); break;
+    case 1: chain_round<T, KS, RL, 1, IO>(sm, plane, sh, cp, d, words, cnt, A); break;
+    case 2: chain_round<T, KS, RL, 2, IO>(sm, plane, sh, cp, d, words, cnt, A); break;
+    default: chain_round<T, KS, RL, 3, IO>(sm, plane, sh, cp, d, words, cnt, A); break;
+  }
+}
+
+constexpr int kChainMaxT = 16;  // letters of a pass
+
+// The first two steps of a closed ring applied to x.  After the first one the
+// carried letter of a state is its top letter (the lastbit value lb), so the
+// second step's sum has one term too:
+//   out(s'_0, s'_1; a' = a) = zu[c][s'_1, a] w1[s'_1][lb]
+//                             zu[a][s'_0, lb] w1[s'_0][q] x(lb, a, below)
+// with q the bottom letter and c the third.  A thread forms all words s'_0
+// s'_1 (those of the mask) of one `below` from its S states.  Against a first
+// step at the load and a full second step this took 0.31 of 1.01 ms off the
+// first BNNNI pass at L = 24 in double-float.
+template <class T, int KS, class IO>
+__device__ __forceinline__ void chain_first_two(unsigned char* sm, int plane, const ChainIO<T, IO>& io,
+                                                const ChainShared<T, KS>& sh, const ChainPass& cp, int L, int lb0,
+                                                uint64_t low0, uint32_t allowed) {
+  constexpr int S = 1 << KS;
+  const int fb = KS * (cp.T - 2) + cp.tb;
+  const int tmask = (1 << cp.tb) - 1;
+  // (small tiles: a thread per s'_0, so that all threads have work)
+  const bool split = (1 << fb) < (int)blockDim.x;
+  for (int item = threadIdx.x; item < (split ? S << fb : 1 << fb); item += blockDim.x) {
+    const int e = item & ((1 << fb) - 1);
+    const int lb = cp.last ? e & tmask : lb0;
+    const uint64_t below = ((uint64_t)(e >> cp.tb) << cp.rest) | (cp.last ? 0ull : low0 | (uint64_t)(e & tmask));
+    T x[S];
+    if (io.u) {
+      uint64_t at[S];
+#pragma unroll
+      for (int a = 0; a < S; ++a) {
+        const uint64_t r = ((uint64_t)lb << (L - KS)) | ((uint64_t)a << (L - 2 * KS)) | below;
+        at[a] = io.smap ? io.smap[r] : r;
+      }
+#pragma unroll
+      for (int a = 0; a < S; ++a) to_elem(io.u[at[a]], x[a]);
+    } else {
+#pragma unroll
+      for (int a = 0; a < S; ++a) {
+        const uint64_t r = ((uint64_t)lb << (L - KS)) | ((uint64_t)a << (L - 2 * KS)) | below;
+        weigh_in(io.x[r], io.pre[r], x[a]);
+      }
+    }
+    // (a ring of two letters: the bottom letter is the second, the third the first)
+    const bool two = L == 2 * KS;
+    const int c = two ? lb : (int)(below >> (L - 3 * KS)) & (S - 1);
+    for (int s0 = split ? item >> fb : 0; s0 < (split ? (item >> fb) + 1 : S); ++s0) {
+      if (!((allowed >> (s0 * S)) & ((1u << S) - 1u))) continue;
+      T xa[S];
+#pragma unroll
+      for (int a = 0; a < S; ++a) {
+        const int q = two ? a : (int)below & (S - 1);
+        xa[a] = sh.tab.zu[a * S * S + (KS == 1 ? s0 * S + lb : lb * S + s0)] * (sh.tab.w1[s0 * S + q] * x[a]);
+      }
+#pragma unroll
+      for (int s1 = 0; s1 < S; ++s1) {
+        if (!((allowed >> (s0 * S + s1)) & 1u)) continue;
+        T o[S];
+#pragma unroll
+        for (int a = 0; a < S; ++a) {
+          if (cp.last)
+            o[a] = sh.tab.zu[c * S * S + (KS == 1 ? s1 * S + a : a * S + s1)] * (sh.tab.w1[s1 * S + lb] * xa[a]);
+          else
+            o[a] = sh.two[c * S * S + s1 * S + a] * xa[a];
+        }
+        slot_st<T, S>(sm, plane, ((s0 * S + s1) << fb) | e, o);
+      }
     }
   }
 }
 
-template <class T, int ZB, class IO>
-__global__ void __launch_bounds__(256, (sizeof(T) == 4 ? 4 : (sizeof(T) == 8 ? 3 : 2))) chain_kernel(T* __restrict__ P, const IO* __restrict__ x,
-                                                    const double* __restrict__ pre, const uint32_t* __restrict__ smap,
-                                                    IO* __restrict__ y, const double* __restrict__ post, double postc,
-                                                    int L, int bc, int dir, AuxCoefT<T> c, ChainPass cp) {
-  chain_block<T, ZB, IO>(P, x, pre, smap, y, post, postc, L, bc, dir, c, cp, blockIdx.x);
+// One block of a pass (the tables in sh are loaded and synchronised).
+//   KS = 1: DNNI (permute_mult_T1 / _last, TMat/tmat.cpp:344-376); KS = 2:
+//   diagonal BNNNI (TMat/tmat.cpp:521-588).
+// bc: 0 closed ring; 5, 9: DNNI open boundaries (TMat/tmat.cpp:392-457), the
+// sites beyond the ends fixed to 0 (9: to 1 below site 0).
+template <class T, int KS, class IO>
+__device__ __forceinline__ void chain_block(const ChainIO<T, IO>& io, ChainShared<T, KS>& sh, const ChainPass& cp,
+                                            const TreeDev& tr, int L, int bc, uint64_t blk) {
+  constexpr int S = 1 << KS, RL = RoundLetters<T, KS>::value;
+  using Acc = typename FoldAcc<T>::A;
+  using V = typename SlotT<T, S>::V;
+  constexpr int kVecs = SlotT<T, S>::kVecs;
+  extern __shared__ __align__(16) unsigned char sm[];
+  const int wbits = KS * cp.T;
+  const int plane = slot_plane(1 << (wbits + cp.tb), SlotT<T, S>::kBytes);
+  __shared__ uint32_t rg0[kChainMaxT + 1], rgn[kChainMaxT + 1];
+  // block -> (lb, node, outer old bits)
+  const int ob = cp.rest - cp.cb;
+  const uint64_t low0 = (blk & ((1ull << ob) - 1)) << cp.cb;
+  const uint64_t nl = blk >> ob;
+  const int lb_outer = cp.last ? 0 : (int)(nl / (uint64_t)cp.nin);
+  const uint64_t node = nl - (uint64_t)lb_outer * (uint64_t)cp.nin;
+  const bool tree = tr.nodes != nullptr;
+  if (threadIdx.x == 0) {
+    // (one range per turn, written at the turn's end: with the first range
+    // written inside the loop and a break at its end, nvcc 13.0 stored the
+    // ranges of one instantiation one place too far)
+    uint32_t r0 = (uint32_t)node, r1 = r0 + 1;
+    rg0[0] = r0;
+    rgn[0] = 1;
+#pragma unroll 1
+    for (int j = 1; j <= cp.T; ++j) {
+      if (tree) {
+        const uint2* nd = tr.nodes + tr.off[cp.t0 + j - 1];
+        const uint2 a = nd[r0], b = nd[r1 - 1];
+        r0 = a.x;
+        r1 = b.x + __popc(b.y);
+      } else {
+        r0 = 0;
+        r1 = 1u << (KS * j);
+      }
+      rg0[j] = r0;
+      rgn[j] = r1 - r0;
+    }
+  }
+  const int tmask = (1 << cp.tb) - 1;
+  const bool two = cp.first && bc == 0 && cp.T >= (cp.last ? 3 : 2);
+  if (two) {
+    __shared__ uint32_t allowed;  // words of the first two letters
+    if (threadIdx.x == 0) {
+      uint32_t m = 0;
+      if (tree) {
+        const uint2 root = tr.nodes[tr.off[0]];
+        for (int s0 = 0, k = 0; s0 < S; ++s0)
+          if ((root.y >> s0) & 1u) m |= tr.nodes[tr.off[1] + root.x + k++].y << (s0 * S);
+      } else {
+        m = S == 4 ? 0xffffu : 0xfu;
+      }
+      allowed = m;
+    }
+    if (!cp.last)
+      for (int k = threadIdx.x; k < S * S * S; k += blockDim.x) {
+        const int c = k / (S * S), s1 = (k / S) % S, a = k % S;
+        sh.two[k] = sh.tab.zu[c * S * S + (KS == 1 ? s1 * S + a : a * S + s1)] * sh.tab.w1[s1 * S + lb_outer];
+      }
+    __syncthreads();
+    chain_first_two<T, KS, IO>(sm, plane, io, sh, cp, L, lb_outer, low0, allowed);
+  } else if (cp.first) {
+    // The first step applied to x: the carried letter of state r is its
+    // bottom letter, the ring's first old letter is its top one (closed: the
+    // lastbit value), which becomes the carried letter.  Two states per
+    // thread and turn, so that their gathers are in flight together.
+    const int fb = KS * (cp.T - 1) + cp.tb;  // tile bits below the first letter
+    constexpr int A0 = S;
+    for (int e0 = threadIdx.x; e0 < (1 << fb); e0 += 2 * blockDim.x) {
+      uint64_t below[2];
+      T v[2][A0];
+      const int na = bc == 0 ? 1 : S;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int e = e0 + h * (int)blockDim.x;
+        const int k = e & tmask;
+        below[h] = ((uint64_t)(e >> cp.tb) << cp.rest) | (cp.last ? 0ull : low0 | (uint64_t)k);
+      }
+      if (io.u) {
+        uint64_t at[2][A0];
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int a = 0; a < A0; ++a) {
+            const int e = e0 + h * (int)blockDim.x;
+            if (e < (1 << fb) && a < na) {
+              const int top = bc ? a : (cp.last ? e & tmask : lb_outer);
+              const uint64_t r = ((uint64_t)top << (L - KS)) | below[h];
+              at[h][a] = io.smap ? io.smap[r] : r;
+            }
+          }
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int a = 0; a < A0; ++a)
+            if (e0 + h * (int)blockDim.x < (1 << fb) && a < na) to_elem(io.u[at[h][a]], v[h][a]);
+      } else {
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int a = 0; a < A0; ++a) {
+            const int e = e0 + h * (int)blockDim.x;
+            if (e < (1 << fb) && a < na) {
+              const int top = bc ? a : (cp.last ? e & tmask : lb_outer);
+              const uint64_t r = ((uint64_t)top << (L - KS)) | below[h];
+              weigh_in(io.x[r], io.pre[r], v[h][a]);
+            }
+          }
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int e = e0 + h * (int)blockDim.x;
+        if (e >= (1 << fb)) break;
+        const int c = (int)(below[h] >> (L - 2 * KS)) & (S - 1);
+        const int lb = cp.last ? e & tmask : lb_outer;
+        int q = (int)(below[h] & (S - 1));
+        if (bc) {
+#pragma unroll
+          for (int a = 0; a < A0; ++a)
+            v[h][a] = v[h][a] * (sh.tab.b2[(int)(below[h] & 1) ^ (bc == 9)] * sh.tab.b2[a & 1]);
+          q = 0;
+        }
+#pragma unroll
+        for (int sv = 0; sv < S; ++sv) {
+          T o[S];
+          if (bc == 0) {
+            // (one product, then selects: all S carried letters' products
+            // would run, predicated or not)
+            const T z = sh.tab.zu[c * S * S + (KS == 1 ? sv * S + lb : lb * S + sv)] * (sh.tab.w1[sv * S + q] * v[h][0]);
+#pragma unroll
+            for (int a = 0; a < S; ++a) o[a] = (a == lb) ? z : T(0);
+          } else {
+#pragma unroll
+            for (int a = 0; a < S; ++a)
+              o[a] = sh.tab.zu[c * S * S + (KS == 1 ? sv * S + a : a * S + sv)] * (sh.tab.w1[sv * S + q] * v[h][a]);
+          }
+          slot_st<T, S>(sm, plane, (sv << fb) | e, o);
+        }
+      }
+    }
+  }
+  __syncthreads();
+  RoundArgs<T, IO> A;
+  A.io = &io;
+  A.src0 = (((uint64_t)lb_outer * cp.nin + node) << (cp.rest + wbits)) + low0;
+  A.src_lb = (uint64_t)cp.nin << (cp.rest + wbits);
+  A.dst0 = (((uint64_t)lb_outer * cp.nout) << cp.rest) + low0;
+  A.out0 = tree ? 0 : node << wbits;
+  A.low0 = low0;
+  A.end_ctl = bc == 0 ? -1 : (bc == 9 ? 1 : 0);
+  // a tree's children are looked up one letter at a time: its last round has
+  // one letter
+  const int d0 = two ? 2 : (cp.first ? 1 : 0);
+  for (int d = d0; d < cp.T;) {
+    const int left = cp.T - d;
+    int n = left < RL ? left : RL;
+    if (tree && !cp.last && n == left && n > 1) --n;
+    const bool out = !cp.last && d + n == cp.T;
+    const uint16_t* words = tree ? tr.words + tr.off[cp.t0 + d] + rg0[d] : nullptr;
+    A.nodes = (tree && out) ? tr.nodes + tr.off[cp.t0 + d] + rg0[d] : nullptr;
+    chain_round_n<T, KS, RL, IO>(n, (d == 0 ? kRoundIn : 0) | (out ? kRoundOut : 0), sm, plane, sh, cp, d, words,
+                                 (int)rgn[d], A);
+    d += n;
+  }
+  if (cp.last) {
+    const uint16_t* words = tree ? tr.words + tr.off[cp.t0 + cp.T] + rg0[cp.T] : nullptr;
+    const uint64_t out0 = tree ? rg0[cp.T] : node << wbits;
+    for (int i = threadIdx.x; i < (int)rgn[cp.T]; i += blockDim.x) {
+      const int w = words ? ((int)__ldg(words + i) & ((1 << wbits) - 1)) : i;
+      Acc acc = Acc(0);
+#pragma unroll
+      for (int t = 0; t < S; ++t) {
+        if (t > tmask) break;
+        T v[S];
+        slot_ld<T, S>(sm, plane, (w << cp.tb) | t, v);
+#pragma unroll
+        for (int q = 0; q < S; ++q) acc = fold_add(acc, v[q]);
+      }
+      const uint64_t r = out0 + i;
+      double t = io.tv[r];
+      if (io.dup) t *= (double)io.dup[r];
+      if constexpr (sizeof(IO) == 4)
+        io.y[r] = scale_round(acc, t, io.post);
+      else
+        io.y[r] = (double)acc * t * io.post.f64;
+    }
+  } else if (d0 == cp.T) {
+    // (a pass of the first letters alone: the tile goes out as it is)
+    const uint16_t* words = tree ? tr.words + tr.off[cp.t0 + cp.T] + rg0[cp.T] : nullptr;
+    const uint64_t out0 = tree ? rg0[cp.T] : node << wbits;
+    V* dst = reinterpret_cast<V*>(io.dst) + (A.dst0 + (out0 << cp.rest)) * kVecs;
+    for (int e = threadIdx.x; e < ((int)rgn[cp.T] << cp.cb) * kVecs; e += blockDim.x) {
+      const int i = e / kVecs, k = e % kVecs;
+      const int n = i >> cp.cb;
+      const int w = words ? ((int)__ldg(words + n) & ((1 << wbits) - 1)) : n;
+      const V raw = *slot_vec<T, S>(sm, plane, (w << cp.cb) | (i & tmask), k);
+      dst[(((uint64_t)n << cp.rest) | (uint64_t)(i & tmask)) * kVecs + k] = raw;
+    }
+  }
 }
 
-// ------------------------------------------------------------------ reduced contract
+// Measured at the sizes of the sweep and the full operators, against in-place
+// passes of all 2^L states with four multiply-adds and one multiply per
+// output: BNNNI (reduced) at L = 24 in double-float 10.1 -> 1.47 ms, DNNI
+// (full) at L = 26 in FP32 5.18 -> 2.03 ms.  What is left: the FP32 pipes
+// (45% busy in the first double-float pass) and, in FP32, memory (4.3 GB of
+// pass buffers at L = 26, 0.65 ms at the copy rate) behind shared-memory
+// round trips of three letters each.
 template <class T>
-__global__ void red_contract(const T* __restrict__ z, const uint32_t* __restrict__ idx, const uint16_t* __restrict__ dup,
-                             const double* __restrict__ tv, double post, T* __restrict__ y, int64_t n) {
+constexpr int chain_min_blocks() {
+  return sizeof(T) == 4 ? 4 : 2;
+}
+
+template <class T, int KS, class IO>
+__global__ void __launch_bounds__(256, chain_min_blocks<T>())
+    chain_kernel(const __grid_constant__ ChainIO<T, IO> io, const __grid_constant__ ChainTab<T> tab,
+                 const __grid_constant__ ChainPass cp, const __grid_constant__ TreeDev tr, int L, int bc) {
+  __shared__ __align__(16) ChainShared<T, KS> sh;
+  chain_tables<T, KS>(sh, tab);
+  __syncthreads();
+  chain_block<T, KS, IO>(io, sh, cp, tr, L, bc, blockIdx.x);
+}
+
+// u = x tvec in the product's arithmetic
+template <class U, class IO>
+__global__ void chain_scale_in(const IO* __restrict__ x, const double* __restrict__ tv, U* __restrict__ u, int64_t n) {
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t st = (int64_t)gridDim.x * blockDim.x;
-  for (; i < n; i += st) y[i] = (T)((double)z[idx[i]] * post * (double)dup[i] * tv[i]);
-}
-
-__device__ __forceinline__ int64_t chain_pass_blocks_dev(const ChainPass& cp) {
-  return (int64_t)(cp.last ? 1 : cp.nlb) << cp.no;
+  for (; i < n; i += st) {
+    U v;
+    weigh_in(x[i], tv[i], v);
+    u[i] = v;
+  }
 }
 
 // ------------------------------------------------------------------ batched product
-// One pass over every batch member's tiles: a block takes its member from the
-// per-block member map, then runs the same tile body as chain_kernel on
-// kBatchTiles consecutive tiles of that member's geometry (copied to shared
-// memory).  km[i] = (Krylov column the member extends, product mode).
-template <class T, int ZB, class IO, int MODE>
-__global__ void __launch_bounds__(256, (sizeof(T) == 4 ? 4 : (sizeof(T) == 8 ? 3 : 2)))
-    chain_batch_kernel(const ChainInst* __restrict__ inst, const int2* __restrict__ km, const int64_t* __restrict__ start,
-                       const int* __restrict__ bmem, int pass, int theta) {
-  __shared__ ChainPass cps;
-  const int s_i = bmem[blockIdx.x];  // the member of this block
-  const ChainInst& I = inst[s_i];
-  const int64_t blk = (int64_t)blockIdx.x - start[s_i];
-  const int np = (sizeof(T) == 4) ? I.np4 : (sizeof(T) == 8 ? I.np8 : I.np16);
-  const int2 kmi = km[s_i];
-  if (kmi.y != MODE || pass >= np) return;  // uniform over the block
-  const int j = kmi.x;
-  {
-    const int* src = reinterpret_cast<const int*>((sizeof(T) == 4) ? &I.p4[pass]
-                                                  : (sizeof(T) == 8 ? &I.p8[pass] : &I.p16[pass]));
-    int* dst = reinterpret_cast<int*>(&cps);
-    for (int q = threadIdx.x; q < (int)(sizeof(ChainPass) / sizeof(int)); q += blockDim.x) dst[q] = src[q];
-  }
-  __syncthreads();
-  const int64_t ntiles = chain_pass_blocks_dev(cps);
-  const IO* x = (MODE == kModeF32) ? reinterpret_cast<const IO*>(I.x32)
-                                   : reinterpret_cast<const IO*>(I.V + (int64_t)j * I.ldv);
-  const AuxCoefT<T>* c;
-  if constexpr (MODE == kModeF32)
-    c = reinterpret_cast<const AuxCoefT<T>*>(&I.c32);
-  else if constexpr (MODE == kModeDF)
-    c = reinterpret_cast<const AuxCoefT<T>*>(&I.cdf);
-  else if constexpr (MODE == kModeTangent)
-    c = reinterpret_cast<const AuxCoefT<T>*>(&I.ctan[theta]);
-  else
-    c = reinterpret_cast<const AuxCoefT<T>*>(&I.c64);
-  for (int q = 0; q < kBatchTiles; ++q) {
-    const int64_t tile = blk * kBatchTiles + q;
-    if (tile >= ntiles) break;  // uniform over the block
-    if (q) __syncthreads();     // the previous tile's last reads of shared memory
-    chain_block<T, ZB, IO>(reinterpret_cast<T*>(I.P), x, I.tvec, I.smap, reinterpret_cast<IO*>(I.fold), nullptr, 1.0,
-                           I.L, I.bc, I.dir, *c, cps, (uint64_t)tile);
-  }
-}
-
-// w[k] = fold[idx[k]] * gs * dup[k] * tvec[k] (reduced) or fold[k] * gs * nf *
-// tvec[k] (full), per member; kSweepRows rows per block
-template <class IO, int MODE>
-__global__ void __launch_bounds__(256) contract_batch_kernel(const ChainInst* __restrict__ inst,
-                                                             const int2* __restrict__ km,
-                                                             const int64_t* __restrict__ rstart,
-                                                             const int* __restrict__ rmem) {
+// u of every member in `MODE` (kSweepRows rows per block)
+template <class U, int MODE>
+__global__ void __launch_bounds__(256) chain_batch_scale_in(const ChainInst* __restrict__ inst,
+                                                            const int2* __restrict__ km,
+                                                            const int64_t* __restrict__ rstart,
+                                                            const int* __restrict__ rmem) {
   const int s_i = rmem[blockIdx.x];  // the member of this row block
   const ChainInst& I = inst[s_i];
   const int2 kmi = km[s_i];
   if (kmi.y != MODE) return;
   const int64_t r0 = ((int64_t)blockIdx.x - rstart[s_i]) * kSweepRows;
   const int64_t r1 = min(r0 + (int64_t)kSweepRows, I.n);
-  const double gs = (MODE == kModeF32) ? I.gs32 : (MODE == kModeF64 ? I.gs64 : I.gsdf);  // tangent steps as DF
-  const IO* z = reinterpret_cast<const IO*>(I.fold);
+  const double* x = I.V + (int64_t)kmi.x * I.ldv;
+  U* u = reinterpret_cast<U*>(I.u);
   for (int64_t r = r0 + threadIdx.x; r < r1; r += blockDim.x) {
-    const double f = I.idx ? (double)z[I.idx[r]] * (double)I.dup[r] : (double)z[r] * I.nf;
-    I.w[r] = f * gs * I.tvec[r];
+    U v;
+    weigh_in(x[r], I.tvec[r], v);
+    u[r] = v;
+  }
+}
+
+template <class T, int MODE>
+__device__ __forceinline__ const ChainTab<T>* inst_tab(const ChainInst& I, int theta) {
+  if constexpr (MODE == kModeF32)
+    return &I.c32;
+  else if constexpr (MODE == kModeDF)
+    return &I.cdf;
+  else if constexpr (MODE == kModeTangent)
+    return &I.ctan[theta];
+  else
+    return &I.c64;
+}
+
+// One pass over every batch member's tiles: a block takes its member from the
+// per-block member map, then runs the same tile body as chain_kernel on
+// kBatchTiles consecutive tiles of that member's geometry (copied to shared
+// memory).  km[i] = (Krylov column the member extends, product mode).
+template <class T, int KS, int MODE>
+__global__ void __launch_bounds__(256, chain_min_blocks<T>())
+    chain_batch_kernel(const ChainInst* __restrict__ inst, const int2* __restrict__ km, const int64_t* __restrict__ start,
+                       const int* __restrict__ bmem, int pass, int theta) {
+  __shared__ ChainPass cps;
+  __shared__ TreeDev trs;
+  __shared__ __align__(16) ChainShared<T, KS> sh;
+  const int s_i = bmem[blockIdx.x];  // the member of this block
+  const ChainInst& I = inst[s_i];
+  const int64_t blk = (int64_t)blockIdx.x - start[s_i];
+  const int np = (sizeof(T) == 4) ? I.np4 : (sizeof(T) == 8 ? I.np8 : I.np16);
+  const int2 kmi = km[s_i];
+  if (kmi.y != MODE || pass >= np) return;  // uniform over the block
+  auto copy = [](void* dst, const void* src, int bytes) {
+    for (int q = threadIdx.x; q < bytes / 4; q += blockDim.x)
+      reinterpret_cast<uint32_t*>(dst)[q] = reinterpret_cast<const uint32_t*>(src)[q];
+  };
+  copy(&cps, (sizeof(T) == 4) ? &I.p4[pass] : (sizeof(T) == 8 ? &I.p8[pass] : &I.p16[pass]), (int)sizeof(ChainPass));
+  copy(&trs, &I.tree, (int)sizeof(TreeDev));
+  chain_tables<T, KS>(sh, *inst_tab<T, MODE>(I, theta));
+  __syncthreads();
+  const int64_t ntiles = ((int64_t)(cps.last ? 1 : cps.nlb) * cps.nin) << (cps.rest - cps.cb);
+  ChainIO<T, double> io;
+  T* const buf[2] = {reinterpret_cast<T*>(I.P), reinterpret_cast<T*>(trs.nodes ? I.Q : I.P)};
+  io.src = buf[(pass + 1) & 1];
+  io.dst = buf[pass & 1];
+  io.u = reinterpret_cast<const typename ChainIn<T>::U*>(I.u);
+  io.x = nullptr;
+  io.pre = nullptr;
+  io.smap = I.smap;
+  io.y = I.w;
+  io.tv = I.tvec;
+  io.dup = I.dup;
+  const double gs = (MODE == kModeF32) ? I.gs32 : (MODE == kModeF64 ? I.gs64 : I.gsdf);  // tangent steps as DF
+  io.post.f64 = gs * I.nf;
+  for (int q = 0; q < kBatchTiles; ++q) {
+    const int64_t tile = blk * kBatchTiles + q;
+    if (tile >= ntiles) break;  // uniform over the block
+    if (q) __syncthreads();     // the previous tile's last reads of shared memory
+    chain_block<T, KS, double>(io, sh, cps, trs, I.L, I.bc, (uint64_t)tile);
   }
 }
 
@@ -533,35 +856,112 @@ AuxCoef coef_of(const Op& op) {
   return c;
 }
 
-// largest row sum of one sweep step (bound used to normalise FP32 steps)
-double step_bound(const Op& op, const AuxCoef& c, int dir) {
-  double best = 0.0;
-  const bool zb = (op.kind == K_ZBT || op.kind == K_ZBM);
+namespace {
+
+// value and derivative by one parameter (host)
+struct Dual {
+  double v = 0.0, d = 0.0;
+  Dual() {}
+  Dual(double v_, double d_ = 0.0) : v(v_), d(d_) {}
+};
+Dual operator*(Dual a, Dual b) { return Dual(a.v * b.v, a.d * b.v + a.v * b.d); }
+Dual operator/(Dual a, Dual b) { return Dual(a.v / b.v, (a.d - a.v / b.v * b.d) / b.v); }
+
+template <class T>
+T tab_elem(Dual x) {
+  if constexpr (std::is_same<T, tangent>::value)
+    return tangent(x.v, x.d);
+  else
+    return (T)x.v;
+}
+
+// The step tables (see ChainTab) from the factors b1 = e^{+-K}, b2 =
+// e^{-+K kappa}, b3 = e^{-+K kappa2} (TMat/tmat.cpp:344-376, 521-588) and
+// their derivatives; returns the largest row sum of a step, whose inverse
+// normalises the FP32 and double-float steps.  The ring is walked from the
+// top, so the carried letter q is the neighbour above and the control c the
+// one below: the reference's factors of the lower neighbour (dir 0: b1[sr^al]
+// b2[sr^ar] b2[sl^al]; dir 1: b2[sr^ar] b2[sl^al]) belong to c, those of the
+// upper one (dir 0: b2[sr^fr] b2[sl^fl]; dir 1: b1[sl^fr] b2[sr^fr]
+// b2[sl^fl]) to q.
+template <class T>
+double chain_tab(bool zb, int dir, const AuxCoef& c, const AuxCoef* dc, bool norm, ChainTab<T>& tab,
+                 double* bias = nullptr) {
+  Dual b1[2], b2[2], b3[2];
+  for (int k = 0; k < 2; ++k) {
+    b1[k] = Dual(c.b1[k], dc ? dc->b1[k] : 0.0);
+    b2[k] = Dual(c.b2[k], dc ? dc->b2[k] : 0.0);
+    b3[k] = Dual(c.b3[k], dc ? dc->b3[k] : 0.0);
+  }
+  const int S = zb ? 4 : 2;
+  Dual rho1 = b2[1] / b2[0], rho2[4], w1[16], zu[64];
   if (!zb) {
     for (int s = 0; s < 2; ++s)
-      for (int a = 0; a < 2; ++a)
-        for (int nb = 0; nb < 2; ++nb)
-          best = std::max(best, c.b1[s ^ a] * c.b2[nb ^ s] * (c.b2[s] + c.b2[s ^ 1]));
+      for (int q = 0; q < 2; ++q) {
+        w1[s * 2 + q] = (s == q) ? Dual(1.0) : rho1;
+        for (int k = 0; k < 2; ++k) zu[k * 4 + s * 2 + q] = b2[k ^ s] * b1[s ^ q] * b2[0];  // q is a' here
+      }
   } else {
-    for (int sl = 0; sl < 2; ++sl)
-      for (int sr = 0; sr < 2; ++sr)
-        for (int pl = 0; pl < 2; ++pl)
-          for (int pr = 0; pr < 2; ++pr)
-            for (int fl = 0; fl < 2; ++fl)
-              for (int fr = 0; fr < 2; ++fr) {
-                double v = !dir ? c.b1[sr ^ pl] * c.b2[sr ^ fr] * c.b2[sl ^ fl] * c.b3[sr ^ pr] * c.b3[sl ^ pl]
-                                : c.b1[sl ^ fr] * c.b1[sl ^ pr] * c.b2[sr ^ fr] * c.b2[sl ^ fl] * c.b3[sr ^ pr] *
-                                      c.b3[sl ^ pl];
-                double d = 0.0;
-                for (int q = 0; q < 4; ++q) {
-                  int al = q >> 1, ar = q & 1;
-                  d += !dir ? c.b1[sr ^ al] * c.b2[sr ^ ar] * c.b2[sl ^ al] : c.b2[sr ^ ar] * c.b2[sl ^ al];
-                }
-                best = std::max(best, v * d);
-              }
+    for (int s = 0; s < 4; ++s) {
+      const int sl = s >> 1, sr = s & 1;
+      Dual f = b2[0] * b2[sr];
+      rho2[s] = b2[sr ^ 1] / b2[sr];
+      if (dir) {
+        f = f * b1[sl];
+        rho2[s] = rho2[s] * b1[sl ^ 1] / b1[sl];
+      }
+      for (int q = 0; q < 4; ++q) {
+        const int ql = q >> 1, qr = q & 1;
+        w1[s * 4 + q] = (sl == ql ? Dual(1.0) : rho1) * (qr ? rho2[s] : Dual(1.0));
+        // q as a' = (pl, pr)
+        const Dual u = (dir ? b1[sl ^ qr] : b1[sr ^ ql]) * b3[sr ^ qr] * b3[sl ^ ql];
+        for (int k = 0; k < 4; ++k) {
+          const int cl = k >> 1, cr = k & 1;
+          const Dual z = dir ? b2[sr ^ cr] * b2[sl ^ cl] : b1[sr ^ cl] * b2[sr ^ cr] * b2[sl ^ cl];
+          zu[k * 16 + q * 4 + s] = z * u * f;
+        }
+      }
+    }
   }
-  return best;
+  double gb = 0.0;
+  for (int k = 0; k < S; ++k)
+    for (int s = 0; s < S; ++s) {
+      double sum = 0.0;
+      for (int q = 0; q < S; ++q) sum += w1[s * S + q].v;
+      for (int a = 0; a < S; ++a) gb = std::max(gb, zu[k * S * S + (zb ? a * S + s : s * S + a)].v * sum);
+    }
+  // What rounding the tables adds to a step, as the ratio of its exact to its
+  // rounded sum over all inputs and outputs: every step shares it, so the
+  // product's output factor takes it out (FP32: 3e-8 per entry, L of them).
+  const Dual g(norm ? 1.0 / gb : 1.0);
+  if (std::is_same<T, float>::value && bias) {
+    const float r1 = (float)rho1.v;
+    double exact = 0.0, rounded = 0.0;
+    for (int k = 0; k < S; ++k)
+      for (int s = 0; s < S; ++s) {
+        double se = 0.0, sr = 0.0;
+        for (int q = 0; q < S; ++q) {
+          se += w1[s * S + q].v;
+          sr += !zb ? (s == q ? 1.0 : (double)r1)
+                    : ((s >> 1) == (q >> 1) ? 1.0 : (double)r1) * ((q & 1) ? (double)(float)rho2[s].v : 1.0);
+        }
+        for (int a = 0; a < S; ++a) {
+          const double z = zu[k * S * S + (zb ? a * S + s : s * S + a)].v * g.v;
+          exact += z * se;
+          rounded += (double)(float)z * sr;
+        }
+      }
+    *bias = exact / rounded;
+  }
+  tab.rho1 = tab_elem<T>(rho1);
+  for (int k = 0; k < 4; ++k) tab.rho2[k] = tab_elem<T>(rho2[k]);
+  for (int k = 0; k < 2; ++k) tab.b2[k] = tab_elem<T>(b2[k]);
+  for (int k = 0; k < 16; ++k) tab.w1[k] = tab_elem<T>(w1[k]);
+  for (int k = 0; k < 64; ++k) tab.zu[k] = tab_elem<T>(zu[k] * g);
+  return gb;
 }
+
+}  // namespace
 
 // Batch members keep no product buffers of their own: the batch owns them.
 static thread_local bool g_batch_member = false;
@@ -570,14 +970,22 @@ BatchMemberScope::~BatchMemberScope() { g_batch_member = prev; }
 
 void build_aux(Op& op) {
   const int L = op.L;
-  const int64_t N = 1ll << L;
   const bool zb = (op.kind == K_ZBT || op.kind == K_ZBM);
+  const bool reduced = (op.kind == K_XDM || op.kind == K_ZBM);
   if (zb && L % 2) fail(TM_ERR_ARG, "diagonal BNNNI operators need an even width");
+  if (reduced) build_prefix_tree(op, L, std::vector<int>(zb ? L / 2 : L, zb ? 2 : 1), true, op.tree);
   if (g_batch_member) return;
-  // one in-place pass buffer of nlb * 2^NA * 2^L elements (FP64 size)
-  const int64_t per = zb ? 16 * N : 4 * N;
-  op.ws_a.alloc((size_t)per * 8);
-  if (op.kind == K_XDM || op.kind == K_ZBM) op.xp.alloc((size_t)N * 8);  // full-space result before contraction
+  // the two pass buffers of any plan the tuning table can choose
+  int64_t most[2] = {1, 1};
+  for (size_t elem : {(size_t)4, (size_t)8})
+    for (int tb = 10; tb <= (elem == 8 ? 13 : 14); ++tb) {
+      int64_t need[2];
+      chain_buffer_elems(op, chain_plan(op, elem, tb), need);
+      for (int k = 0; k < 2; ++k) most[k] = std::max(most[k], need[k] * (int64_t)elem);
+    }
+  op.ws_a.alloc((size_t)most[0]);
+  op.ws_b.alloc((size_t)most[1]);
+  if (reduced) op.ws_c.alloc((size_t)op.n * 8);
 }
 
 // ------------------------------------------------------------------ autotuner inputs
@@ -611,10 +1019,11 @@ void to_f32_dev(const double* x, float* y, int64_t n, cudaStream_t s) {
 
 // ------------------------------------------------------------------ pass plans and tuning
 // Tile bits and threads per block of the chain passes, per (element size,
-// carried bits, width).  Defaults: 2^13-element tiles for 4-byte elements and
-// 2^12 for 8-byte ones (32 KB either way), 256 threads, except where the
-// built-in table of measured choices has an entry; tm_chain_autotune and
-// tm_chain_set_tuning override entries at run time.
+// carried bits, width): 2^13-element tiles and 256 threads for 4-byte
+// elements, 2^12 and 128 for 8-byte ones (32 KB either way; 64 or more groups
+// per warp-round at either size).  Over BNNNI widths 16-24 and DNNI widths
+// 20-26 these are within 10% of the fastest of all tile and block sizes;
+// tm_chain_autotune and tm_chain_set_tuning override entries at run time.
 namespace {
 struct ChainTune {
   int tile_bits = 0, threads = 0;
@@ -623,17 +1032,6 @@ std::mutex g_tune_mu;
 ChainTune g_tune[2][2][33];  // [elem 4/8][zb][L]
 }  // namespace
 
-// Choices of the autotuner (python -m latttmat_gb300.autotune) measured on a
-// GB300 for the diagonal BNNNI widths of the 256-point parameter sweep:
-// {L, tile bits, threads} for 4-byte and for 8-byte elements.
-struct TunedEntry {
-  int L, tb4, th4, tb8, th8;
-};
-constexpr TunedEntry kTunedBNNNI[] = {
-    {16, 11, 128, 11, 128}, {18, 13, 256, 13, 256}, {20, 11, 128, 11, 128},
-    {22, 13, 128, 13, 128}, {24, 12, 128, 12, 128},
-};
-
 void chain_tuning(int L, size_t elem, bool zb, int& tile_bits, int& threads) {
   if (elem >= 16) {  // tangent pairs (adjoint): 32 KB tiles, fewer threads
     tile_bits = 11;
@@ -641,14 +1039,8 @@ void chain_tuning(int L, size_t elem, bool zb, int& tile_bits, int& threads) {
     return;
   }
   tile_bits = (elem == 8) ? 12 : 13;
-  threads = 256;
+  threads = (elem == 8) ? 128 : 256;
   if (L < 0 || L > 32) return;
-  if (zb)
-    for (const TunedEntry& t : kTunedBNNNI)
-      if (t.L == L) {
-        tile_bits = (elem == 8) ? t.tb8 : t.tb4;
-        threads = (elem == 8) ? t.th8 : t.th4;
-      }
   std::lock_guard<std::mutex> lock(g_tune_mu);
   const ChainTune& t = g_tune[elem == 8][zb ? 1 : 0][L];
   if (t.tile_bits) tile_bits = t.tile_bits;
@@ -663,116 +1055,129 @@ void chain_set_tuning(int L, size_t elem, bool zb, int tile_bits, int threads) {
   g_tune[elem == 8][zb ? 1 : 0][L] = ChainTune{tile_bits, threads};
 }
 
-// The passes of one product: the first holds up to cap0 steps (its sites
-// start at 0), the others up to cap1 (they carry a few contiguous low sites
-// for coalescing); the steps are spread evenly over the passes needed.
-std::vector<ChainPass> chain_plan(int L, bool zb, int nlb, int tile_bits) {
-  const int NA = zb ? 2 : 1, KS = zb ? 2 : 1;
-  const int nsteps = zb ? L / 2 : L;
-  const int cbn = zb ? 2 : 3;
-  const int cap0 = std::max(1, (tile_bits - NA) / KS), cap1 = std::max(1, (tile_bits - NA - cbn) / KS);
-  const int npass = (nsteps <= cap0) ? 1 : 1 + (nsteps - cap0 + cap1 - 1) / cap1;
+// The passes of one product.  A tile of 2^tile_bits elements holds the carried
+// letter, a chunk of the old bits below the pass's letters (at
+// least 128 bytes' worth of slots, for coalescing) and the pass's letters; the
+// last pass has no bits below, holds the lastbit values instead and takes as
+// many letters as fit; the others share the rest evenly, the first one (whose
+// gathers want long chunks) the fewest.
+std::vector<ChainPass> chain_plan(const Op& op, size_t elem, int tile_bits) {
+  const bool zb = (op.kind == K_ZBT || op.kind == K_ZBM);
+  const int KS = zb ? 2 : 1, m = op.L / KS;
+  const int bc = zb ? 0 : op.boundary;
+  const int slot = (1 << KS) * (int)elem;
+  const int cbn = (slot == 8) ? 4 : (slot == 16) ? 3 : (slot == 32) ? 2 : 1;
+  const int lbb = (bc == 0) ? KS : 0;
+  const int capl = std::min(kChainMaxT, std::max(1, (tile_bits - KS - lbb) / KS));
+  const int cap = std::min(kChainMaxT, std::max(1, (tile_bits - KS - cbn) / KS));
+  const int lead = std::max(0, m - capl);  // letters before the last pass
+  const int npass = 1 + (lead + cap - 1) / cap;
   std::vector<ChainPass> out;
-  int t0 = 0, pass = 0;
-  while (t0 < nsteps) {
-    // tile state bits: contiguous low sites for coalescing (none when the
-    // steps start at site 0), then the sites of this pass's steps
-    const int cb = (t0 == 0) ? 0 : std::min(KS * t0, cbn);
-    const int left = npass - pass;
-    const int even = (nsteps - t0 + left - 1) / left;
-    const int T_ = std::max(1, std::min(nsteps - t0, std::min(even, t0 == 0 ? cap0 : cap1)));
-    ++pass;
+  int t0 = 0;
+  auto nodes = [&](int t) { return op.tree.nlev ? op.tree.n[t] : (int64_t)1 << (KS * t); };
+  for (int p = 0; p < npass; ++p) {
     ChainPass cp{};
-    std::vector<int> sp;
-    for (int k = 0; k < cb; ++k) sp.push_back(k);
-    for (int k = 0; k < KS * T_; ++k) sp.push_back(KS * t0 + k);
-    cp.nst = (int)sp.size();
-    for (int k = 0; k < cp.nst; ++k) cp.spos[k] = sp[k];
-    uint64_t used = 0;
-    for (int k : sp) used |= 1ull << k;
-    cp.no = 0;
-    for (int b = 0; b < L; ++b)
-      if (!((used >> b) & 1ull)) cp.opos[cp.no++] = b;
     cp.t0 = t0;
-    cp.T = T_;
-    cp.jbit0 = cb;
-    cp.first = (t0 == 0);
-    cp.last = (t0 + T_ >= nsteps);
-    cp.nlb = nlb;
+    cp.T = (p == npass - 1) ? m - t0 : (lead - t0) / (npass - 1 - p);
+    cp.rest = op.L - KS * (t0 + cp.T);
+    cp.cb = std::min(std::max(cbn, tile_bits - KS - KS * cp.T), cp.rest);
+    cp.first = (p == 0);
+    cp.last = (p == npass - 1);
+    cp.nlb = (bc == 0) ? 1 << KS : 1;
+    cp.tb = cp.last ? lbb : cp.cb;
+    cp.nin = nodes(t0);
+    cp.nout = nodes(t0 + cp.T);
     out.push_back(cp);
-    t0 += T_;
+    t0 += cp.T;
   }
   return out;
 }
 
 // blocks of one pass and its dynamic shared memory
-int64_t chain_pass_blocks(const ChainPass& cp) { return (int64_t)(cp.last ? 1 : cp.nlb) << cp.no; }
-size_t chain_pass_smem(const ChainPass& cp, bool zb, size_t elem) {
-  const int NA = zb ? 2 : 1;
-  const int tile = 1 << (NA + cp.nst);
-  return chain_acc_offset(tile, elem) + (cp.last ? (size_t)(tile >> NA) * 8 : 0);
+int64_t chain_pass_blocks(const ChainPass& cp) {
+  return ((int64_t)(cp.last ? 1 : cp.nlb) * cp.nin) << (cp.rest - cp.cb);
 }
+size_t chain_pass_smem(const ChainPass& cp, bool zb, size_t elem) {
+  const int KS = zb ? 2 : 1, bytes = (1 << KS) * (int)elem;
+  const int vec = std::min(bytes, 16);
+  return (size_t)slot_plane(1 << (KS * cp.T + cp.tb), bytes) * (bytes / vec) * vec;
+}
+// (a full operator's passes write every element where they read it: one
+// buffer, in place)
+void chain_buffer_elems(const Op& op, const std::vector<ChainPass>& plan, int64_t need[2]) {
+  const bool zb = (op.kind == K_ZBT || op.kind == K_ZBM);
+  need[0] = need[1] = 0;
+  for (size_t p = 0; p + 1 < plan.size(); ++p)
+    need[op.tree.nlev ? p & 1 : 0] = std::max(need[op.tree.nlev ? p & 1 : 0], ((int64_t)plan[p].nlb * plan[p].nout) << (plan[p].rest + (zb ? 2 : 1)));
+}
+
+namespace {
+TreeDev tree_dev(const Op& op) {
+  TreeDev t{};
+  if (!op.tree.nlev) return t;
+  t.nodes = op.tree.nodes.as<uint2>();
+  t.words = op.tree.words.as<uint16_t>();
+  for (int i = 0; i <= op.tree.nlev; ++i) t.off[i] = (uint32_t)op.tree.off[i];
+  return t;
+}
+}  // namespace
 
 // y = T x (or T^T x for transposed views); scaled: FP32 result divided by the
 // returned factor.
 // T: arithmetic and pass-buffer type (float, double, or dfloat: FP64-accurate
 // products on the FP32 pipes); IO: element type of x and y.
-template <class T>
-T coef_with_derivative(double v, double d) {
-  if constexpr (std::is_same<T, tangent>::value)
-    return tangent(v, d);
-  else
-    return (T)v;
-}
-
 template <class T, class IO = T>
 double matvec_aux_dir(const Op& op, const IO* x, IO* y, bool scaled, int dir, cudaStream_t s,
-                      const AuxCoef* dcoef = nullptr, void* pass_buf = nullptr) {
+                      const AuxCoef* dcoef = nullptr, void* buf0 = nullptr, void* buf1 = nullptr) {
+  using U = typename ChainIn<T>::U;
   const int L = op.L;
   const bool reduced = (op.kind == K_XDM || op.kind == K_ZBM);
   const bool zb = (op.kind == K_ZBT || op.kind == K_ZBM);
-  AuxCoef c64 = coef_of(op);
-  const double gb = step_bound(op, c64, dir);
   // FP32 and double-float steps (tangent pairs included) are normalised
   // (FP32 exponent range)
-  const bool norm = (sizeof(T) == 4) || std::is_same<T, dfloat>::value || std::is_same<T, tangent>::value;
-  AuxCoefT<T> c;
-  for (int k = 0; k < 2; ++k) {
-    c.b1[k] = coef_with_derivative<T>(c64.b1[k], dcoef ? dcoef->b1[k] : 0.0);
-    c.b2[k] = coef_with_derivative<T>(c64.b2[k], dcoef ? dcoef->b2[k] : 0.0);
-    c.b3[k] = coef_with_derivative<T>(c64.b3[k], dcoef ? dcoef->b3[k] : 0.0);
-  }
-  c.g = norm ? (T)(1.0 / gb) : (T)1;
+  const bool norm = !std::is_same<T, double>::value;
+  ChainTab<T> tab;
+  double bias = 1.0;
+  const double gb = chain_tab<T>(zb, dir, coef_of(op), dcoef, norm, tab, &bias);
   const int nsteps = zb ? L / 2 : L;
   const double gscale = norm ? std::pow(gb, (double)nsteps) : 1.0;
-  const double sf = scaled ? 1.0 : gscale;
+  const double sf = (scaled ? 1.0 : gscale) * std::pow(bias, (double)nsteps);
   const int bc = zb ? 0 : op.boundary;
-  const int nlb = zb ? 4 : (bc == 0 ? 2 : 1);
   int tile_bits = 0, threads = 0;
   chain_tuning(L, sizeof(T), zb, tile_bits, threads);
-  T* P = pass_buf ? static_cast<T*>(pass_buf) : op.ws_a.as<T>();
-  const uint32_t* smap = reduced ? op.smap.as<uint32_t>() : nullptr;
-  IO* fold_out = reduced ? op.xp.as<IO>() : y;
-  const double postc = zb ? sf : (reduced ? sf : op.normfactor * sf);
-  const double* post = reduced ? nullptr : op.tvec.as<double>();
-  for (const ChainPass& cp : chain_plan(L, zb, nlb, tile_bits)) {
+  T* buf[2] = {buf0 ? static_cast<T*>(buf0) : op.ws_a.as<T>(), buf1 ? static_cast<T*>(buf1) : op.ws_b.as<T>()};
+  if (!op.tree.nlev) buf[1] = buf[0];
+  ChainIO<T, IO> io{};
+  io.tv = op.tvec.as<double>();
+  io.y = y;
+  io.post = scale_factor(((zb || reduced) ? 1.0 : op.normfactor) * sf);
+  if (reduced) {
+    U* u = op.ws_c.as<U>();
+    chain_scale_in<U, IO><<<grid_for(op.n), 256, 0, s>>>(x, op.tvec.as<double>(), u, op.n);
+    TM_CKK("chain_scale_in");
+    io.u = u;
+    io.smap = op.smap.as<uint32_t>();
+    io.dup = op.dup.as<uint16_t>();
+  } else {
+    io.x = x;
+    io.pre = op.tvec.as<double>();
+  }
+  const TreeDev tr = tree_dev(op);
+  int p = 0;
+  for (const ChainPass& cp : chain_plan(op, sizeof(T), tile_bits)) {
     const int64_t nblocks = chain_pass_blocks(cp);
     const size_t shm = chain_pass_smem(cp, zb, sizeof(T));
+    io.src = buf[(p + 1) & 1];
+    io.dst = buf[p & 1];
     if (zb) {
-      raise_smem_limit((const void*)chain_kernel<T, 1, IO>, shm);
-      chain_kernel<T, 1, IO><<<(unsigned)nblocks, threads, shm, s>>>(P, x, op.tvec.as<double>(), smap, fold_out, post,
-                                                                postc, L, bc, dir, c, cp);
+      raise_smem_limit((const void*)chain_kernel<T, 2, IO>, shm);
+      chain_kernel<T, 2, IO><<<(unsigned)nblocks, threads, shm, s>>>(io, tab, cp, tr, L, bc);
     } else {
-      raise_smem_limit((const void*)chain_kernel<T, 0, IO>, shm);
-      chain_kernel<T, 0, IO><<<(unsigned)nblocks, threads, shm, s>>>(P, x, op.tvec.as<double>(), smap, fold_out, post,
-                                                                postc, L, bc, dir, c, cp);
+      raise_smem_limit((const void*)chain_kernel<T, 1, IO>, shm);
+      chain_kernel<T, 1, IO><<<(unsigned)nblocks, threads, shm, s>>>(io, tab, cp, tr, L, bc);
     }
     TM_CKK("aux_chain");
-  }
-  if (reduced) {
-    red_contract<IO><<<grid_for(op.n), 256, 0, s>>>(fold_out, op.idx.as<uint32_t>(), op.dup.as<uint16_t>(),
-                                                   op.tvec.as<double>(), 1.0, y, op.n);
-    TM_CKK("red_contract");
+    ++p;
   }
   return scaled ? gscale : 1.0;
 }
@@ -786,53 +1191,39 @@ void chain_inst_fill(const Op& op, int dir, ChainInst& rec, int tb4, int tb8) {
   rec.zb = zb;
   rec.bc = zb ? 0 : op.boundary;
   rec.dir = dir;
-  rec.nlb = zb ? 4 : (rec.bc == 0 ? 2 : 1);
+  rec.nlb = (rec.bc == 0) ? (zb ? 4 : 2) : 1;
   rec.n = op.n;
   // full DNNI applies the normfactor at the output; the BNNNI Tvec holds it
   rec.nf = (reduced || zb) ? 1.0 : op.normfactor;
   const AuxCoef c = coef_of(op);
-  const double gb = step_bound(op, c, dir);
+  double bias = 1.0;
+  const double gb = chain_tab<float>(zb, dir, c, nullptr, true, rec.c32, &bias);
+  chain_tab<dfloat>(zb, dir, c, nullptr, true, rec.cdf);
+  chain_tab<double>(zb, dir, c, nullptr, false, rec.c64);
   const int nsteps = zb ? L / 2 : L;
-  for (int q = 0; q < 2; ++q) {
-    rec.c32.b1[q] = (float)c.b1[q];
-    rec.c32.b2[q] = (float)c.b2[q];
-    rec.c32.b3[q] = (float)c.b3[q];
-    rec.cdf.b1[q] = dfloat(c.b1[q]);
-    rec.cdf.b2[q] = dfloat(c.b2[q]);
-    rec.cdf.b3[q] = dfloat(c.b3[q]);
-    rec.c64.b1[q] = c.b1[q];
-    rec.c64.b2[q] = c.b2[q];
-    rec.c64.b3[q] = c.b3[q];
-  }
-  rec.c32.g = (float)(1.0 / gb);
-  rec.cdf.g = dfloat(1.0 / gb);
-  rec.c64.g = 1.0;
-  rec.gs32 = rec.gsdf = std::pow(gb, (double)nsteps);
+  rec.gsdf = std::pow(gb, (double)nsteps);
+  rec.gs32 = rec.gsdf * std::pow(bias, (double)nsteps);
   rec.gs64 = 1.0;
   int th = 0;
   if (tb4 <= 0) chain_tuning(L, 4, zb, tb4, th);
   if (tb8 <= 0) chain_tuning(L, 8, zb, tb8, th);
   int tb16 = 0;
   chain_tuning(L, 16, zb, tb16, th);
-  const std::vector<ChainPass> p16 = chain_plan(L, zb, rec.nlb, tb16);
+  const std::vector<ChainPass> p16 = chain_plan(op, 16, tb16);
   if ((int)p16.size() > kChainMaxPass) fail(TM_ERR_LIMIT, "too many chain passes");
   rec.np16 = (int)p16.size();
   for (int q = 0; q < rec.np16; ++q) rec.p16[q] = p16[q];
   for (int t = 0; t < 3; ++t) {
     const AuxCoef db = aux_coef_derivative(op.mp.betaJ, op.mp.kappa, op.mp.kappa2, t);
-    for (int q = 0; q < 2; ++q) {
-      rec.ctan[t].b1[q] = tangent(c.b1[q], db.b1[q]);
-      rec.ctan[t].b2[q] = tangent(c.b2[q], db.b2[q]);
-      rec.ctan[t].b3[q] = tangent(c.b3[q], db.b3[q]);
-    }
-    rec.ctan[t].g = tangent(1.0 / gb);  // a constant: no derivative
+    chain_tab<tangent>(zb, dir, c, &db, true, rec.ctan[t]);  // the normalisation is a constant: no derivative
   }
+  rec.tree = tree_dev(op);
   rec.kind = op.kind;
   rec.bj = op.mp.betaJ;
   rec.kap = op.mp.kappa;
   rec.kap2 = op.mp.kappa2;
   rec.h = op.mp.h;
-  const std::vector<ChainPass> p4 = chain_plan(L, zb, rec.nlb, tb4), p8 = chain_plan(L, zb, rec.nlb, tb8);
+  const std::vector<ChainPass> p4 = chain_plan(op, 4, tb4), p8 = chain_plan(op, 8, tb8);
   if ((int)p4.size() > kChainMaxPass || (int)p8.size() > kChainMaxPass) fail(TM_ERR_LIMIT, "too many chain passes");
   rec.np4 = (int)p4.size();
   rec.np8 = (int)p8.size();
@@ -845,51 +1236,33 @@ void chain_inst_fill(const Op& op, int dir, ChainInst& rec, int tb4, int tb8) {
 }
 
 namespace {
-template <class T, int ZB, class IO, int MODE>
-void launch_batch_pass(const ChainInst* inst, const int2* km, const int64_t* start, const int* bmem, int pass,
-                       int64_t nblk, int threads, size_t smem, cudaStream_t s, int theta) {
-  raise_smem_limit((const void*)chain_batch_kernel<T, ZB, IO, MODE>, smem);
-  chain_batch_kernel<T, ZB, IO, MODE><<<(unsigned)nblk, threads, smem, s>>>(inst, km, start, bmem, pass, theta);
-  TM_CKK("chain_batch");
-}
-
-template <int ZB, int MODE>
-int batch_product_mode(const ChainBatch& B, const int2* km, const ChainBatch::Plan& P, cudaStream_t s, int theta) {
-  int launches = 0;
+template <class T, int KS, int MODE>
+int batch_passes(const ChainBatch& B, const int2* km, const ChainBatch::Plan& P, cudaStream_t s, int theta) {
+  int launches = 1;
+  chain_batch_scale_in<typename ChainIn<T>::U, MODE><<<(unsigned)B.nrblk, 256, 0, s>>>(B.inst, km, B.rstart, B.rmem);
+  TM_CKK("chain_batch_scale_in");
   for (int p = 0; p < P.np; ++p) {
     if (P.nblk[p] == 0) continue;
-    const int64_t* st = P.start + (size_t)p * (B.count + 1);
-    const int* bm = P.bmem + P.boff[p];
-    if constexpr (MODE == kModeF32)
-      launch_batch_pass<float, ZB, float, MODE>(B.inst, km, st, bm, p, P.nblk[p], P.threads, P.smem, s, theta);
-    else if constexpr (MODE == kModeDF)
-      launch_batch_pass<dfloat, ZB, double, MODE>(B.inst, km, st, bm, p, P.nblk[p], P.threads, P.smem, s, theta);
-    else if constexpr (MODE == kModeTangent)
-      launch_batch_pass<tangent, ZB, double, MODE>(B.inst, km, st, bm, p, P.nblk[p], P.threads, P.smem, s, theta);
-    else
-      launch_batch_pass<double, ZB, double, MODE>(B.inst, km, st, bm, p, P.nblk[p], P.threads, P.smem, s, theta);
+    raise_smem_limit((const void*)chain_batch_kernel<T, KS, MODE>, P.smem);
+    chain_batch_kernel<T, KS, MODE><<<(unsigned)P.nblk[p], P.threads, P.smem, s>>>(
+        B.inst, km, P.start + (size_t)p * (B.count + 1), P.bmem + P.boff[p], p, theta);
+    TM_CKK("chain_batch");
     ++launches;
   }
-  if constexpr (MODE == kModeF32)
-    contract_batch_kernel<float, MODE><<<(unsigned)B.nrblk, 256, 0, s>>>(B.inst, km, B.rstart, B.rmem);
-  else
-    contract_batch_kernel<double, MODE><<<(unsigned)B.nrblk, 256, 0, s>>>(B.inst, km, B.rstart, B.rmem);
-  TM_CKK("contract_batch");
-  return launches + 1;
+  return launches;
+}
+
+template <int KS>
+int batch_product(const ChainBatch& B, const int2* km, int mode, cudaStream_t s, int theta) {
+  if (mode == kModeF32) return batch_passes<float, KS, kModeF32>(B, km, B.p4, s, theta);
+  if (mode == kModeDF) return batch_passes<dfloat, KS, kModeDF>(B, km, B.p8, s, theta);
+  if (mode == kModeTangent) return batch_passes<tangent, KS, kModeTangent>(B, km, B.p16, s, theta);
+  return batch_passes<double, KS, kModeF64>(B, km, B.p8, s, theta);
 }
 }  // namespace
 
 int chain_batch_product(const ChainBatch& B, const int2* km, int mode, cudaStream_t s, int theta) {
-  if (B.zb) {
-    if (mode == kModeF32) return batch_product_mode<1, kModeF32>(B, km, B.p4, s, theta);
-    if (mode == kModeDF) return batch_product_mode<1, kModeDF>(B, km, B.p8, s, theta);
-    if (mode == kModeTangent) return batch_product_mode<1, kModeTangent>(B, km, B.p16, s, theta);
-    return batch_product_mode<1, kModeF64>(B, km, B.p8, s, theta);
-  }
-  if (mode == kModeF32) return batch_product_mode<0, kModeF32>(B, km, B.p4, s, theta);
-  if (mode == kModeDF) return batch_product_mode<0, kModeDF>(B, km, B.p8, s, theta);
-  if (mode == kModeTangent) return batch_product_mode<0, kModeTangent>(B, km, B.p16, s, theta);
-  return batch_product_mode<0, kModeF64>(B, km, B.p8, s, theta);
+  return B.zb ? batch_product<2>(B, km, mode, s, theta) : batch_product<1>(B, km, mode, s, theta);
 }
 
 // ------------------------------------------------------------------ autotuner
@@ -973,13 +1346,17 @@ template double matvec_aux<double>(const Op&, const double*, double*, bool, cuda
 // steps differentiated with respect to one parameter whose effect on the step
 // factors b1, b2, b3 is `db` (the Boltzmann weights Tvec held fixed), FP64.
 void matvec_aux_tangent(const Op& op, const double* x, double* y, const AuxCoef& db, int dir, cudaStream_t s) {
-  // the pass buffer at 16 bytes per element (the operator's holds 8)
+  // pass buffers at 16 bytes per element (the operator's hold 8)
   const bool zb = (op.kind == K_ZBT || op.kind == K_ZBM);
-  const int64_t per = (zb ? 16ll : 4ll) << op.L;
+  int tb = 0, th = 0;
+  chain_tuning(op.L, 16, zb, tb, th);
+  int64_t need[2];
+  chain_buffer_elems(op, chain_plan(op, 16, tb), need);
   AllocStream guard(s);
-  DBuf P;
-  P.alloc((size_t)per * sizeof(tangent));
-  matvec_aux_dir<tangent, double>(op, x, y, false, dir, s, &db, P.p);
+  DBuf P, Q;
+  P.alloc((size_t)need[0] * 16);
+  Q.alloc((size_t)need[1] * 16);
+  matvec_aux_dir<tangent, double>(op, x, y, false, dir, s, &db, P.p, Q.p);
 }
 
 // FP64-accurate product in double-float arithmetic (the solver's refinement

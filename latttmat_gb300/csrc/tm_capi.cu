@@ -332,8 +332,10 @@ static void build_op(Op& op) {
       build_state_map(op);
       op.ws_a.release();
       op.ws_b.release();
-      op.ws_c.alloc((size_t)op.n * 8);
-      if (bfly_core(op.kind)) build_bfly(op);
+      if (bfly_core(op.kind)) {
+        op.ws_c.alloc((size_t)op.n * 8);
+        build_bfly(op);
+      }
     }
   } else {
     if (op.L > 30) fail(TM_ERR_LIMIT, "full operators support L <= 30");

@@ -14,25 +14,51 @@ struct AuxCoef {
   double b1[2], b2[2], b3[2];
 };
 
+// Step tables of one arithmetic, formed on the host in FP64 and rounded once.
+// One step rewrites a letter (KS sites, S = 2^KS values) of the state:
+//   out(a', s') = zu[c][s', a'] sum_q w1[s'][q] in(q, a'),
+// q the carried old letter, a' the old letter here, c the old letter next in
+// line.  The sum runs as one (DNNI) or two (BNNNI) levels of two-term sums
+// x + rho y, whose common factors are folded into zu, as is the step
+// normalisation:
+//   DNNI:  d(s') = in(s') + rho1 in(1 - s')
+//   BNNNI: t(sl, qr) = in(ql = sl, qr) + rho1 in(1 - sl, qr),
+//          d(sl, sr) = t(sl, 0) + rho2[s'] t(sl, 1)
+// zu: DNNI [c][s'][a'], BNNNI [c][a'][s'].  w1[s'][q]: the same sum's
+// coefficients, for the first step (one q only).  b2: open-boundary factors.
 template <class T>
-struct AuxCoefT {
-  T b1[2], b2[2], b3[2];
-  T g;  // step normalisation (multiply)
+struct ChainTab {
+  T rho1;
+  T rho2[4];
+  T b2[2];
+  T w1[16];
+  T zu[64];
 };
 
-// Geometry of one pass.  Element index in HBM: ((lb << L | r) << NA) | aux.
-// Tile index e: bits [0, NA) aux, then tile state bits k -> state position
-// spos[k]; the outer index (blockIdx) deposits into opos[] (state bits) and,
-// when the lastbit pass is outer, into lb.
+// Geometry of one pass: letters [t0, t0 + T) of the state, top letter first.
+// Between passes an element is (lb, prefix node, remaining old bits, carried
+// letter), the carried letter fastest; the node runs over the prefixes of new
+// letters (all of them in a full operator, those leading to a representative
+// in a reduced one).  A block takes one (lb, node, outer old bits) and holds
+// the pass's letters times 2^cb contiguous remaining bits in shared memory.
 struct ChainPass {
-  int nst;         // tile state bits
-  int spos[16];
-  int no;          // outer state bits
-  int opos[32];
-  int t0, T;       // steps [t0, t0 + T)
-  int jbit0;       // tile state bit of step t0's lowest site
+  int t0, T;
+  int rest;        // old bits below the pass's letters
+  int cb;          // chunk bits (of rest) in the tile
+  int nlb;         // lastbit values (the ring's first old letter; 1 when open)
+  int tb;          // low bits of a tile slot: cb, in the last pass log2(nlb) (a tile holds all of them)
   int first, last; // build from x / fold into y
-  int nlb;         // lastbit passes (DNNI 2 or 1, BNNNI 4)
+  int64_t nin, nout;  // nodes before and after the pass
+};
+
+// A reduced operator's prefix tree, one level per letter (tm_tree.cu);
+// nodes null: a full operator.  (No member initialisers: blocks keep a copy in
+// shared memory, where a constructor would run in every thread, over what
+// others have already copied there.)
+struct TreeDev {
+  const uint2* nodes;
+  const uint16_t* words;
+  uint32_t off[kTreeMaxLevels + 1];
 };
 
 constexpr int kChainMaxPass = 8;
@@ -53,21 +79,21 @@ struct ChainInst {
   int L, bc, dir, zb, nlb, kind;
   double bj, kap, kap2, h;       // model parameters (the adjoint's weight derivatives)
   int64_t n;                    // rows
-  AuxCoefT<float> c32;
-  AuxCoefT<dfloat> cdf;
-  AuxCoefT<double> c64;
-  AuxCoefT<tangent> ctan[3];    // FP64 factors with their derivative by betaJ, kappa, kappa2
+  ChainTab<float> c32;
+  ChainTab<dfloat> cdf;
+  ChainTab<double> c64;
+  ChainTab<tangent> ctan[3];    // with the derivatives by betaJ, kappa, kappa2
+  TreeDev tree;
   double gs32, gsdf, gs64;      // output factors undoing the step normalisation
   double nf;                    // normfactor (full operators)
   const uint32_t* smap;         // state -> rank (reduced) or null
   const double* tvec;
   const uint32_t* idx;          // reduced: representatives (null for full operators)
   const uint16_t* dup;
-  void* P;                      // pass buffer (8-byte elements, 16-byte for tangent products)
-  void* fold;                   // fold output, 2^L (8-byte) elements
+  void *P, *Q;                  // pass buffers, written by even and odd passes
   double* V;                    // Krylov basis: column c at V + c * ldv
   int64_t ldv;
-  float* x32;                   // FP32 product input
+  void* u;                      // product input times Tvec (n elements of the step's arithmetic)
   double* w;                    // product output and CGS work vector
   double* sc;                   // small per-instance values (kSweepScal doubles)
 };
@@ -122,14 +148,14 @@ inline AuxCoef aux_coef_derivative(double bj, double k, double k2, int t) {
   return db;
 }
 
-// Coefficients and scales of an operator's product in the three arithmetics.
 AuxCoef coef_of(const Op& op);
-double step_bound(const Op& op, const AuxCoef& c, int dir);
 void chain_tuning(int L, size_t elem, bool zb, int& tile_bits, int& threads);
 void chain_set_tuning(int L, size_t elem, bool zb, int tile_bits, int threads);
-std::vector<ChainPass> chain_plan(int L, bool zb, int nlb, int tile_bits);
+std::vector<ChainPass> chain_plan(const Op& op, size_t elem, int tile_bits);
 int64_t chain_pass_blocks(const ChainPass& cp);
 size_t chain_pass_smem(const ChainPass& cp, bool zb, size_t elem);
+// elements of the two pass buffers that a plan writes
+void chain_buffer_elems(const Op& op, const std::vector<ChainPass>& plan, int64_t need[2]);
 
 // Fill the geometry and coefficients of `rec` for operator `op` (an aux-bit
 // operator; dir 1 for its transpose), with tiles of 2^tb4 (4-byte) and 2^tb8
@@ -156,8 +182,8 @@ struct ChainBatch {
 };
 
 // Batched product of every member in `mode` (input: column km[i].x of its
-// basis, or its x32 in FP32): one launch per pass over all members' tiles,
-// then one contraction launch into each w.  In kModeTangent the product is
+// basis): one launch that scales the inputs by Tvec, then one launch per pass
+// over all members' tiles, the last writing each w.  In kModeTangent the product is
 // the chain's derivative by parameter `theta` (0 betaJ, 1 kappa, 2 kappa2)
 // between the fixed Boltzmann weights.  Returns the launches issued.
 int chain_batch_product(const ChainBatch& B, const int2* km, int mode, cudaStream_t s, int theta = 0);

@@ -397,7 +397,7 @@ void build_bfly(Op& op) {
     steps.push_back((op.L - b + nlev - i - 1) / (nlev - i));
     b += steps.back();
   }
-  build_prefix_tree(op, op.L, steps, op.tree);
+  build_prefix_tree(op, op.L, steps, false, op.tree);
   int64_t most[2] = {1, 1};
   for (int i = 0; i + 1 < nlev; ++i)
     most[i & 1] = std::max(most[i & 1], op.tree.n[i + 1] << (op.L - op.tree.b[i + 1]));

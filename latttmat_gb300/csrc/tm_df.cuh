@@ -89,6 +89,37 @@ __device__ __forceinline__ dfloat& operator*=(dfloat& a, dfloat b) {
   return a;
 }
 
+// Double-float values two to a lane pair: hi words in one float2, lo words in
+// another.  df2_fma_unnorm is df_fma_unnorm (tm_df.cuh) on both lanes with the
+// same operation sequence (so the same results), on the packed FP32 pipes;
+// differences are taken as fma(b, -1, a), and -p comes from -r.hi, so no
+// operand needs a separate negation.
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }
+__device__ __forceinline__ void df2_fma_unnorm(float2 rh, float2 rl, float2 rhn, float2 xh, float2 xl, float2 yh,
+                                               float2 yl, float2& oh, float2& ol) {
+  const float2 np = __fmul2_rn(rhn, xh);  // -p, p = r.hi x.hi
+  float2 pe = __ffma2_rn(rh, xh, np);     // r.hi x.hi - p (exact)
+  pe = __ffma2_rn(rh, xl, pe);
+  pe = __ffma2_rn(rl, xh, pe);
+  const float2 sm = sub2(yh, np);            // p + y.hi
+  const float2 bb = __fadd2_rn(sm, np);      // s - p
+  const float2 t = sub2(sm, bb);             // s - bb
+  const float2 e2 = sub2(yh, bb);            // y.hi - bb
+  const float2 se = sub2(e2, __fadd2_rn(np, t));  // (p - (s - bb)) + (y.hi - bb)
+  oh = sm;
+  ol = __fadd2_rn(se, __fadd2_rn(pe, yl));
+}
+
+// x * w on both lanes (operator*, renormalised), w = (wh, wl)
+__device__ __forceinline__ void df2_mul(float2 xh, float2 xl, float2 wh, float2 wl, float2& oh, float2& ol) {
+  const float2 np = __fmul2_rn(xh, make_float2(-wh.x, -wh.y));  // -p
+  float2 e = __ffma2_rn(xh, wh, np);
+  e = __ffma2_rn(xh, wl, e);
+  e = __ffma2_rn(xl, wh, e);
+  oh = sub2(e, np);                  // p + e
+  ol = sub2(e, __fadd2_rn(oh, np));  // e - (h - p)
+}
+
 // A constant factor of a result rounded to FP32 once (scale_round): f64, and
 // the same as two * hl with `two` a power of two near its square root, so
 // that partial products stay near the result's exponent range.
@@ -108,17 +139,42 @@ inline ScaleF scale_factor(double S) {
   return p;
 }
 
+// The FP64 form of scale_round.  Not inlined: as part of the caller it would be
+// predicated, and a predicated FP64 instruction takes its slot on the pipe
+// (73% busy in the first DNNI pass that way).
+static __device__ __noinline__ float scale_round_f64(float vh, float vl, double t, double f) {
+  return (float)(((double)vh + (double)vl) * t * f);
+}
+static __device__ __noinline__ float scale_round_f64(float vh, float vl, float th, float tl, double f) {
+  return (float)(((double)vh + (double)vl) * ((double)th + (double)tl) * f);
+}
+__device__ __forceinline__ float hi_of(float v) { return v; }
+__device__ __forceinline__ float hi_of(dfloat v) { return v.hi; }
+__device__ __forceinline__ float lo_of(float) { return 0.f; }
+__device__ __forceinline__ float lo_of(dfloat v) { return v.lo; }
+
 // (v * sc) * post rounded to FP32 once: the products' rounding errors are
 // carried along (TwoProduct by FMA), so the result is that of FP64 arithmetic
 // to within the last rounding, without the FP64 pipe (two lanes per clock and
-// SM, conversions included).  Zeros, infinities, NaN and products near the
-// ends of the exponent range, where the error terms would be lost, take the
-// FP64 form.
+// SM, conversions included).  Infinities, NaN and products near the ends of
+// the exponent range, where the error terms would be lost, take the FP64 form.
 __device__ __forceinline__ float scale_round(float v, dfloat sc, const ScaleF& post) {
   const float a = v * post.two;  // exact
   const float p = a * sc.hi;
-  if (!(fabsf(p) > 1e-24f && fabsf(p) < 1e24f)) return (float)((double)v * (double)sc * post.f64);
+  if (v == 0.f) return p;
+  if (!(fabsf(p) > 1e-24f && fabsf(p) < 1e24f)) return scale_round_f64(hi_of(v), lo_of(v), sc.hi, sc.lo, post.f64);
   const float e = fmaf(a, sc.lo, fmaf(a, sc.hi, -p));
+  const float q = p * post.hl.hi;
+  return q + fmaf(e, post.hl.hi, fmaf(p, post.hl.lo, fmaf(p, post.hl.hi, -q)));
+}
+
+// the same for a double-float value
+__device__ __forceinline__ float scale_round(dfloat v, dfloat sc, const ScaleF& post) {
+  const float a = v.hi * post.two;  // exact
+  const float p = a * sc.hi;
+  if (v.hi == 0.f) return p;
+  if (!(fabsf(p) > 1e-24f && fabsf(p) < 1e24f)) return scale_round_f64(hi_of(v), lo_of(v), sc.hi, sc.lo, post.f64);
+  const float e = fmaf(v.lo * post.two, sc.hi, fmaf(a, sc.lo, fmaf(a, sc.hi, -p)));
   const float q = p * post.hl.hi;
   return q + fmaf(e, post.hl.hi, fmaf(p, post.hl.lo, fmaf(p, post.hl.hi, -q)));
 }
@@ -126,10 +182,11 @@ __device__ __forceinline__ float scale_round(float v, dfloat sc, const ScaleF& p
 // v * t * post for an FP64 weight t: t is split into a double-float by
 // integer operations (the hi word truncated to 24 bits, the lo word the 29
 // bits below), so nothing runs on the FP64 pipe but the rare cases.
-__device__ __forceinline__ float scale_round(float v, double t, const ScaleF& post) {
+template <class V>
+__device__ __forceinline__ float scale_round(V v, double t, const ScaleF& post) {
   const uint32_t up = (uint32_t)__double2hiint(t), dn = (uint32_t)__double2loint(t);
   const int e = (int)((up >> 20) & 0x7ffu) - 1023;
-  if (e < -70 || e > 90) return (float)((double)v * t * post.f64);
+  if (e < -70 || e > 90) return scale_round_f64(hi_of(v), lo_of(v), t, post.f64);
   const uint32_t sign = up & 0x80000000u;
   const uint32_t m23 = ((up & 0xfffffu) << 3) | (dn >> 29);
   const float hi = __uint_as_float(sign | ((uint32_t)(e + 127) << 23) | m23);

@@ -176,27 +176,6 @@ __device__ __forceinline__ void reg_bfly_f2(float2 (&v)[1 << (NB - 1)], float r,
   }
 }
 
-// Double-float values two to a lane pair: hi words in one float2, lo words in
-// another.  df2_fma_unnorm is df_fma_unnorm (tm_df.cuh) on both lanes with the
-// same operation sequence (so the same results), on the packed FP32 pipes;
-// differences are taken as fma(b, -1, a), and -p comes from -r.hi, so no
-// operand needs a separate negation.
-__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }
-__device__ __forceinline__ void df2_fma_unnorm(float2 rh, float2 rl, float2 rhn, float2 xh, float2 xl, float2 yh,
-                                               float2 yl, float2& oh, float2& ol) {
-  const float2 np = __fmul2_rn(rhn, xh);  // -p, p = r.hi x.hi
-  float2 pe = __ffma2_rn(rh, xh, np);     // r.hi x.hi - p (exact)
-  pe = __ffma2_rn(rh, xl, pe);
-  pe = __ffma2_rn(rl, xh, pe);
-  const float2 sm = sub2(yh, np);            // p + y.hi
-  const float2 bb = __fadd2_rn(sm, np);      // s - p
-  const float2 t = sub2(sm, bb);             // s - bb
-  const float2 e2 = sub2(yh, bb);            // y.hi - bb
-  const float2 se = sub2(e2, __fadd2_rn(np, t));  // (p - (s - bb)) + (y.hi - bb)
-  oh = sm;
-  ol = __fadd2_rn(se, __fadd2_rn(pe, yl));
-}
-
 // reg_bfly for double-float values held as (hi pair, lo pair) per two
 // elements: level 0 within a pair (scalar), every higher level on whole
 // pairs, then one renormalisation per element

@@ -121,7 +121,8 @@ struct PrefixTree {
   int b[kTreeMaxLevels + 1] = {0};   // prefix length per level
   int64_t n[kTreeMaxLevels + 1] = {0};
   int64_t off[kTreeMaxLevels + 1] = {0};
-  DBuf nodes;                        // uint2, level i at off[i]
+  DBuf nodes;                        // uint2, level i < nlev at off[i]
+  DBuf words;                        // u16, level i <= nlev at off[i]: the prefix's last 16 bits
   uint2* level(int i) const { return nodes.as<uint2>() + off[i]; }
 };
 
@@ -174,7 +175,6 @@ struct Op {
   // workspace
   DBuf ws_a, ws_b, ws_c;  // full-space scratch
   DBuf hx, hy;            // device copies for host-vector matvecs
-  DBuf xp;                // full-space result of the aux-bit products before contraction
   DBuf yp;                // pi-ordered result of the even/odd reference-order product
   double scale32 = 1.0;   // FP32 matvec output scale (applied in FP64)
 
@@ -190,7 +190,7 @@ void build_group(Op& op);
 void build_orbit_table(Op& op);          // idx, dup (reference order)
 void build_tvec(Op& op);                 // Tvec for the operator
 void build_state_map(Op& op);            // smap for the generic reduced path
-void build_prefix_tree(const Op& op, int nbits, const std::vector<int>& steps, PrefixTree& out);
+void build_prefix_tree(const Op& op, int nbits, const std::vector<int>& steps, bool words, PrefixTree& out);
 void build_bfly(Op& op);                 // constants, tree and workspace of the Kronecker-core products
 struct EOHostTables;                     // host-side even/odd plan tables (tm_eo.cu)
 std::shared_ptr<EOHostTables> eo_host_tables(int m, int flip);

@@ -9,8 +9,8 @@
 //     member's pass geometry, Boltzmann factors and buffers, whatever its
 //     width;
 //   - each chain pass is ONE launch over the tiles of every member (a block
-//     takes its member from a per-block member map); so are the contraction
-//     and the Krylov vector kernels (row chunks of kSweepRows);
+//     takes its member from a per-block member map); so are the input
+//     scaling and the Krylov vector kernels (row chunks of kSweepRows);
 //   - every step, each active member extends its Arnoldi basis by one column
 //     (member i at its own column j_i, km[i] on the device), so members
 //     restart independently and none waits for another's cycle;
@@ -70,17 +70,6 @@ __device__ __forceinline__ RowBlock row_block(const ChainInst* __restrict__ inst
 
 // km[i] = (column j the member extends this step, product mode or idle)
 __device__ __forceinline__ bool step_on(int2 km) { return km.y != kModeIdle; }
-
-// x32 = (float) V[:, j] for the members in the FP32 phase
-__global__ void __launch_bounds__(256) sw_to_f32(const ChainInst* __restrict__ inst, const int2* __restrict__ km,
-                                                 const int64_t* __restrict__ rstart, int count) {
-  const RowBlock rb = row_block(inst, rstart, count);
-  const int2 k = km[rb.i];
-  if (k.y != kModeF32) return;
-  const ChainInst& I = inst[rb.i];
-  const double* v = I.V + (int64_t)k.x * I.ldv;
-  for (int64_t r = rb.r0 + threadIdx.x; r < rb.r1; r += blockDim.x) I.x32[r] = (float)v[r];
-}
 
 // partial dots of w against columns 0..j: one warp per column, lanes over rows
 __global__ void __launch_bounds__(256) sw_mdot(const ChainInst* __restrict__ inst, const int2* __restrict__ km,
@@ -379,9 +368,29 @@ struct Sweep {
 
   // device memory one member needs in a wave (basis of m+1 columns)
   size_t member_bytes(const Op& o, int m, size_t elem = 8) const {
-    const int64_t N = 1ll << o.L;
-    const int64_t per = zb ? 16 * N : 4 * N;
-    return (size_t)per * elem + (size_t)N * 8 + (size_t)(m + 1) * o.n * 8 + (size_t)o.n * 12 + kScStride * 8 + 4096;
+    return chain_bytes(o, elem) + (size_t)(m + 1) * o.n * 8 + (size_t)o.n * 16 + kScStride * 8 + 4096;
+  }
+  // its pass buffers under any tile size (elem 16: the tangent plan alone)
+  size_t chain_bytes(const Op& o, size_t elem, size_t part[2] = nullptr) const {
+    size_t most[2] = {16, 16};
+    for (size_t e : {(size_t)4, (size_t)8, (size_t)16}) {
+      if ((e == 16) != (elem == 16)) continue;
+      int t0 = 10, t1 = (e == 4) ? 14 : 13, th = 0;
+      if (e == 16) {
+        chain_tuning(o.L, 16, zb, t0, th);
+        t1 = t0;
+      }
+      for (int tb = t0; tb <= t1; ++tb) {
+        int64_t need[2];
+        chain_buffer_elems(o, chain_plan(o, e, tb), need);
+        for (int k = 0; k < 2; ++k) most[k] = std::max(most[k], (size_t)need[k] * e);
+      }
+    }
+    if (part) {
+      part[0] = most[0];
+      part[1] = most[1];
+    }
+    return most[0] + most[1];
   }
 
   std::vector<std::pair<int, int>> waves(int m, size_t elem = 8) const {
@@ -442,18 +451,19 @@ struct Wave {
       ChainInst& I = host[q];
       std::memset(&I, 0, sizeof(I));
       chain_inst_fill(o, sw.dir, I, tb4, tb8);
-      const int64_t N = 1ll << o.L;
       auto mk = [&](size_t bytes) {
         bufs.emplace_back(new DBuf());
         bufs.back()->alloc(bytes);
         return bufs.back()->p;
       };
-      I.P = mk((size_t)(sw.zb ? 16 * N : 4 * N) * (tangent_bufs ? 16 : 8));
-      I.fold = mk((size_t)N * 8);
+      size_t part[2];
+      sw.chain_bytes(o, tangent_bufs ? 16 : 8, part);
+      I.P = mk(part[0]);
+      I.Q = mk(part[1]);
       I.ldv = (o.n + 1) & ~(int64_t)1;
       I.V = static_cast<double*>(mk((size_t)(m + 1) * I.ldv * 8));
       I.w = static_cast<double*>(mk((size_t)o.n * 8));
-      I.x32 = static_cast<float*>(mk((size_t)o.n * 4));
+      I.u = mk((size_t)o.n * 8);
       np4max = std::max(np4max, I.np4);
       np8max = std::max(np8max, I.np8);
       for (int p = 0; p < I.np4; ++p) smem4 = std::max(smem4, chain_pass_smem(I.p4[p], sw.zb, 4));
@@ -554,14 +564,7 @@ struct Wave {
   const int2* km() const { return kmd.as<int2>(); }
 
   int product(int mode, int theta = 0) {
-    int nl = 0;
-    if (mode == kModeF32) {
-      sw_to_f32<<<(unsigned)nrblk, 256, 0, sw.s>>>(I(), km(), rstart.as<int64_t>(), count);
-      TM_CKK("sw_to_f32");
-      ++nl;
-    }
-    nl += chain_batch_product(B, km(), mode, sw.s, theta);
-    return nl;
+    return chain_batch_product(B, km(), mode, sw.s, theta);
   }
 
   // one Arnoldi step of every member taking part (each at its own column)

@@ -30,6 +30,7 @@ struct TreeLevels {
   int nbits;             // bits of a representative
   int b[kTreeMaxLevels + 1];
   uint2* nodes[kTreeMaxLevels + 1];  // levels 0 .. nlev - 1
+  uint16_t* words[kTreeMaxLevels + 1];
 };
 
 // length of the prefix that representative r shares with r - 1 (-1: r = 0)
@@ -112,6 +113,7 @@ __global__ void __launch_bounds__(kTreeBlock) tree_fill_kernel(const uint32_t* _
       uint2* nd = T.nodes[i - 1] + parent;
       atomicOr(&nd->y, 1u << word);
       if (c < T.b[i - 1]) nd->x = node;
+      if (T.words[i]) T.words[i][node] = (uint16_t)(s >> (T.nbits - T.b[i]));
     }
     parent = node;
     __syncthreads();
@@ -121,8 +123,9 @@ __global__ void __launch_bounds__(kTreeBlock) tree_fill_kernel(const uint32_t* _
 }  // namespace
 
 // Levels after steps[0], steps[0] + steps[1], ... bits (each step at most 5
-// bits, together nbits) of the representatives in op.idx.
-void build_prefix_tree(const Op& op, int nbits, const std::vector<int>& steps, PrefixTree& out) {
+// bits, together nbits) of the representatives in op.idx; words: with the
+// last 16 bits of every node's prefix.
+void build_prefix_tree(const Op& op, int nbits, const std::vector<int>& steps, bool words, PrefixTree& out) {
   const int64_t n = op.n;
   cudaStream_t s = op.stream;
   const int nlev = (int)steps.size();
@@ -133,15 +136,15 @@ void build_prefix_tree(const Op& op, int nbits, const std::vector<int>& steps, P
   for (int i = 0; i < nlev; ++i) T.b[i + 1] = T.b[i] + steps[i];
   if (T.b[nlev] != nbits) fail(TM_ERR_ARG, "prefix tree: steps do not cover the state");
   const int64_t nblk = (n + kTreeBlock - 1) / kTreeBlock;
-  DBuf cnt, tot;
-  cnt.alloc((size_t)(nlev + 1) * nblk * 4);
-  tot.alloc((size_t)(nlev + 1) * 4);
+  DBuf cnt;  // counts per level and block, then the totals per level
+  cnt.alloc((size_t)(nlev + 1) * (nblk + 1) * 4);
+  uint32_t* tot = cnt.as<uint32_t>() + (size_t)(nlev + 1) * nblk;
   tree_count_kernel<<<(unsigned)nblk, kTreeBlock, 0, s>>>(op.idx.as<uint32_t>(), n, T, cnt.as<uint32_t>());
   TM_CKK("tree_count");
-  tree_scan_kernel<<<nlev + 1, kTreeBlock, 0, s>>>(cnt.as<uint32_t>(), nblk, tot.as<uint32_t>());
+  tree_scan_kernel<<<nlev + 1, kTreeBlock, 0, s>>>(cnt.as<uint32_t>(), nblk, tot);
   TM_CKK("tree_scan");
   uint32_t h[kTreeMaxLevels + 1];
-  TM_CK(cudaMemcpyAsync(h, tot.p, (size_t)(nlev + 1) * 4, cudaMemcpyDeviceToHost, s));
+  TM_CK(cudaMemcpyAsync(h, tot, (size_t)(nlev + 1) * 4, cudaMemcpyDeviceToHost, s));
   TM_CK(cudaStreamSynchronize(s));
   out.nlev = nlev;
   int64_t sum = 0;
@@ -149,14 +152,17 @@ void build_prefix_tree(const Op& op, int nbits, const std::vector<int>& steps, P
     out.b[i] = T.b[i];
     out.n[i] = (i == 0) ? 1 : h[i];
     out.off[i] = sum;
-    if (i < nlev) sum += out.n[i];
+    sum += out.n[i];
   }
-  out.nodes.alloc((size_t)sum * sizeof(uint2));
-  TM_CK(cudaMemsetAsync(out.nodes.p, 0, (size_t)sum * sizeof(uint2), s));
+  out.nodes.alloc((size_t)out.off[nlev] * sizeof(uint2));
+  TM_CK(cudaMemsetAsync(out.nodes.p, 0, (size_t)out.off[nlev] * sizeof(uint2), s));
+  if (words) out.words.alloc((size_t)sum * 2);
   for (int i = 0; i < nlev; ++i) T.nodes[i] = out.level(i);
+  for (int i = 0; words && i <= nlev; ++i) T.words[i] = out.words.as<uint16_t>() + out.off[i];
   tree_fill_kernel<<<(unsigned)nblk, kTreeBlock, 0, s>>>(op.idx.as<uint32_t>(), n, T, cnt.as<uint32_t>());
   TM_CKK("tree_fill");
-  TM_CK(cudaStreamSynchronize(s));  // the counts are released on return
+  // the counts are released on return: in stream order, or by a synchronising
+  // cudaFree outside an allocation scope
 }
 
 }  // namespace ltm
