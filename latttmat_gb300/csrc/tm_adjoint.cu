@@ -11,11 +11,11 @@
 // where <g>_{l r} = sum l_i r_i g(s_i) / sum l_i r_i.  The first term is a
 // fused weighted reduction over the basis.  The second is nonzero only for
 // theta = betaJ (Th depends on K = betaJ alone for the Kronecker-core
-// operators).  It comes from a tangent sweep: the butterflies carry
-// (value, derivative) pairs, t = [[e^K, e^-K], [e^-K, e^K]] and
-// dt/dK = [[e^K, -e^-K], [-e^-K, e^K]].  The normfactor terms cancel: the
+// operators, which are symmetric: l = r).  It is a weighted sum of squared
+// Hadamard coefficients of Tv' r (kron_power, tm_core.cu).  The normfactor terms cancel: the
 // result is the derivative of the reported eigenvalue lambda/normfactor.
 #include <cmath>
+#include <functional>
 #include <vector>
 
 #include "tm_chain.h"
@@ -123,79 +123,19 @@ __global__ void diag_grad_kernel(GradParams p, const double* __restrict__ qr, co
   }
 }
 
-// v = Tvec .* qr expanded to the full space (reduced: through smap)
-__global__ void tangent_expand(const double* __restrict__ qr, const double* __restrict__ tv,
-                               const uint32_t* __restrict__ smap, int64_t N, double* __restrict__ v,
-                               double* __restrict__ dv) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t st = (int64_t)gridDim.x * blockDim.x;
-  for (; i < N; i += st) {
-    int64_t r = smap ? (int64_t)smap[i] : i;
-    v[i] = qr[r] * tv[r];
-    dv[i] = 0.0;
-  }
-}
-
-__device__ __forceinline__ int spad(int e) { return e + (e >> 5); }
-
-// dual-number butterfly pass over bits [lo, lo+nb) (+ cb contiguous bits)
-__global__ void dual_sweep_kernel(double* __restrict__ v, double* __restrict__ dv, int lo, int nb, int cb, double a,
-                                  double b) {
-  extern __shared__ double sm[];
-  const int tile = 1 << (nb + cb);
-  double* sv = sm;
-  double* sd = sm + tile + tile / 32 + 1;
-  const uint64_t outer = blockIdx.x;
-  const uint64_t lob = (uint64_t)(lo - cb);
-  const uint64_t base = ((outer & ((1ull << lob) - 1)) << cb) | ((outer >> lob) << (lo + nb));
-  auto gidx = [&](int e) -> uint64_t {
-    return base | (uint64_t)(e & ((1 << cb) - 1)) | ((uint64_t)(e >> cb) << lo);
-  };
-  for (int e = threadIdx.x; e < tile; e += blockDim.x) {
-    uint64_t i = gidx(e);
-    sv[spad(e)] = v[i];
-    sd[spad(e)] = dv[i];
-  }
-  __syncthreads();
-  for (int bb = 0; bb < nb; ++bb) {
-    const int bit = cb + bb;
-    for (int q = threadIdx.x; q < tile / 2; q += blockDim.x) {
-      int lowm = (1 << bit) - 1;
-      int e0 = ((q & ~lowm) << 1) | (q & lowm), e1 = e0 | (1 << bit);
-      double x0 = sv[spad(e0)], x1 = sv[spad(e1)];
-      double d0 = sd[spad(e0)], d1 = sd[spad(e1)];
-      sv[spad(e0)] = a * x0 + b * x1;
-      sv[spad(e1)] = b * x0 + a * x1;
-      sd[spad(e0)] = a * d0 + b * d1 + (a * x0 - b * x1);
-      sd[spad(e1)] = b * d0 + a * d1 + (-b * x0 + a * x1);
-    }
-    __syncthreads();
-  }
-  for (int e = threadIdx.x; e < tile; e += blockDim.x) {
-    uint64_t i = gidx(e);
-    v[i] = sv[spad(e)];
-    dv[i] = sd[spad(e)];
-  }
-}
-
-// quad = sum_r ql_r * post_r * dv[state(r)]
-__global__ void tangent_contract(const double* __restrict__ dv, const double* __restrict__ ql,
-                                 const uint32_t* __restrict__ idx, const uint16_t* __restrict__ dup,
-                                 const double* __restrict__ tv, double pc, int64_t n, double* __restrict__ part) {
+// sum_i l_i y_i, block sums
+__global__ void __launch_bounds__(256) dot_kernel(const double* __restrict__ l, const double* __restrict__ y,
+                                                  int64_t n, double* __restrict__ part) {
   double acc = 0.0;
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t st = (int64_t)gridDim.x * blockDim.x;
-  for (; i < n; i += st) {
-    int64_t s = idx ? (int64_t)idx[i] : i;
-    double post = pc * tv[i] * (dup ? (double)dup[i] : 1.0);
-    acc += ql[i] * post * dv[s];
-  }
+  for (; i < n; i += st) acc = fma(l[i], y[i], acc);
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-  __shared__ double sh[32];
+  __shared__ double sh[8];
   if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = acc;
   __syncthreads();
   if (threadIdx.x == 0) {
-    double t = 0;
+    double t = 0.0;
     for (int q = 0; q < (int)(blockDim.x >> 5); ++q) t += sh[q];
     part[blockIdx.x] = t;
   }
@@ -209,7 +149,12 @@ int nblocks(int64_t n) {
 
 void ensure_state_map(Op& op);
 
-void matvec_aux_tangent(const Op& op, const double* x, double* y, const AuxCoef& db, int dir, cudaStream_t s);
+// the chain's tangent products by betaJ, kappa and (BNNNI) kappa2, each handed
+// to `take` before the next overwrites y (tm_aux.cu)
+void matvec_aux_tangents(const Op& op, const double* x, double* y, cudaStream_t s,
+                         const std::function<void(int)>& take);
+// v^T (dTh / dK) v of the Kronecker factor, block sums (tm_core.cu)
+int64_t kron_power(const Op& op, const double* x, DBuf& part, cudaStream_t s);
 
 // Aux-bit operators (DNNI, diagonal BNNNI): T = D_out C D_in with the
 // diagonal Boltzmann weights D (Tvec, times dup in the reduced output) and
@@ -217,27 +162,7 @@ void matvec_aux_tangent(const Op& op, const double* x, double* y, const AuxCoef&
 // b3 = e^{-+bJ k2}.  d ln(lambda) = 2 <g>_{lr} + <l, D_out (dC) D_in r> /
 // (lambda <l, r>); the second term is a tangent product of the chain
 // (matvec_aux_tangent) per parameter the gates depend on.
-static void adjoint_grad_aux(const Op& op, const double* dqr, const double* qlp, double lam, double wsum,
-                             double grad[4]) {
-  cudaStream_t s = op.stream;
-  const int64_t n = op.n;
-  const bool zb = (op.kind == K_ZBT || op.kind == K_ZBM);
-  DBuf y;
-  y.alloc((size_t)n * 8);
-  std::vector<double> yh(n), lh(n);
-  TM_CK(cudaMemcpyAsync(lh.data(), qlp ? qlp : dqr, (size_t)n * 8, cudaMemcpyDeviceToHost, s));
-  for (int t = 0; t < 3; ++t) {
-    if (t == 2 && !zb) break;  // DNNI gates do not depend on kappa2
-    const AuxCoef db = aux_coef_derivative(op.mp.betaJ, op.mp.kappa, op.mp.kappa2, t);
-    matvec_aux_tangent(op, dqr, y.as<double>(), db, 0, s);
-    TM_CK(cudaMemcpyAsync(yh.data(), y.p, (size_t)n * 8, cudaMemcpyDeviceToHost, s));
-    TM_CK(cudaStreamSynchronize(s));
-    double quad = 0.0;
-    for (int64_t i = 0; i < n; ++i) quad += lh[i] * yh[i];
-    grad[t] += quad / (lam * wsum);
-  }
-}
-
+// (the partial sums of every term come back in one copy)
 void adjoint_grad(const Op& op, const double* qr_h, const double* ql_h, double lam, double grad[4]) {
   const bool aux = (op.kind == K_ZBT || op.kind == K_ZBM || op.kind == K_XDT || op.kind == K_XDM);
   if (op.kind != K_XAT && op.kind != K_XAM && op.kind != K_XAM3 && !aux)
@@ -255,12 +180,30 @@ void adjoint_grad(const Op& op, const double* qr_h, const double* ql_h, double l
     qlp = dql.as<double>();
   }
   GradParams gp{op.kind, op.L, op.size1, op.size2, op.boundary, op.mp.betaJ, op.mp.kappa, op.mp.kappa2, op.mp.h};
-  int nb = nblocks(n);
-  part.alloc((size_t)nb * 5 * 8 + 64);
+  const int nb = nblocks(n);
+  part.alloc((size_t)nb * 8 * 8);  // 5 sums per block, then up to 3 quadratic forms
   diag_grad_kernel<<<nb, 256, 0, s>>>(gp, dqr.as<double>(), qlp, reduced ? op.idx.as<uint32_t>() : nullptr, n,
                                       part.as<double>());
   TM_CKK("diag_grad");
-  std::vector<double> hp((size_t)nb * 5);
+  const int nquad = !aux ? 1 : (op.kind == K_ZBT || op.kind == K_ZBM) ? 3 : 2;  // DNNI gates: no kappa2
+  std::vector<double> hp((size_t)nb * 5), hq;
+  DBuf quad;
+  int64_t per = nb;  // partial sums per quadratic form
+  if (aux) {
+    DBuf y;
+    y.alloc((size_t)n * 8);
+    matvec_aux_tangents(op, dqr.as<double>(), y.as<double>(), s, [&](int t) {
+      dot_kernel<<<nb, 256, 0, s>>>(qlp ? qlp : dqr.as<double>(), y.as<double>(), n,
+                                    part.as<double>() + (size_t)nb * (5 + t));
+      TM_CKK("grad_dot");
+    });
+    hp.resize((size_t)nb * (5 + nquad));
+  } else {
+    if (reduced) ensure_state_map(const_cast<Op&>(op));
+    per = kron_power(op, dqr.as<double>(), quad, s);
+    hq.resize((size_t)per);
+    TM_CK(cudaMemcpyAsync(hq.data(), quad.p, hq.size() * 8, cudaMemcpyDeviceToHost, s));
+  }
   TM_CK(cudaMemcpyAsync(hp.data(), part.p, hp.size() * 8, cudaMemcpyDeviceToHost, s));
   TM_CK(cudaStreamSynchronize(s));
   double sums[5] = {0, 0, 0, 0, 0};
@@ -268,52 +211,13 @@ void adjoint_grad(const Op& op, const double* qr_h, const double* ql_h, double l
     for (int k = 0; k < 5; ++k) sums[k] += hp[(size_t)b * 5 + k];
   const double wsum = sums[4];
   for (int k = 0; k < 4; ++k) grad[k] = 2.0 * sums[k] / wsum;
-  if (aux) {
-    adjoint_grad_aux(op, dqr.as<double>(), qlp, lam, wsum, grad);
-    return;
-  }
-
-  // tangent term for betaJ through the full space
-  if (reduced) ensure_state_map(const_cast<Op&>(op));
-  const int L = op.L;
-  const int64_t N = 1ll << L;
-  DBuf v, dv;
-  v.alloc((size_t)N * 8);
-  dv.alloc((size_t)N * 8);
-  tangent_expand<<<nblocks(N) * 4, 256, 0, s>>>(dqr.as<double>(), op.tvec.as<double>(),
-                                               reduced ? op.smap.as<uint32_t>() : nullptr, N, v.as<double>(),
-                                               dv.as<double>());
-  TM_CKK("tangent_expand");
-  const double K = op.mp.betaJ, a = std::exp(K), b = std::exp(-K);
-  const int NB = 11, CB = 4;
-  int lo = 0;
-  while (lo < L) {
-    int cb = (lo == 0) ? 0 : std::min(CB, lo);
-    int nbits = std::min(L - lo, NB - cb);
-    int tile = 1 << (nbits + cb);
-    size_t shm = (size_t)2 * (tile + tile / 32 + 1) * 8;
-    int64_t nblk = (int64_t)1 << (L - nbits - cb);
-    dual_sweep_kernel<<<(unsigned)nblk, std::min(256, std::max(32, tile / 2)), shm, s>>>(v.as<double>(),
-                                                                                      dv.as<double>(), lo, nbits,
-                                                                                      cb, a, b);
-    TM_CKK("dual_sweep");
-    lo += nbits;
-  }
   const double pc = (op.kind == K_XAT) ? op.normfactor : 1.0;
-  DBuf part2;
-  int nb2 = nblocks(n);
-  part2.alloc((size_t)nb2 * 8 + 64);
-  tangent_contract<<<nb2, 256, 0, s>>>(dv.as<double>(), qlp ? qlp : dqr.as<double>(),
-                                       reduced ? op.idx.as<uint32_t>() : nullptr,
-                                       reduced ? op.dup.as<uint16_t>() : nullptr, op.tvec.as<double>(), pc, n,
-                                       part2.as<double>());
-  TM_CKK("tangent_contract");
-  std::vector<double> h2(nb2);
-  TM_CK(cudaMemcpyAsync(h2.data(), part2.p, nb2 * 8, cudaMemcpyDeviceToHost, s));
-  TM_CK(cudaStreamSynchronize(s));
-  double quad = 0;
-  for (double x : h2) quad += x;
-  grad[0] += quad / (lam * wsum);
+  for (int t = 0; t < nquad; ++t) {
+    const double* h = aux ? hp.data() + (size_t)nb * (5 + t) : hq.data();
+    double q = 0.0;
+    for (int64_t b = 0; b < per; ++b) q += h[b];
+    grad[t] += pc * q / (lam * wsum);
+  }
 }
 
 }  // namespace ltm

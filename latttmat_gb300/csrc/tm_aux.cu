@@ -31,6 +31,7 @@
 // applied at the output.
 #include <algorithm>
 #include <cmath>
+#include <functional>
 #include <mutex>
 #include <type_traits>
 #include <vector>
@@ -1342,10 +1343,11 @@ double matvec_aux(const Op& op, const T* x, T* y, bool scaled, cudaStream_t s) {
 template double matvec_aux<float>(const Op&, const float*, float*, bool, cudaStream_t);
 template double matvec_aux<double>(const Op&, const double*, double*, bool, cudaStream_t);
 
-// Tangent product of the adjoint: y = D_out (dC/dtheta) D_in x, the chain
-// steps differentiated with respect to one parameter whose effect on the step
-// factors b1, b2, b3 is `db` (the Boltzmann weights Tvec held fixed), FP64.
-void matvec_aux_tangent(const Op& op, const double* x, double* y, const AuxCoef& db, int dir, cudaStream_t s) {
+// Tangent products of the adjoint: y = D_out (dC/dtheta) D_in x, the chain
+// steps differentiated with respect to betaJ, kappa and (BNNNI) kappa2 in turn
+// (the Boltzmann weights Tvec held fixed); take(t) uses y before the next.
+void matvec_aux_tangents(const Op& op, const double* x, double* y, cudaStream_t s,
+                         const std::function<void(int)>& take) {
   // pass buffers at 16 bytes per element (the operator's hold 8)
   const bool zb = (op.kind == K_ZBT || op.kind == K_ZBM);
   int tb = 0, th = 0;
@@ -1353,10 +1355,14 @@ void matvec_aux_tangent(const Op& op, const double* x, double* y, const AuxCoef&
   int64_t need[2];
   chain_buffer_elems(op, chain_plan(op, 16, tb), need);
   AllocStream guard(s);
-  DBuf P, Q;
-  P.alloc((size_t)need[0] * 16);
-  Q.alloc((size_t)need[1] * 16);
-  matvec_aux_dir<tangent, double>(op, x, y, false, dir, s, &db, P.p, Q.p);
+  DBuf P;
+  P.alloc((size_t)(need[0] + need[1]) * 16 + 16);
+  tangent* buf = P.as<tangent>();
+  for (int t = 0; t < (zb ? 3 : 2); ++t) {
+    const AuxCoef db = aux_coef_derivative(op.mp.betaJ, op.mp.kappa, op.mp.kappa2, t);
+    matvec_aux_dir<tangent, double>(op, x, y, false, 0, s, &db, buf, buf + need[0]);
+    take(t);
+  }
 }
 
 // FP64-accurate product in double-float arithmetic (the solver's refinement

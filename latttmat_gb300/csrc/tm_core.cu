@@ -39,11 +39,60 @@ Kron<T> kron_of(const Op& op) {
   return Kron<T>{(T)std::exp(-2.0 * std::fabs(op.mp.betaJ)), op.mp.betaJ < 0 ? 1 : 0};
 }
 
+// The Walsh-Hadamard transform (x0 + x1, x0 - x1), for the adjoint.
+struct Had {};
+
+template <class T, int NB>
+__device__ __forceinline__ void bfly(T (&v)[1 << NB], const Kron<T>& c) {
+  reg_bfly<T, NB>(v, c.r, c.swap);
+}
+template <class T, int NB>
+__device__ __forceinline__ void bfly(T (&v)[1 << NB], const Had&) {
+#pragma unroll
+  for (int lv = 0; lv < NB; ++lv)
+#pragma unroll
+    for (int i = 0; i < (1 << NB); ++i)
+      if (!(i & (1 << lv))) {
+        const T x0 = v[i], x1 = v[i | (1 << lv)];
+        v[i] = x0 + x1;
+        v[i | (1 << lv)] = x0 - x1;
+      }
+}
+// the two outputs of one butterfly (no exchange)
+template <class T>
+__device__ __forceinline__ T out0(const Kron<T>& c, T x0, T x1) { return fma_t(c.r, x1, x0); }
+template <class T>
+__device__ __forceinline__ T out1(const Kron<T>& c, T x0, T x1) { return fma_t(c.r, x0, x1); }
+template <class T>
+__device__ __forceinline__ T out0(const Had&, T x0, T x1) { return x0 + x1; }
+template <class T>
+__device__ __forceinline__ T out1(const Had&, T x0, T x1) { return x0 - x1; }
+template <class T>
+__device__ __forceinline__ bool swapped(const Kron<T>& c) { return c.swap; }
+__device__ __forceinline__ bool swapped(const Had&) { return false; }
+
+// Weights of the squared Hadamard coefficients by bit count (adjoint), and
+// the sum of one block's terms.
+struct PowerTab {
+  double d[33];
+};
+__device__ __forceinline__ void block_sum(double acc, double* __restrict__ part) {
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+  __shared__ double sh[32];
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = acc;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double t = 0.0;
+    for (int q = 0; q < (int)(blockDim.x >> 5); ++q) t += sh[q];
+    part[blockIdx.x] = t;
+  }
+}
+
 // ------------------------------------------------------------------ tile passes
 // One butterfly round on tile bits [G0, G0 + GS) of every row (a row is the
 // 2^nb mixed positions of one chunk position).
-template <class T, int G0, int GS>
-__device__ __forceinline__ void tile_round(T* sm, int nb, int cb, int pitch, const Kron<T>& c) {
+template <class T, int G0, int GS, class C>
+__device__ __forceinline__ void tile_round(T* sm, int nb, int cb, int pitch, const C& c) {
   const int fb = nb - GS;
   for (int f = threadIdx.x; f < (1 << (fb + cb)); f += blockDim.x) {
     const int g = f & ((1 << fb) - 1);
@@ -51,7 +100,7 @@ __device__ __forceinline__ void tile_round(T* sm, int nb, int cb, int pitch, con
     T v[1 << GS];
 #pragma unroll
     for (int i = 0; i < (1 << GS); ++i) v[i] = b[spad(i << G0)];
-    reg_bfly<T, GS>(v, c.r, c.swap);
+    bfly<T, GS>(v, c);
 #pragma unroll
     for (int i = 0; i < (1 << GS); ++i) b[spad(i << G0)] = v[i];
   }
@@ -60,8 +109,8 @@ __device__ __forceinline__ void tile_round(T* sm, int nb, int cb, int pitch, con
 
 constexpr int kTileMix = 11;  // most mixed bits of a tile
 
-template <class T, int KB, int R = 0>
-__device__ __forceinline__ void tile_rounds(T* sm, int nb, int cb, int pitch, const Kron<T>& c) {
+template <class T, int KB, class C, int R = 0>
+__device__ __forceinline__ void tile_rounds(T* sm, int nb, int cb, int pitch, const C& c) {
   constexpr int G0 = R * KB;
   const int left = nb - G0;
   if (left <= 0) return;
@@ -76,7 +125,7 @@ __device__ __forceinline__ void tile_rounds(T* sm, int nb, int cb, int pitch, co
       if (left == 1) tile_round<T, G0, 1>(sm, nb, cb, pitch, c);
     return;
   }
-  if constexpr ((R + 1) * KB < kTileMix) tile_rounds<T, KB, R + 1>(sm, nb, cb, pitch, c);
+  if constexpr ((R + 1) * KB < kTileMix) tile_rounds<T, KB, C, R + 1>(sm, nb, cb, pitch, c);
 }
 
 // x * pre * fac (load) and v * sc * fac (store) in the vector's type
@@ -115,7 +164,7 @@ __global__ void __launch_bounds__(512) kron_tile_kernel(const T* __restrict__ x,
     sm[(e & kmask) * pitch + spad(e >> cb)] = v;
   }
   __syncthreads();
-  tile_rounds<T, KB>(sm, nb, cb, pitch, c);
+  tile_rounds<T, KB, Kron<T>>(sm, nb, cb, pitch, c);
   for (int e = threadIdx.x; e < tile; e += blockDim.x) {
     const uint64_t i = base | (uint64_t)(e & kmask) | ((uint64_t)(e >> cb) << lo);
     T v = sm[(e & kmask) * pitch + spad(e >> cb)];
@@ -142,25 +191,42 @@ void launch_tile(int64_t nblocks, int threads, size_t shm, cudaStream_t s, const
 // (L = 12 in one 4096-element block took 38 us).  Threads: 16 elements each
 // (one round of four levels in registers) in large tiles, 2 or 4 in small
 // ones, so that all four schedulers of an SM have a warp.
+struct TilePass {
+  int nb, cb, kb, threads;
+  size_t shm;
+  int64_t nblocks;
+};
+int tile_passes(int L, size_t elem) {
+  const int most = (elem == 8) ? 9 : 10;
+  return (L <= 9) ? 1 : std::max(2, (L + most - 1) / most);
+}
+// the pass that starts at bit lo, with `left` passes to go
+TilePass tile_pass(int L, int lo, int left, size_t elem) {
+  TilePass t;
+  t.nb = (L - lo + left - 1) / left;
+  t.cb = std::min(std::min(4, lo), std::max(0, L - t.nb - 7));
+  const int tb = t.nb + t.cb;
+  t.kb = (tb >= 11) ? 4 : (tb >= 9 ? 2 : 1);
+  t.threads = std::min(512, std::max(32, (1 << tb) >> t.kb));
+  t.shm = ((size_t)(((1 << t.nb) + (1 << t.nb) / 32) | 1) << t.cb) * elem;
+  t.nblocks = (int64_t)1 << (L - tb);
+  return t;
+}
 template <class T>
 void run_sweep(const Op& op, const T* x, T* out, int load_mode, const double* pre, double fin, const uint32_t* map,
                int store_mode, const double* scale, double fout, cudaStream_t s) {
   const int L = op.L;
   const Kron<T> c = kron_of<T>(op);
-  const int most = (sizeof(T) == 8) ? 9 : 10;
-  const int npass = (L <= 9) ? 1 : std::max(2, (L + most - 1) / most);
+  const int npass = tile_passes(L, sizeof(T));
   const ScaleF fi = scale_factor(fin), fo = scale_factor(fout);
   int lo = 0;
   const T* src = x;
   for (int p = 0; p < npass; ++p) {
-    const int nb = (L - lo + npass - p - 1) / (npass - p);
-    const int cb = std::min(std::min(4, lo), std::max(0, L - nb - 7));
-    const int tb = nb + cb;
-    const int kb = (tb >= 11) ? 4 : (tb >= 9 ? 2 : 1);
-    const int threads = std::min(512, std::max(32, (1 << tb) >> kb));
-    const size_t shm = ((size_t)(((1 << nb) + (1 << nb) / 32) | 1) << cb) * sizeof(T);
+    const TilePass t = tile_pass(L, lo, npass - p, sizeof(T));
+    const int nb = t.nb, cb = t.cb, kb = t.kb, threads = t.threads;
+    const size_t shm = t.shm;
+    const int64_t nblocks = t.nblocks;
     const bool first = (p == 0), last = (p == npass - 1);
-    const int64_t nblocks = (int64_t)1 << (L - tb);
     auto go = [&](auto k) {
       launch_tile<T, decltype(k)::value>(nblocks, threads, shm, s, src, out, lo, nb, cb, c, first ? load_mode : 0, pre,
                                          fi, map, last ? store_mode : 0, scale, fo);
@@ -176,14 +242,50 @@ void run_sweep(const Op& op, const T* x, T* out, int load_mode, const double* pr
   }
 }
 
+// A pass of the Hadamard transform, as kron_tile_kernel: input x, through map
+// or times pre where given; the last pass stores nothing but the block's sum
+// of d[bit count] value^2.  Bound by the FP64 pipe (one addition per element
+// and level).
+template <int KB>
+__global__ void __launch_bounds__(512) had_tile_kernel(const double* x, double* out, int lo, int nb, int cb,
+                                                       const uint32_t* __restrict__ map,
+                                                       const double* __restrict__ pre, double* __restrict__ part,
+                                                       PowerTab pw) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  double* sm = reinterpret_cast<double*>(smem_raw);
+  const int tile = 1 << (nb + cb), kmask = (1 << cb) - 1;
+  const int pitch = spad(1 << nb) | 1;
+  const uint64_t outer = blockIdx.x;
+  const int low_outer = lo - cb;
+  const uint64_t base = ((outer & ((1ull << low_outer) - 1)) << cb) | ((outer >> low_outer) << (lo + nb));
+  for (int e = threadIdx.x; e < tile; e += blockDim.x) {
+    const uint64_t i = base | (uint64_t)(e & kmask) | ((uint64_t)(e >> cb) << lo);
+    double v = map ? x[map[i]] : x[i];
+    if (pre) v *= pre[i];
+    sm[(e & kmask) * pitch + spad(e >> cb)] = v;
+  }
+  __syncthreads();
+  tile_rounds<double, KB, Had>(sm, nb, cb, pitch, Had());
+  double acc = 0.0;
+  for (int e = threadIdx.x; e < tile; e += blockDim.x) {
+    const uint64_t i = base | (uint64_t)(e & kmask) | ((uint64_t)(e >> cb) << lo);
+    const double v = sm[(e & kmask) * pitch + spad(e >> cb)];
+    if (part)
+      acc = fma(pw.d[__popcll(i)], v * v, acc);
+    else
+      out[i] = v;
+  }
+  if (part) block_sum(acc, part);
+}
+
 // ------------------------------------------------------------------ prefix-tree passes
 // The butterflies (x0 + r x1, x1 + r x0) on a thread's 2^KB values, top bit
 // first, forming output blocks below which the mask has a child.  The mask is
 // the same for the whole warp and each block of outputs is one branch: a
 // predicated or selected FMA would take its slot on the FP64 pipe all the
 // same.  The last two levels of a block of four outputs go together.
-template <class T, int KB, int B = KB - 1, int H = 0>
-__device__ __forceinline__ void tree_bfly(T (&v)[1 << KB], uint32_t mask, T r) {
+template <class T, int KB, class C, int B = KB - 1, int H = 0>
+__device__ __forceinline__ void tree_bfly(T (&v)[1 << KB], uint32_t mask, const C& c) {
   constexpr uint32_t kSub = (1u << (1 << B)) - 1u;  // the 2^B leaves of one output block
   constexpr int J0 = (2 * H) << B, J1 = (2 * H + 1) << B;
   const bool a0 = (mask >> J0) & kSub, a1 = (mask >> J1) & kSub;
@@ -191,22 +293,22 @@ __device__ __forceinline__ void tree_bfly(T (&v)[1 << KB], uint32_t mask, T r) {
 #pragma unroll
     for (int i = 0; i < (1 << B); ++i) {
       const T x0 = v[J0 + i], x1 = v[J1 + i];
-      v[J0 + i] = fma_t(r, x1, x0);
-      v[J1 + i] = fma_t(r, x0, x1);
+      v[J0 + i] = out0<T>(c, x0, x1);
+      v[J1 + i] = out1<T>(c, x0, x1);
     }
     if constexpr (B > 0) {
-      tree_bfly<T, KB, B - 1, 2 * H>(v, B == 1 ? 3u << J0 : mask, r);
-      tree_bfly<T, KB, B - 1, 2 * H + 1>(v, B == 1 ? 3u << J1 : mask, r);
+      tree_bfly<T, KB, C, B - 1, 2 * H>(v, B == 1 ? 3u << J0 : mask, c);
+      tree_bfly<T, KB, C, B - 1, 2 * H + 1>(v, B == 1 ? 3u << J1 : mask, c);
     }
   } else if constexpr (B > 1) {
     if (a0) {
 #pragma unroll
-      for (int i = 0; i < (1 << B); ++i) v[J0 + i] = fma_t(r, v[J1 + i], v[J0 + i]);
-      tree_bfly<T, KB, B - 1, 2 * H>(v, mask, r);
+      for (int i = 0; i < (1 << B); ++i) v[J0 + i] = out0<T>(c, v[J0 + i], v[J1 + i]);
+      tree_bfly<T, KB, C, B - 1, 2 * H>(v, mask, c);
     } else if (a1) {
 #pragma unroll
-      for (int i = 0; i < (1 << B); ++i) v[J1 + i] = fma_t(r, v[J0 + i], v[J1 + i]);
-      tree_bfly<T, KB, B - 1, 2 * H + 1>(v, mask, r);
+      for (int i = 0; i < (1 << B); ++i) v[J1 + i] = out1<T>(c, v[J0 + i], v[J1 + i]);
+      tree_bfly<T, KB, C, B - 1, 2 * H + 1>(v, mask, c);
     }
   }
 }
@@ -222,17 +324,22 @@ __device__ __forceinline__ void tree_bfly(T (&v)[1 << KB], uint32_t mask, T r) {
 //          with the input scaling (u = x tvec gin) folded in where tv is given
 //          (few enough rows that gathering the weights too costs less than a
 //          launch);
-//   LAST:  the children are the representatives: y = post dup tvec value.
+//   LAST:  the children are the representatives: y = post dup tvec value; of
+//          the Hadamard transform (C = Had) the sum over the block's
+//          representatives of dup d[bit count] value^2.
 // Bound by the FP64 pipe in FP64 (78% busy in the first level at L = 25), by
 // the map gather in FP32.  FP64 products against three full-space tile passes
 // with two FP64 operations per element and bit: x-ANNNI at L = 25 without
 // flip 3.17 -> 0.465 ms, the 5x5 layer with flip 3.16 -> 0.142 ms.
-template <class T, int KB, bool FIRST, bool LAST>
+template <class T, int KB, bool FIRST, bool LAST, class C>
 __global__ void __launch_bounds__(256) kron_tree_kernel(const T* __restrict__ src, const uint32_t* __restrict__ smap,
                                                         const uint2* __restrict__ nodes, int64_t nnode, int rest,
-                                                        Kron<T> c, T* __restrict__ dst,
+                                                        C c, T* __restrict__ dst,
                                                         const uint16_t* __restrict__ dup,
-                                                        const double* __restrict__ tv, double post) {
+                                                        const double* __restrict__ tv, double post,
+                                                        const uint32_t* __restrict__ idx, PowerTab pw) {
+  constexpr bool kPower = LAST && std::is_same<C, Had>::value;
+  double acc = 0.0;
   const int64_t total = nnode << rest;
   const int64_t span = (total + 31) & ~(int64_t)31;  // whole warps (the mask is combined over the warp)
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < span; t += (int64_t)gridDim.x * blockDim.x) {
@@ -246,7 +353,7 @@ __global__ void __launch_bounds__(256) kron_tree_kernel(const T* __restrict__ sr
 #pragma unroll
       for (int j = 0; j < (1 << KB); ++j) {
         const int64_t i = ((int64_t)j << rest) | low;
-        at[j] = __ldcs(smap + (c.swap ? ((int64_t)1 << (rest + KB)) - 1 - i : i));
+        at[j] = __ldcs(smap + (swapped(c) ? ((int64_t)1 << (rest + KB)) - 1 - i : i));
       }
 #pragma unroll
       for (int j = 0; j < (1 << KB); ++j) v[j] = __ldg(src + at[j]);
@@ -259,12 +366,14 @@ __global__ void __launch_bounds__(256) kron_tree_kernel(const T* __restrict__ sr
 #pragma unroll
       for (int j = 0; j < (1 << KB); ++j) v[j] = p[(int64_t)j << rest];
     }
-    tree_bfly<T, KB>(v, __reduce_or_sync(0xffffffffu, nd.y), c.r);
+    tree_bfly<T, KB, C>(v, __reduce_or_sync(0xffffffffu, nd.y), c);
     int64_t child = nd.x;
 #pragma unroll
     for (int j = 0; j < (1 << KB); ++j) {
       if ((nd.y >> j) & 1u) {
-        if constexpr (LAST)
+        if constexpr (kPower)
+          acc = fma((double)dup[child] * pw.d[__popc(idx[child])], (double)v[j] * (double)v[j], acc);
+        else if constexpr (LAST)
           dst[child] = (T)((double)v[j] * post * (double)dup[child] * tv[child]);
         else
           dst[(child << rest) | low] = v[j];
@@ -272,6 +381,7 @@ __global__ void __launch_bounds__(256) kron_tree_kernel(const T* __restrict__ sr
       }
     }
   }
+  if constexpr (kPower) block_sum(acc, dst);
 }
 
 int grid_for(int64_t n, int threads = 256) {
@@ -280,13 +390,19 @@ int grid_for(int64_t n, int threads = 256) {
   return (int)std::max<int64_t>(1, std::min(b, cap));
 }
 
-template <class T, bool FIRST, bool LAST>
-void launch_tree(int kb, const T* src, const uint32_t* smap, const uint2* nodes, int64_t nnode, int rest,
-                 const Kron<T>& c, T* dst, const uint16_t* dup, const double* tv, double post, cudaStream_t s) {
-  const int grid = (int)std::min<int64_t>(((nnode << rest) + 255) / 256, (int64_t)num_sms() * 64);
+int tree_grid(int64_t nnode, int rest) {
+  return (int)std::min<int64_t>(((nnode << rest) + 255) / 256, (int64_t)num_sms() * 64);
+}
+
+template <class T, bool FIRST, bool LAST, class C>
+void launch_tree(int kb, const T* src, const uint32_t* smap, const uint2* nodes, int64_t nnode, int rest, const C& c,
+                 T* dst, const uint16_t* dup, const double* tv, double post, cudaStream_t s,
+                 const uint32_t* idx = nullptr, const PowerTab* pw = nullptr) {
+  const int grid = tree_grid(nnode, rest);
+  const PowerTab tab = pw ? *pw : PowerTab{};
   auto go = [&](auto k) {
-    kron_tree_kernel<T, decltype(k)::value, FIRST, LAST><<<grid, 256, 0, s>>>(src, smap, nodes, nnode, rest, c, dst,
-                                                                              dup, tv, post);
+    kron_tree_kernel<T, decltype(k)::value, FIRST, LAST, C><<<grid, 256, 0, s>>>(src, smap, nodes, nnode, rest, c, dst,
+                                                                                 dup, tv, post, idx, tab);
   };
   switch (kb) {
     case 4: go(std::integral_constant<int, 4>()); break;
@@ -313,11 +429,11 @@ void run_tree(const Op& op, const T* u, T* y, bool fold, double gin, double post
     T* dst = last ? y : buf[i & 1];
     const uint32_t* smap = op.smap.as<uint32_t>();
     if (first)
-      launch_tree<T, true, false>(kb, src, smap, t.level(i), t.n[i], rest, c, dst, dup, fold ? tv : nullptr, gin, s);
+      launch_tree<T, true, false, Kron<T>>(kb, src, smap, t.level(i), t.n[i], rest, c, dst, dup, fold ? tv : nullptr, gin, s);
     else if (!last)
-      launch_tree<T, false, false>(kb, src, smap, t.level(i), t.n[i], rest, c, dst, dup, tv, post, s);
+      launch_tree<T, false, false, Kron<T>>(kb, src, smap, t.level(i), t.n[i], rest, c, dst, dup, tv, post, s);
     else
-      launch_tree<T, false, true>(kb, src, smap, t.level(i), t.n[i], rest, c, dst, dup, tv, post, s);
+      launch_tree<T, false, true, Kron<T>>(kb, src, smap, t.level(i), t.n[i], rest, c, dst, dup, tv, post, s);
     src = dst;
   }
 }
@@ -340,7 +456,7 @@ __global__ void __launch_bounds__(512) kron_small_kernel(const T* x, const uint3
     sm[spad(i)] = (T)((double)x[q] * tv[q] * gin);
   }
   __syncthreads();
-  tile_rounds<T, 2>(sm, L, 0, 0, c);
+  tile_rounds<T, 2, Kron<T>>(sm, L, 0, 0, c);
   for (int i = threadIdx.x; i < n; i += blockDim.x)
     y[i] = (T)((double)sm[spad((int)idx[i])] * post * (double)dup[i] * tv[i]);
 }
@@ -366,6 +482,23 @@ __global__ void contract_kernel(const T* __restrict__ z, const uint32_t* __restr
 
 }  // namespace
 
+// four bits per level, the odd ones out in threes at the end
+static std::vector<int> tree_steps(int L) {
+  std::vector<int> steps;
+  const int nlev = (L + 3) / 4;
+  for (int i = 0, b = 0; i < nlev; ++i) {
+    steps.push_back((L - b + nlev - i - 1) / (nlev - i));
+    b += steps.back();
+  }
+  return steps;
+}
+// elements of the two buffers that the levels write in turn
+static void tree_buffer_elems(const Op& op, int64_t most[2]) {
+  most[0] = most[1] = 1;
+  for (int i = 0; i + 1 < op.tree.nlev; ++i)
+    most[i & 1] = std::max(most[i & 1], op.tree.n[i + 1] << (op.L - op.tree.b[i + 1]));
+}
+
 // Constants of a Kronecker-core operator, and the workspace of its generic
 // reduced product: the prefix tree of the translation groups with its two
 // level buffers, or the full-space vector.
@@ -390,19 +523,106 @@ void build_bfly(Op& op) {
     op.ws_a.alloc((size_t)op.nstate * 8);
     return;
   }
-  // four bits per level, the odd ones out in threes at the end
-  std::vector<int> steps;
-  const int nlev = (op.L + 3) / 4;
-  for (int i = 0, b = 0; i < nlev; ++i) {
-    steps.push_back((op.L - b + nlev - i - 1) / (nlev - i));
-    b += steps.back();
-  }
-  build_prefix_tree(op, op.L, steps, false, op.tree);
-  int64_t most[2] = {1, 1};
-  for (int i = 0; i + 1 < nlev; ++i)
-    most[i & 1] = std::max(most[i & 1], op.tree.n[i + 1] << (op.L - op.tree.b[i + 1]));
+  build_prefix_tree(op, op.L, tree_steps(op.L), false, op.tree);
+  int64_t most[2];
+  tree_buffer_elems(op, most);
   op.ws_a.alloc((size_t)most[0] * 8);
   op.ws_b.alloc((size_t)most[1] * 8);
+}
+
+// v^T (dTh / dK) v of the Kronecker factor for v = Tvec x expanded to the full
+// space (x: device, the operator's rows), as block sums in part; returns
+// their number.  All 2 x 2 factors are diagonal in the Hadamard basis, so
+//   v^T dTh v = 2^-L sum_w lambda'_{|w|} vhat(w)^2,
+//   lambda_k = (2 cosh K)^(L-k) (2 sinh K)^k,
+// one addition per element and level where tangent pairs (value, derivative)
+// took eight FP64 operations per pair and level, and no cancellation that T
+// itself does not have.  vhat has the symmetries of v: with translations and
+// no spin flip only representatives' prefixes are formed (as in the
+// products); a flip-symmetric v has vhat(w) = 0 at odd |w| and twice the
+// transform of its lower half at even |w|.  A gradient of the reduced L = 24
+// operator (no flip) took 4.79 ms with tangent pairs on all 2^24 states and
+// takes 0.39 ms, its copies included.
+int64_t kron_power(const Op& op, const double* x, DBuf& part, cudaStream_t s) {
+  const int L = op.L;
+  const double c2 = 2.0 * std::cosh(op.mp.betaJ), s2 = 2.0 * std::sinh(op.mp.betaJ);
+  auto dlam = [&](int k) {  // (s^(L-k) d^k)' with s' = d, d' = s
+    double r = 0.0;
+    if (k < L) r += (L - k) * std::pow(c2, L - k - 1) * std::pow(s2, k + 1);
+    if (k > 0) r += k * std::pow(c2, L - k + 1) * std::pow(s2, k - 1);
+    return r * std::ldexp(1.0, -L);
+  };
+  const double* tv = op.tvec.as<double>();
+  const bool reduced = op.kind != K_XAT;
+  const bool shifts = (op.kind == K_XAM && op.grp.periodic) || op.kind == K_XAM3;
+  PowerTab pw{};
+  DBuf u, a, b;
+  if (reduced) {
+    u.alloc((size_t)op.n * 8);
+    scale_in_kernel<double><<<grid_for(op.n), 256, 0, s>>>(x, tv, 1.0, u.as<double>(), op.n);
+    TM_CKK("scale_in");
+  }
+  const uint32_t* smap = op.smap.as<uint32_t>();
+  if (reduced && shifts && !op.grp.flip && L > kSmallBits) {
+    // (an even/odd operator has no tree of its own; it keeps this one)
+    if (!op.tree.nlev) build_prefix_tree(op, L, tree_steps(L), false, const_cast<Op&>(op).tree);
+    const PrefixTree& t = op.tree;
+    for (int k = 0; k <= L; ++k) pw.d[k] = dlam(k);
+    int64_t most[2];
+    tree_buffer_elems(op, most);
+    a.alloc((size_t)most[0] * 8);
+    b.alloc((size_t)most[1] * 8);
+    const double* src = u.as<double>();
+    const uint16_t* dup = op.dup.as<uint16_t>();
+    const Had had;
+    for (int i = 0; i < t.nlev; ++i) {
+      const int kb = t.b[i + 1] - t.b[i], rest = L - t.b[i + 1];
+      double* dst = (i & 1) ? b.as<double>() : a.as<double>();
+      if (i == 0) {
+        launch_tree<double, true, false, Had>(kb, src, smap, t.level(i), t.n[i], rest, had, dst, dup, nullptr, 1.0, s);
+      } else if (i + 1 < t.nlev) {
+        launch_tree<double, false, false, Had>(kb, src, smap, t.level(i), t.n[i], rest, had, dst, dup, nullptr, 1.0, s);
+      } else {
+        const int64_t np = tree_grid(t.n[i], rest);
+        part.alloc((size_t)np * 8);
+        launch_tree<double, false, true, Had>(kb, src, smap, t.level(i), t.n[i], rest, had, part.as<double>(), dup,
+                                              nullptr, 1.0, s, op.idx.as<uint32_t>(), &pw);
+        return np;
+      }
+      src = dst;
+    }
+  }
+  const bool half = reduced && op.grp.flip;
+  const int n = half ? L - 1 : L;
+  for (int k = 0; k <= n; ++k) pw.d[k] = half ? 4.0 * dlam(k + (k & 1)) : dlam(k);
+  a.alloc(((size_t)1 << n) * 8);
+  int lo = 0;
+  const int npass = tile_passes(n, 8);
+  int64_t np = 0;
+  for (int p = 0; p < npass; ++p) {
+    const TilePass t = tile_pass(n, lo, npass - p, 8);
+    const bool last = (p == npass - 1);
+    np = t.nblocks;
+    if (last) part.alloc((size_t)np * 8);
+    const double* src = p ? a.as<double>() : (reduced ? u.as<double>() : x);
+    auto go = [&](auto k) {
+      constexpr int KB = decltype(k)::value;
+      if (t.shm > 48 * 1024) raise_smem_limit((const void*)had_tile_kernel<KB>, t.shm);
+      had_tile_kernel<KB><<<(unsigned)t.nblocks, t.threads, t.shm, s>>>(src, a.as<double>(), lo, t.nb, t.cb,
+                                                                       (p || !reduced) ? nullptr : smap,
+                                                                       (p || reduced) ? nullptr : tv,
+                                                                       last ? part.as<double>() : nullptr, pw);
+    };
+    if (t.kb == 4)
+      go(std::integral_constant<int, 4>());
+    else if (t.kb == 2)
+      go(std::integral_constant<int, 2>());
+    else
+      go(std::integral_constant<int, 1>());
+    TM_CKK("had_tile");
+    lo += t.nb;
+  }
+  return np;
 }
 
 // y = T x on the full space (K_XAT) or on the reduced basis through the full
