@@ -29,47 +29,9 @@ namespace ltm {
 namespace {
 
 template <class T>
-struct Kron {
-  T r;       // min(a, b) / max(a, b)
-  int swap;  // b > a
-};
-
-template <class T>
 Kron<T> kron_of(const Op& op) {
   return Kron<T>{(T)std::exp(-2.0 * std::fabs(op.mp.betaJ)), op.mp.betaJ < 0 ? 1 : 0};
 }
-
-// The Walsh-Hadamard transform (x0 + x1, x0 - x1), for the adjoint.
-struct Had {};
-
-template <class T, int NB>
-__device__ __forceinline__ void bfly(T (&v)[1 << NB], const Kron<T>& c) {
-  reg_bfly<T, NB>(v, c.r, c.swap);
-}
-template <class T, int NB>
-__device__ __forceinline__ void bfly(T (&v)[1 << NB], const Had&) {
-#pragma unroll
-  for (int lv = 0; lv < NB; ++lv)
-#pragma unroll
-    for (int i = 0; i < (1 << NB); ++i)
-      if (!(i & (1 << lv))) {
-        const T x0 = v[i], x1 = v[i | (1 << lv)];
-        v[i] = x0 + x1;
-        v[i | (1 << lv)] = x0 - x1;
-      }
-}
-// the two outputs of one butterfly (no exchange)
-template <class T>
-__device__ __forceinline__ T out0(const Kron<T>& c, T x0, T x1) { return fma_t(c.r, x1, x0); }
-template <class T>
-__device__ __forceinline__ T out1(const Kron<T>& c, T x0, T x1) { return fma_t(c.r, x0, x1); }
-template <class T>
-__device__ __forceinline__ T out0(const Had&, T x0, T x1) { return x0 + x1; }
-template <class T>
-__device__ __forceinline__ T out1(const Had&, T x0, T x1) { return x0 - x1; }
-template <class T>
-__device__ __forceinline__ bool swapped(const Kron<T>& c) { return c.swap; }
-__device__ __forceinline__ bool swapped(const Had&) { return false; }
 
 // Weights of the squared Hadamard coefficients by bit count (adjoint), and
 // the sum of one block's terms.
@@ -89,60 +51,29 @@ __device__ __forceinline__ void block_sum(double acc, double* __restrict__ part)
 }
 
 // ------------------------------------------------------------------ tile passes
-// One butterfly round on tile bits [G0, G0 + GS) of every row (a row is the
-// 2^nb mixed positions of one chunk position).
-template <class T, int G0, int GS, class C>
-__device__ __forceinline__ void tile_round(T* sm, int nb, int cb, int pitch, const C& c) {
-  const int fb = nb - GS;
-  for (int f = threadIdx.x; f < (1 << (fb + cb)); f += blockDim.x) {
-    const int g = f & ((1 << fb) - 1);
-    T* b = sm + (f >> fb) * pitch + spad((g & ((1 << G0) - 1)) | ((g >> G0) << (G0 + GS)));
-    T v[1 << GS];
-#pragma unroll
-    for (int i = 0; i < (1 << GS); ++i) v[i] = b[spad(i << G0)];
-    bfly<T, GS>(v, c);
-#pragma unroll
-    for (int i = 0; i < (1 << GS); ++i) b[spad(i << G0)] = v[i];
-  }
-  __syncthreads();
-}
-
-constexpr int kTileMix = 11;  // most mixed bits of a tile
-
-template <class T, int KB, class C, int R = 0>
-__device__ __forceinline__ void tile_rounds(T* sm, int nb, int cb, int pitch, const C& c) {
-  constexpr int G0 = R * KB;
-  const int left = nb - G0;
-  if (left <= 0) return;
-  if (left >= KB) {
-    tile_round<T, G0, KB>(sm, nb, cb, pitch, c);
-  } else {
-    if constexpr (KB > 3)
-      if (left == 3) tile_round<T, G0, 3>(sm, nb, cb, pitch, c);
-    if constexpr (KB > 2)
-      if (left == 2) tile_round<T, G0, 2>(sm, nb, cb, pitch, c);
-    if constexpr (KB > 1)
-      if (left == 1) tile_round<T, G0, 1>(sm, nb, cb, pitch, c);
-    return;
-  }
-  if constexpr ((R + 1) * KB < kTileMix) tile_rounds<T, KB, C, R + 1>(sm, nb, cb, pitch, c);
-}
-
 // x * pre * fac (load) and v * sc * fac (store) in the vector's type
+// (FP64 loads take no factor: it costs a slot on the FP64 pipe per element, and
+// the output factor can hold it)
 __device__ __forceinline__ double weigh(double v, double t, const ScaleF& f) { return v * t * f.f64; }
+__device__ __forceinline__ double weigh_load(double v, double t, const ScaleF&) { return v * t; }
+__device__ __forceinline__ float weigh_load(float v, double t, const ScaleF& f) { return scale_round(v, t, f); }
 __device__ __forceinline__ float weigh(float v, double t, const ScaleF& f) { return scale_round(v, t, f); }
 
 // One pass: 2^nb positions of bits [lo, lo + nb) times 2^cb contiguous
 // positions of bits [0, cb) (only when lo > 0), for one value of the other
 // bits per block.
-//   load_mode 0: v = x[i]; 1: v = x[i]*pre[i]*fin; 2: v = x[map[i]]
-//   store_mode 0: out[i] = v; 1: out[i] = v*scale[i]*fout
+//   load_mode 0: v = x[i]; 1: v = x[i]*pre[i] (FP32: *fin); 2: v = x[map[i]];
+//             3: as 1 from the layer-swapped position of a two-layer state
+//   store_mode 0: out[i] = v; 1: out[i] = v*scale[i]*fout;
+//              2: v [* scale] to the layer-swapped position
+// (swapped positions are contiguous along the mixed bits, which then start at
+// bit half, the layer width, so those modes walk the tile along them)
 template <class T, int KB>
 __global__ void __launch_bounds__(512) kron_tile_kernel(const T* __restrict__ x, T* __restrict__ out, int lo, int nb,
                                                         int cb, Kron<T> c, int load_mode,
                                                         const double* __restrict__ pre, ScaleF fin,
                                                         const uint32_t* __restrict__ map, int store_mode,
-                                                        const double* __restrict__ scale, ScaleF fout) {
+                                                        const double* __restrict__ scale, ScaleF fout, int half) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* sm = reinterpret_cast<T*>(smem_raw);
   const int tile = 1 << (nb + cb);
@@ -151,20 +82,38 @@ __global__ void __launch_bounds__(512) kron_tile_kernel(const T* __restrict__ x,
   const uint64_t outer = blockIdx.x;
   const int low_outer = lo - cb;
   const uint64_t base = ((outer & ((1ull << low_outer) - 1)) << cb) | ((outer >> low_outer) << (lo + nb));
-  const int kmask = (1 << cb) - 1;
-  for (int e = threadIdx.x; e < tile; e += blockDim.x) {
-    const uint64_t i = base | (uint64_t)(e & kmask) | ((uint64_t)(e >> cb) << lo);
-    T v;
-    if (load_mode == 0)
-      v = x[i];
-    else if (load_mode == 1)
-      v = weigh(x[i], pre[i], fin);
-    else
-      v = x[map[i]];
-    sm[(e & kmask) * pitch + spad(e >> cb)] = v;
+  const int kmask = (1 << cb) - 1, jmask = (1 << nb) - 1;
+  const uint64_t hmask = (1ull << half) - 1;
+  if (load_mode == 3) {
+    for (int e = threadIdx.x; e < tile; e += blockDim.x) {
+      const uint64_t i = base | (uint64_t)(e >> nb) | ((uint64_t)(e & jmask) << lo);
+      const uint64_t o = (i >> half) | ((i & hmask) << half);
+      sm[(e >> nb) * pitch + spad(e & jmask)] = weigh_load(x[o], pre[o], fin);
+    }
+  } else {
+    for (int e = threadIdx.x; e < tile; e += blockDim.x) {
+      const uint64_t i = base | (uint64_t)(e & kmask) | ((uint64_t)(e >> cb) << lo);
+      T v;
+      if (load_mode == 0)
+        v = x[i];
+      else if (load_mode == 1)
+        v = weigh_load(x[i], pre[i], fin);
+      else
+        v = x[map[i]];
+      sm[(e & kmask) * pitch + spad(e >> cb)] = v;
+    }
   }
   __syncthreads();
   tile_rounds<T, KB, Kron<T>>(sm, nb, cb, pitch, c);
+  if (store_mode == 2) {
+    for (int e = threadIdx.x; e < tile; e += blockDim.x) {
+      const uint64_t i = base | (uint64_t)(e >> nb) | ((uint64_t)(e & jmask) << lo);
+      const uint64_t o = (i >> half) | ((i & hmask) << half);
+      const T v = sm[(e >> nb) * pitch + spad(e & jmask)];
+      out[o] = scale ? weigh_load(v, scale[o], fout) : v;
+    }
+    return;
+  }
   for (int e = threadIdx.x; e < tile; e += blockDim.x) {
     const uint64_t i = base | (uint64_t)(e & kmask) | ((uint64_t)(e >> cb) << lo);
     T v = sm[(e & kmask) * pitch + spad(e >> cb)];
@@ -176,10 +125,10 @@ __global__ void __launch_bounds__(512) kron_tile_kernel(const T* __restrict__ x,
 template <class T, int KB>
 void launch_tile(int64_t nblocks, int threads, size_t shm, cudaStream_t s, const T* x, T* out, int lo, int nb, int cb,
                  const Kron<T>& c, int load_mode, const double* pre, const ScaleF& fin, const uint32_t* map,
-                 int store_mode, const double* scale, const ScaleF& fout) {
+                 int store_mode, const double* scale, const ScaleF& fout, int half = 1) {
   if (shm > 48 * 1024) raise_smem_limit((const void*)kron_tile_kernel<T, KB>, shm);
   kron_tile_kernel<T, KB><<<(unsigned)nblocks, threads, shm, s>>>(x, out, lo, nb, cb, c, load_mode, pre, fin, map,
-                                                                  store_mode, scale, fout);
+                                                                  store_mode, scale, fout, half);
   TM_CKK("kron_tile");
 }
 
@@ -277,6 +226,58 @@ __global__ void __launch_bounds__(512) had_tile_kernel(const double* x, double* 
   }
   if (part) block_sum(acc, part);
 }
+
+}  // namespace
+
+// The full two-layer y-ANNNI products (YATMatVecProd2D and _T): the Kronecker
+// factor [[w0, w1], [w1, w0]], w0 = e^{-K kappa}, w1 = 1 / w0, on one layer's
+// bits and the layer swap with its weights.  y = nf Tvec .* swap(K_high x) is
+// top bits first and the swap in the last store; T^T x = nf swap(K_low (Tvec
+// .* x)) = nf K_high swap(Tvec .* x) takes the swap in its first load.  Bound
+// by the FP64 pipe (one FMA per bit and a multiply): at L = 12 two passes take
+// 0.45 ms where separate mixing and swap kernels with two operations per bit
+// took 0.94 ms.
+void kron_swap_product(const Op& op, const double* x, double* y, double* ws, bool transposed, cudaStream_t s) {
+  const int L = op.L;
+  const double kk = op.mp.betaJ * op.mp.kappa;
+  const Kron<double> c{std::exp(-2.0 * std::fabs(kk)), kk > 0 ? 1 : 0};
+  const double* tv = op.tvec.as<double>();
+  const ScaleF one = scale_factor(1.0);  // (Tvec holds the output factor)
+  const int npass = std::max(2, (L + 7) / 8);
+  int cut[8] = {0};  // pass boundaries within the layer's bits
+  for (int p = 0; p < npass; ++p) cut[p + 1] = cut[p] + (L - cut[p] + npass - p - 1) / (npass - p);
+  for (int q = 0; q < npass; ++q) {
+    const int p = transposed ? q : npass - 1 - q;
+    const bool first = (q == 0), last = (q == npass - 1);
+    const int lo = L + cut[p], nb = cut[p + 1] - cut[p];
+    const int cb = std::min(std::min(4, L), std::max(0, 2 * L - nb - 7)), tb = nb + cb;
+    const int kb = (tb >= 11) ? 4 : (tb >= 9 ? 2 : 1);
+    const int threads = std::min(512, std::max(32, (1 << tb) >> kb));
+    const size_t shm = ((size_t)(((1 << nb) + (1 << nb) / 32) | 1) << cb) * 8;
+    const double* src = first ? x : ws;
+    double* dst = last ? y : ws;
+    auto go = [&](auto k) {
+      launch_tile<double, decltype(k)::value>((int64_t)1 << (2 * L - tb), threads, shm, s, src, dst, lo, nb, cb, c,
+                                              first && transposed ? 3 : 0, tv, one, nullptr,
+                                              last && !transposed ? 2 : 0, tv, one, L);
+    };
+    if (kb == 4)
+      go(std::integral_constant<int, 4>());
+    else if (kb == 2)
+      go(std::integral_constant<int, 2>());
+    else
+      go(std::integral_constant<int, 1>());
+  }
+}
+
+// e^{|K'| L} of a Kronecker factor with coupling K' on L bits, with the factor
+// that the rounding of its r adds to a constant vector taken out
+double kron_out_factor(double coupling, int L, double r) {
+  const long double a = std::fabs((long double)coupling), n = (long double)L, rl = std::exp(-2.0L * a);
+  return (double)(std::exp(a * n) * std::pow((1.0L + rl) / (1.0L + (long double)r), n));
+}
+
+namespace {
 
 // ------------------------------------------------------------------ prefix-tree passes
 // The butterflies (x0 + r x1, x1 + r x0) on a thread's 2^KB values, top bit
@@ -636,7 +637,8 @@ double matvec_bfly(const Op& op, const T* x, T* y, bool scaled, cudaStream_t s) 
   const double* tv = op.tvec.as<double>();
   if (op.kind == K_XAT) {
     // y = nf * Tv^(1/2) * Th * Tv^(1/2) * x   (TMat/tmat.cpp:71-102)
-    run_sweep<T>(op, x, y, 1, tv, kc.gin, nullptr, 1, tv, op.normfactor * sf, s);
+    const double gin = (sizeof(T) == 8) ? 1.0 : kc.gin;
+    run_sweep<T>(op, x, y, 1, tv, gin, nullptr, 1, tv, op.normfactor * sf * (kc.gin / gin), s);
     return ret;
   }
   const uint32_t* smap = op.smap.as<uint32_t>();

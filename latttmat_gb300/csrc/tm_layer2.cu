@@ -25,126 +25,105 @@
 #include <cmath>
 #include <vector>
 
+#include "tm_bfly.cuh"
 #include "tm_bits.cuh"
 #include "tm_group.cuh"
 #include "tm_internal.h"
 
 namespace ltm {
 
+void kron_swap_product(const Op& op, const double* x, double* y, double* ws, bool transposed, cudaStream_t s);
+double kron_out_factor(double coupling, int L, double r);
+
 namespace {
 
 constexpr int kMaxTileBits = 12;  // 4096 doubles = 32 KB per tile
 
-__device__ __forceinline__ int spad(int e) { return e + (e >> 5); }
-
-struct Mat4 {
-  double c[16];
+// Y2ATMatVecProd2D's factor on one bit pair (low site p & 1, high site p >> 1):
+//   out(p) = e1[j] (e2[0] in(p) + in(p^2)) + e1[j^1] (e2[1] in(p^3) + in(p^1)),
+// j = low ^ high, e2[1] = 1 / e2[0].  With a(p) = e2[0] in(p) + in(p^2) the
+// second bracket is e2[1] a(p^1), and the factor e1[j] of the output state can
+// wait until all pairs are done (it is e^{K (L - 2 popc(low ^ high))} then):
+//   out(p) = e1[j] (a(p) + rho_j a(p^1)), rho_j = e1[j^1] e2[1] / e1[j],
+// two FMAs per element and pair where the 4 x 4 matrix takes four.
+struct PairCoef {
+  double e2;      // e2[0]
+  double rho[2];
 };
-
-struct TileMap {
-  int nt;        // tile bits
-  int pos[16];   // tile bit k -> state bit pos[k]
-  int no;        // outer bits
-  int opos[32];  // outer bit j -> state bit opos[j]
-};
-
-__device__ __forceinline__ uint64_t deposit(uint64_t v, const int* pos, int nb) {
-  uint64_t g = 0;
-  for (int k = 0; k < nb; ++k) g |= ((v >> k) & 1ull) << pos[k];
-  return g;
-}
-
-// One tile pass.  MODE 0: Kronecker [[w0, w1], [w1, w0]] on tile bits
-// [k0, nt).  MODE 1: the 4x4 matrix m4 (row-major, p = low + 2*high) on the
-// tile bit pairs (k0 + j, k0 + np + j), j < np.  pre / post_sc: optional
-// per-state input / output weights; post: output scale.
-template <int MODE>
-__global__ void __launch_bounds__(512) tile_kernel(const double* __restrict__ x, double* __restrict__ y, TileMap tm,
-                                                   int k0, int np, double w0, double w1, Mat4 m4,
-                                                   const double* __restrict__ pre,
-                                                   const double* __restrict__ post_sc, double post) {
-  extern __shared__ double sm[];
-  const int tile = 1 << tm.nt;
-  const uint64_t base = deposit((uint64_t)blockIdx.x, tm.opos, tm.no);
-  for (int e = threadIdx.x; e < tile; e += blockDim.x) {
-    const uint64_t g = base | deposit((uint64_t)e, tm.pos, tm.nt);
-    double v = x[g];
-    if (pre) v *= pre[g];
-    sm[spad(e)] = v;
-  }
-  __syncthreads();
-  if (MODE == 0) {
-    for (int k = k0; k < tm.nt; ++k) {
-      const int lowm = (1 << k) - 1;
-      for (int p = threadIdx.x; p < (tile >> 1); p += blockDim.x) {
-        const int e0 = ((p & ~lowm) << 1) | (p & lowm), e1 = e0 | (1 << k);
-        const double a = sm[spad(e0)], b = sm[spad(e1)];
-        sm[spad(e0)] = w0 * a + w1 * b;
-        sm[spad(e1)] = w1 * a + w0 * b;
-      }
-      __syncthreads();
-    }
-  } else {
-    for (int j = 0; j < np; ++j) {
-      const int ba = k0 + j, bb = k0 + np + j;  // ba < bb
-      const int ma = 1 << ba, mb = 1 << bb;
-      for (int q = threadIdx.x; q < (tile >> 2); q += blockDim.x) {
-        // insert zeros at bits ba and bb
-        int e = q;
-        e = ((e >> ba) << (ba + 1)) | (e & (ma - 1));
-        e = ((e >> bb) << (bb + 1)) | (e & (mb - 1));
-        double in[4], out[4];
-        in[0] = sm[spad(e)];
-        in[1] = sm[spad(e | ma)];
-        in[2] = sm[spad(e | mb)];
-        in[3] = sm[spad(e | ma | mb)];
+__device__ __forceinline__ void pair_step(double (&v)[4], const PairCoef& c) {
+  double a[4];
 #pragma unroll
-        for (int p = 0; p < 4; ++p)
-          out[p] = m4.c[p * 4 + 0] * in[0] + m4.c[p * 4 + 1] * in[1] + m4.c[p * 4 + 2] * in[2] +
-                   m4.c[p * 4 + 3] * in[3];
-        sm[spad(e)] = out[0];
-        sm[spad(e | ma)] = out[1];
-        sm[spad(e | mb)] = out[2];
-        sm[spad(e | ma | mb)] = out[3];
-      }
-      __syncthreads();
-    }
-  }
-  for (int e = threadIdx.x; e < tile; e += blockDim.x) {
-    const uint64_t g = base | deposit((uint64_t)e, tm.pos, tm.nt);
-    double v = sm[spad(e)] * post;
-    if (post_sc) v *= post_sc[g];
-    y[g] = v;
-  }
+  for (int p = 0; p < 4; ++p) a[p] = fma(c.e2, v[p], v[p ^ 2]);
+#pragma unroll
+  for (int p = 0; p < 4; ++p) v[p] = fma(c.rho[(p & 1) ^ (p >> 1)], a[p ^ 1], a[p]);
 }
 
-// y[h*N + l] = post * sc[h*N + l] * v[l*N + h]  (layer swap, N = 2^L)
-__global__ void swap_scale_kernel(const double* __restrict__ v, double* __restrict__ y, int L,
-                                  const double* __restrict__ sc, double post) {
-  __shared__ double tile[32][33];
-  const int64_t N = 1ll << L;
-  const int T = blockDim.x;
-  const int64_t bx = (int64_t)blockIdx.x * T, by = (int64_t)blockIdx.y * T;
-  for (int r = threadIdx.y; r < T; r += blockDim.y) tile[r][threadIdx.x] = v[(by + r) * N + bx + threadIdx.x];
+struct PairTab {
+  double d[16];  // e^{K (L - 2 q)} times the output factor, by q = popc(low ^ high)
+};
+
+// One tile pass: bit pairs (lo + j, L + lo + j), j < np, and cb contiguous low
+// bits.  Tile index: chunk bits, then the low sites, then the high sites.
+// pre / post_sc: per-state input / output weights (first / last pass).
+// Bound by the FP64 pipe.
+__global__ void __launch_bounds__(512) pair_kernel(const double* x, double* y, int L, int lo, int np, int cb,
+                                                   PairCoef c, const double* __restrict__ pre,
+                                                   const double* __restrict__ post_sc, PairTab tab) {
+  extern __shared__ double sm[];
+  const int tile = 1 << (cb + 2 * np);
+  const int cmask = (1 << cb) - 1, nmask = (1 << np) - 1;
+  // block index -> bits [cb, lo), [lo + np, L) and [L, L + lo), [L + lo + np, 2L)
+  uint64_t o = blockIdx.x;
+  uint64_t base = (o & ((1ull << (lo - cb)) - 1)) << cb;
+  o >>= lo - cb;
+  base |= (o & ((1ull << (L - lo - np)) - 1)) << (lo + np);
+  o >>= L - lo - np;
+  base |= (o & ((1ull << lo) - 1)) << L;
+  o >>= lo;
+  base |= o << (L + lo + np);
+  auto state = [&](int e) -> uint64_t {
+    return base | (uint64_t)(e & cmask) | ((uint64_t)((e >> cb) & nmask) << lo) | ((uint64_t)(e >> (cb + np)) << (L + lo));
+  };
+  for (int e = threadIdx.x; e < tile; e += blockDim.x) {
+    const uint64_t g = state(e);
+    sm[spad(e)] = pre ? x[g] * pre[g] : x[g];
+  }
   __syncthreads();
-  for (int r = threadIdx.y; r < T; r += blockDim.y) {
-    const int64_t o = (bx + r) * N + by + threadIdx.x;
-    double val = tile[threadIdx.x][r] * post;
-    if (sc) val *= sc[o];
-    y[o] = val;
+  for (int j = 0; j < np; ++j) {
+    const int ba = cb + j, bb = cb + np + j;  // ba < bb
+    const int o1 = 1 << ba, o2 = 1 << bb;
+    for (int q = threadIdx.x; q < (tile >> 2); q += blockDim.x) {
+      // insert zeros at bits ba and bb
+      int e = ((q >> ba) << (ba + 1)) | (q & (o1 - 1));
+      e = ((e >> bb) << (bb + 1)) | (e & (o2 - 1));
+      double v[4] = {sm[spad(e)], sm[spad(e | o1)], sm[spad(e | o2)], sm[spad(e | o1 | o2)]};
+      pair_step(v, c);
+      sm[spad(e)] = v[0];
+      sm[spad(e | o1)] = v[1];
+      sm[spad(e | o2)] = v[2];
+      sm[spad(e | o1 | o2)] = v[3];
+    }
+    __syncthreads();
+  }
+  const uint64_t lm = (1ull << L) - 1;
+  for (int e = threadIdx.x; e < tile; e += blockDim.x) {
+    const uint64_t g = state(e);
+    const double v = sm[spad(e)];
+    y[g] = post_sc ? v * (post_sc[g] * tab.d[__popcll((g ^ (g >> L)) & lm)]) : v;
   }
 }
 
 // --- Tvec of the full forms
 // YATMatVecProd2D::genTvec (TMat/tmat.hpp:361-366, TMat/tmat.cpp:668-684):
 // entry (row = low layer, col = high layer) of the dense NN-only x-ANNNI TM
-__global__ void yat_tvec_kernel(double* __restrict__ tv, int L, double bj, double h) {
+// (times the product's output factor f)
+__global__ void yat_tvec_kernel(double* __restrict__ tv, int L, double bj, double h, double f) {
   const int64_t n = 1ll << (2 * L);
   const uint64_t lm = (1ull << L) - 1;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const uint64_t row = (uint64_t)i & lm, col = (uint64_t)i >> L;
     const int n1 = popc64(row ^ rotr(row, L, 1)), n0 = popc64(row), nx = popc64(row ^ col);
-    tv[i] = exp(-bj * (2 * n1 - L) - bj * h * (2 * n0 - L) - bj * (2 * nx - L));
+    tv[i] = f * exp(-bj * (2 * n1 - L) - bj * h * (2 * n0 - L) - bj * (2 * nx - L));
   }
 }
 
@@ -205,14 +184,16 @@ __device__ __forceinline__ uint32_t layer_act(uint32_t x, int L, int gi) {
 }
 
 // YAMMatVecProd2D::perform_op (TMat/tmatreduce.cpp:827-876), transposed:
-// YAMMatVecProd2D_T::perform_op (:953-1016).  One CTA per left-layer block.
+// YAMMatVecProd2D_T::perform_op (:953-1016).  One CTA per left-layer block,
+// KB bits of the right layer per round in registers.
+template <int KB>
 __global__ void __launch_bounds__(512) yam_block_kernel(const double* __restrict__ x, double* __restrict__ y,
                                                         const uint32_t* __restrict__ idx,
                                                         const uint16_t* __restrict__ dup,
                                                         const double* __restrict__ tv,
                                                         const uint32_t* __restrict__ swp,
                                                         const uint32_t* __restrict__ bstart, int L, int ng,
-                                                        int transposed, double w0, double w1) {
+                                                        int transposed, Kron<double> c, double post) {
   extern __shared__ double tmp[];
   __shared__ int stab[64];
   __shared__ int nstab;
@@ -231,72 +212,15 @@ __global__ void __launch_bounds__(512) yam_block_kernel(const double* __restrict
     for (int q = 0; q < ns; ++q) tmp[spad((int)layer_act(rt, L, stab[q]))] = v;
   }
   __syncthreads();
-  const int half = 1 << (L - 1);
-  for (int b = 0; b < L; ++b) {
-    const int lowm = (1 << b) - 1;
-    for (int p = threadIdx.x; p < half; p += blockDim.x) {
-      const int e0 = ((p & ~lowm) << 1) | (p & lowm), e1 = e0 | (1 << b);
-      const double a = tmp[spad(e0)], c = tmp[spad(e1)];
-      tmp[spad(e0)] = w0 * a + w1 * c;
-      tmp[spad(e1)] = w1 * a + w0 * c;
-    }
-    __syncthreads();
-  }
+  tile_rounds<double, KB, Kron<double>>(tmp, L, 0, 0, c);
   for (uint32_t r = r0 + threadIdx.x; r < r1; r += blockDim.x) {
     const uint32_t dst = transposed ? r : swp[r];
-    y[dst] = tv[dst] * (double)dup[dst] * tmp[spad((int)(idx[r] & lm))];
+    y[dst] = tv[dst] * (double)dup[dst] * (tmp[spad((int)(idx[r] & lm))] * post);
   }
 }
 
 int grid_n(int64_t n) {
   return (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, (int64_t)num_sms() * 16));
-}
-
-// tile map: tile bits = `tb` (in order), outer bits = all others below nbits
-TileMap make_map(const std::vector<int>& tb, int nbits) {
-  TileMap m{};
-  m.nt = (int)tb.size();
-  uint64_t used = 0;
-  for (int k = 0; k < m.nt; ++k) {
-    m.pos[k] = tb[k];
-    used |= 1ull << tb[k];
-  }
-  m.no = 0;
-  for (int b = 0; b < nbits; ++b)
-    if (!((used >> b) & 1ull)) m.opos[m.no++] = b;
-  return m;
-}
-
-template <int MODE>
-void launch_tile(const double* x, double* y, const TileMap& m, int k0, int np, double w0, double w1, const Mat4& m4,
-                 const double* pre, const double* post_sc, double post, cudaStream_t s) {
-  const int tile = 1 << m.nt;
-  const size_t shm = (size_t)(tile + tile / 32 + 1) * sizeof(double);
-  const int threads = std::min(512, std::max(32, tile / 4));
-  tile_kernel<MODE><<<(unsigned)(1u << m.no), threads, shm, s>>>(x, y, m, k0, np, w0, w1, m4, pre, post_sc, post);
-  TM_CKK("two_layer_tile");
-}
-
-// Kronecker [[w0, w1], [w1, w0]] over state bits [lo, hi) of a 2L-bit vector
-void kron_range(const double* x, double* y, int nbits, int lo, int hi, double w0, double w1, const double* pre,
-                const double* post_sc, double post, cudaStream_t s) {
-  const Mat4 none{};
-  int b = lo;
-  bool first = true;
-  const double* src = x;
-  while (b < hi) {
-    const int cb = (b == 0) ? 0 : std::min(5, b);  // contiguous low bits for coalescing
-    const int nb = std::min(hi - b, kMaxTileBits - cb);
-    std::vector<int> tb;
-    for (int k = 0; k < cb; ++k) tb.push_back(k);
-    for (int k = 0; k < nb; ++k) tb.push_back(b + k);
-    const bool last = (b + nb >= hi);
-    launch_tile<0>(src, y, make_map(tb, nbits), cb, 0, w0, w1, none, first ? pre : nullptr,
-                   last ? post_sc : nullptr, last ? post : 1.0, s);
-    src = y;
-    first = false;
-    b += nb;
-  }
 }
 
 }  // namespace
@@ -307,12 +231,15 @@ void build_two_layer(Op& op) {
   const double bj = op.mp.betaJ, k = op.mp.kappa, k2 = op.mp.kappa2, h = op.mp.h;
   op.nstate = 1ll << (2 * L);
   cudaStream_t s = op.stream;
+  // output factor of the r-form butterflies (K_YAT, K_YAM)
+  op.kron.out64 = kron_out_factor(bj * k, L, std::exp(-2.0 * std::fabs(bj * k))) *
+                  (op.kind == K_YAT ? op.normfactor : 1.0);
   if (op.kind == K_YAT || op.kind == K_Y2AT) {
     op.n = op.nstate;
     op.tvec.alloc((size_t)op.n * 8);
     op.ws_a.alloc((size_t)op.n * 8);
     if (op.kind == K_YAT)
-      yat_tvec_kernel<<<grid_n(op.n), 256, 0, s>>>(op.tvec.as<double>(), L, bj, h);
+      yat_tvec_kernel<<<grid_n(op.n), 256, 0, s>>>(op.tvec.as<double>(), L, bj, h, op.kron.out64);
     else
       y2at_tvec_kernel<<<grid_n(op.n), 256, 0, s>>>(op.tvec.as<double>(), L, bj, h);
     TM_CKK("two_layer_tvec");
@@ -357,56 +284,49 @@ void matvec_two_layer(const Op& op, const double* x, double* y, cudaStream_t s) 
   const int L = b.L;
   const double bj = b.mp.betaJ, k = b.mp.kappa;
   if (b.kind == K_YAT) {
-    // bzwj2 = e^{-+K kappa} (TMat/tmat.cpp:110-113)
-    const double w0 = std::exp(-bj * k), w1 = 1.0 / w0;
-    double* v = b.ws_a.as<double>();
-    const int T = std::min(32, 1 << L);
-    const dim3 grid((1u << L) / T, (1u << L) / T), blk(T, std::min(T, 8));
-    if (!tr) {
-      kron_range(x, v, 2 * L, L, 2 * L, w0, w1, nullptr, nullptr, 1.0, s);
-      swap_scale_kernel<<<grid, blk, 0, s>>>(v, y, L, b.tvec.as<double>(), b.normfactor);
-    } else {
-      kron_range(x, v, 2 * L, 0, L, w0, w1, b.tvec.as<double>(), nullptr, 1.0, s);
-      swap_scale_kernel<<<grid, blk, 0, s>>>(v, y, L, nullptr, b.normfactor);
-    }
-    TM_CKK("two_layer_swap_scale");
+    kron_swap_product(b, x, y, b.ws_a.as<double>(), tr, s);
   } else if (b.kind == K_Y2AT) {
-    // bzwj1 = e^{+-K}, bzwj2 = e^{-+2K kappa} (TMat/tmat.cpp:247-253); the 4x4
-    // matrix on a bit pair with p = low + 2*high, j = low ^ high:
-    //   out(p) = w1[j] (w2[0] in(p) + in(p^2)) + w1[j^1] (w2[1] in(p^3) + in(p^1))
-    const double e1[2] = {std::exp(bj), std::exp(-bj)};
-    const double e2[2] = {std::exp(-2.0 * bj * k), std::exp(2.0 * bj * k)};
-    Mat4 m4{};
-    for (int p = 0; p < 4; ++p) {
-      const int j = (p & 1) ^ (p >> 1);
-      m4.c[p * 4 + p] += e1[j] * e2[0];
-      m4.c[p * 4 + (p ^ 2)] += e1[j];
-      m4.c[p * 4 + (p ^ 3)] += e1[j ^ 1] * e2[1];
-      m4.c[p * 4 + (p ^ 1)] += e1[j ^ 1];
-    }
+    // bzwj1 = e^{+-K}, bzwj2 = e^{-+2K kappa} (TMat/tmat.cpp:247-253)
+    const double r1 = std::exp(-2.0 * bj), e21 = std::exp(2.0 * bj * k);  // e1[1] / e1[0], e2[1]
+    PairCoef c;
+    c.e2 = std::exp(-2.0 * bj * k);
+    c.rho[0] = r1 * e21;
+    c.rho[1] = e21 / r1;
+    PairTab tab{};
+    for (int q = 0; q <= L; ++q) tab.d[q] = b.normfactor * std::exp(bj * (L - 2.0 * q));
+    const double* tv = b.tvec.as<double>();
     int lo = 0;
     const double* src = x;
     while (lo < L) {
       const int cb = (lo == 0) ? 0 : std::min(3, lo);
       const int np = std::min(L - lo, (kMaxTileBits - cb) / 2);
-      std::vector<int> tb;
-      for (int q = 0; q < cb; ++q) tb.push_back(q);
-      for (int q = 0; q < np; ++q) tb.push_back(lo + q);
-      for (int q = 0; q < np; ++q) tb.push_back(L + lo + q);
-      const bool first = (lo == 0), last = (lo + np >= L);
-      launch_tile<1>(src, y, make_map(tb, 2 * L), cb, np, 0.0, 0.0, m4, first ? b.tvec.as<double>() : nullptr,
-                     last ? b.tvec.as<double>() : nullptr, last ? b.normfactor : 1.0, s);
+      const int tile = 1 << (cb + 2 * np);
+      const size_t shm = (size_t)(tile + tile / 32 + 1) * sizeof(double);
+      const bool last = (lo + np >= L);
+      pair_kernel<<<(unsigned)(1u << (2 * L - cb - 2 * np)), std::min(512, std::max(32, tile / 4)), shm, s>>>(
+          src, y, L, lo, np, cb, c, lo == 0 ? tv : nullptr, last ? tv : nullptr, tab);
+      TM_CKK("two_layer_pairs");
       src = y;
       lo += np;
     }
   } else if (b.kind == K_YAM) {
-    const double w0 = std::exp(-bj * k), w1 = 1.0 / w0;
     const size_t shm = (size_t)((1 << L) + (1 << L) / 32 + 1) * sizeof(double);
-    raise_smem_limit((const void*)yam_block_kernel, shm);
     const int ng = 2 * L * (b.censym ? 2 : 1);
-    yam_block_kernel<<<(unsigned)b.nblocks, 512, shm, s>>>(x, y, b.idx.as<uint32_t>(), b.dup.as<uint16_t>(),
-                                                           b.tvec.as<double>(), b.swp.as<uint32_t>(),
-                                                           b.bstart.as<uint32_t>(), L, ng, tr ? 1 : 0, w0, w1);
+    const Kron<double> c{std::exp(-2.0 * std::fabs(bj * k)), bj * k > 0 ? 1 : 0};
+    auto go = [&](auto kb) {
+      constexpr int KB = decltype(kb)::value;
+      raise_smem_limit((const void*)yam_block_kernel<KB>, shm);
+      const int threads = std::min(512, std::max(128, (1 << L) >> KB));
+      yam_block_kernel<KB><<<(unsigned)b.nblocks, threads, shm, s>>>(
+          x, y, b.idx.as<uint32_t>(), b.dup.as<uint16_t>(), b.tvec.as<double>(), b.swp.as<uint32_t>(),
+          b.bstart.as<uint32_t>(), L, ng, tr ? 1 : 0, c, b.kron.out64);
+    };
+    if (L >= 12)
+      go(std::integral_constant<int, 4>());
+    else if (L >= 9)
+      go(std::integral_constant<int, 2>());
+    else
+      go(std::integral_constant<int, 1>());
     TM_CKK("two_layer_block");
   } else {
     fail(TM_ERR_ARG, "not a two-layer operator");
