@@ -162,7 +162,8 @@ struct Arnoldi {
   cudaStream_t s;
   int64_t n;
   int m;
-  DBuf V, W, x32, y32, h1, h2, part, nsq, Hd, Wd;
+  DBuf V, W, x32, y32, h1, h2, part, nsq, Hd, Wd, cgs;
+  CgsScratch cg{};
   int matvecs = 0, matvecs64 = 0, restarts = 0;
   std::vector<double> Hh;  // host copy (m+1)^2
 
@@ -175,6 +176,10 @@ struct Arnoldi {
     nsq.alloc(8);
     Hd.alloc((size_t)(m + 1) * (m + 1) * 8);
     Wd.alloc((size_t)64 * 64 * 8);
+    if (n <= kCgsRows) {
+      cgs.alloc(cgs_scratch_bytes());
+      cg = cgs_scratch(cgs, s);
+    }
   }
   double* v(int j) const { return V.as<double>() + (int64_t)j * n; }
 
@@ -199,6 +204,11 @@ struct Arnoldi {
       else
         apply_internal(op, v(j), w, nullptr, nullptr, false, s);
       ++matvecs64;
+      if (cg.h1) {
+        ++matvecs;
+        cgs_step(v(0), n, j, w, n, Hd.as<double>(), m + 1, false, cg, v(j + 1), s);
+        return;
+      }
       mdot(v(0), n, j + 1, w, n, h1.as<double>(), part.as<double>(), s);
       maxpy(v(0), n, j + 1, h1.as<double>(), w, n, s);
     }

@@ -39,6 +39,22 @@ void fill_uniform(double* v, int64_t n, uint64_t seed, cudaStream_t s);
 // count of non-finite entries (device counter)
 void count_nonfinite(const double* v, int64_t n, unsigned int* cnt_dev, cudaStream_t s);
 
+// One CGS2 step of a short vector (tm_cgs.cu): w orthogonalised twice against
+// V[:, 0..j], column j of H (leading dimension ldh; sym: its mirror too),
+// vnext = w / |w|.  For n <= kCgsRows: solves of full x-ANNNI operators take, one
+// kernel after the other / by this step, 2.98 / 2.02 ms at 2^14 rows, 4.10 / 3.01
+// at 2^16, 4.55 / 4.01 at 2^17, 6.10 / 5.72 at 2^18, where the products and the
+// full grids of the separate kernels have all but closed the gap.
+constexpr int64_t kCgsRows = 262144;
+struct CgsScratch {
+  double *h1, *h2, *nsq, *part;
+  unsigned* ctr;
+};
+size_t cgs_scratch_bytes();
+CgsScratch cgs_scratch(const DBuf& b, cudaStream_t s);
+void cgs_step(const double* V, int64_t ldv, int j, double* w, int64_t n, double* H, int ldh, bool sym,
+              const CgsScratch& c, double* vnext, cudaStream_t s);
+
 // Leading dimension of a Krylov basis of length-n columns: columns start on
 // 256-byte boundaries, so the 16-byte vector forms of the kernels apply.
 inline int64_t col_ld(int64_t n) { return (n + 63) & ~(int64_t)63; }

@@ -172,7 +172,8 @@ struct Lanczos {
   cudaStream_t s;
   int64_t n, ld;  // vector length, basis leading dimension
   int m;
-  DBuf V, W, x32, y32, h1, h2, part, nsq, Hd, wd, Zd, Ysel;
+  DBuf V, W, x32, y32, h1, h2, part, nsq, Hd, wd, Zd, Ysel, cgs;
+  CgsScratch cg{};
   int matvecs = 0, matvecs64 = 0, restarts = 0;
 
   int vcols = 0;  // columns of V allocated (m + 1 once full)
@@ -191,6 +192,10 @@ struct Lanczos {
     wd.alloc(64 * 8);
     Zd.alloc(64 * 64 * 8);
     Ysel.alloc(64 * 64 * 8);
+    if (n <= kCgsRows) {
+      cgs.alloc(cgs_scratch_bytes());
+      cg = cgs_scratch(cgs, s);
+    }
   }
   double* v(int j) const { return V.as<double>() + (int64_t)j * ld; }
 
@@ -224,6 +229,11 @@ struct Lanczos {
     } else {
       apply_internal(op, v(j), w, nullptr, nullptr, false, s);
       ++matvecs64;
+      if (cg.h1) {
+        ++matvecs;
+        cgs_step(v(0), ld, j, w, n, Hd.as<double>(), m + 1, true, cg, v(j + 1), s);
+        return;
+      }
       mdot(v(0), ld, j + 1, w, n, h1.as<double>(), part.as<double>(), s);
       maxpy(v(0), ld, j + 1, h1.as<double>(), w, n, s);
     }
