@@ -325,7 +325,6 @@ static void build_op(Op& op) {
       op.ws_c.alloc((size_t)op.n * 8);
       op.eo.w1_32.alloc(((size_t)op.eo.n_orep << op.eo.m) * 4);
       op.eo.w1_64.alloc(((size_t)op.eo.n_orep << op.eo.m) * 8);
-      if (const size_t xb = eo_xchg_bytes(op.eo)) op.eo.xchg.alloc(xb);
       op.yp.alloc((size_t)op.n * 8);
     } else {
       if (op.L > 30) fail(TM_ERR_LIMIT, "generic reduced path supports L <= 30");

@@ -39,7 +39,7 @@
 // A tile of 2^m elements is split over a cluster of 2^c CTAs (FP32 m=16: two
 // CTAs x 2^15 elements in 135 KB of shared memory), CTA `rank` holding the
 // patterns whose top c bits are `rank`.  The butterflies on those top bits
-// combine the CTAs' tiles through DSMEM once all local rounds are done.
+// run between the CTAs' tiles through DSMEM once all local rounds are done.
 // Inside a CTA each thread owns 2^KB elements per round: KB butterfly levels
 // in registers, with a padded shared-memory transpose between rounds.
 #include <atomic>
@@ -350,145 +350,87 @@ __device__ __forceinline__ void st_stream(V* p, V v) {
     __stcs(p, v);
 }
 
-// acc += c * v over the 16 / sizeof(T) elements of a 16-byte chunk
-template <class T>
-__device__ __forceinline__ void axpy16(float4& acc, const float4& v, T c);
-template <>
-__device__ __forceinline__ void axpy16<float>(float4& acc, const float4& v, float c) {
-  acc.x = fmaf(c, v.x, acc.x);
-  acc.y = fmaf(c, v.y, acc.y);
-  acc.z = fmaf(c, v.z, acc.z);
-  acc.w = fmaf(c, v.w, acc.w);
+// One butterfly between the 16 / sizeof(T) elements of two 16-byte chunks.
+__device__ __forceinline__ void bfly16(float4& x, float4& y, float r, int swap) {
+  const float2 r2 = make_float2(r, r);
+  const float2 x0 = make_float2(x.x, x.y), x1 = make_float2(x.z, x.w);
+  const float2 y0 = make_float2(y.x, y.y), y1 = make_float2(y.z, y.w);
+  const float2 a0 = __ffma2_rn(r2, y0, x0), a1 = __ffma2_rn(r2, y1, x1);
+  const float2 b0 = __ffma2_rn(r2, x0, y0), b1 = __ffma2_rn(r2, x1, y1);
+  const float4 a = make_float4(a0.x, a0.y, a1.x, a1.y), b = make_float4(b0.x, b0.y, b1.x, b1.y);
+  x = swap ? b : a;
+  y = swap ? a : b;
 }
-template <>
-__device__ __forceinline__ void axpy16<double>(float4& acc, const float4& v, double c) {
-  double2 a = *reinterpret_cast<double2*>(&acc);
-  const double2 x = *reinterpret_cast<const double2*>(&v);
-  a.x = fma(c, x.x, a.x);
-  a.y = fma(c, x.y, a.y);
-  acc = *reinterpret_cast<float4*>(&a);
+__device__ __forceinline__ void bfly16(double2& x, double2& y, double r, int swap) {
+  const double2 a = make_double2(fma(r, y.x, x.x), fma(r, y.y, x.y));
+  const double2 b = make_double2(fma(r, x.x, y.x), fma(r, x.y, y.y));
+  x = swap ? b : a;
+  y = swap ? a : b;
 }
-template <>
-__device__ __forceinline__ void axpy16<dfloat>(float4& acc, const float4& v, dfloat c) {
-  const dfloat a0 = df_fma(c, dfloat(v.x, v.y), dfloat(acc.x, acc.y));
-  const dfloat a1 = df_fma(c, dfloat(v.z, v.w), dfloat(acc.z, acc.w));
-  acc = make_float4(a0.hi, a0.lo, a1.hi, a1.lo);
-}
-
-// 16-byte chunks of one CTA's exchange slot: the padded tile rounded up to
-// whole 128-byte lines
-__host__ __device__ __forceinline__ int64_t xchg_slot_chunks(int n, int elem) {
-  const int64_t chunks = ((int64_t)((1 << n) + (1 << n) / 32) * elem) / 16;
-  return (chunks + 7) & ~(int64_t)7;
+__device__ __forceinline__ void bfly16(float4& x, float4& y, dfloat r, int swap) {
+  const dfloat x0(x.x, x.y), x1(x.z, x.w), y0(y.x, y.y), y1(y.z, y.w);
+  const dfloat a0 = df_fma(r, y0, x0), a1 = df_fma(r, y1, x1), b0 = df_fma(r, x0, y0), b1 = df_fma(r, x1, y1);
+  const float4 a = make_float4(a0.hi, a0.lo, a1.hi, a1.lo), b = make_float4(b0.hi, b0.lo, b1.hi, b1.lo);
+  x = swap ? b : a;
+  y = swap ? a : b;
 }
 
-// Combine the cluster's 2^c partial tiles (butterflies on the top c tile
-// bits) in place: afterwards sm[spad(j)] holds the final value of local
-// element j.  The combination is elementwise at equal positions of the
-// padded tiles, so it runs over raw 16-byte chunks of the buffer (the padding
-// slots carry values nobody reads).
-//
-// With an exchange buffer (xchg), each CTA first stores its tile to its own
-// slot (CTA index order, 128-byte aligned); after a cluster barrier, whose
-// release/acquire orders those stores before the partners' loads, every
-// thread reads its chunks of the partners' tiles from L2 and of its own tile
-// from shared memory.  A second barrier marks the partners' reads done; each
-// CTA then discards its slot's lines from L2, so the buffer is never written
-// back to DRAM.  Without one, the partners' tiles are read through DSMEM, and
-// the write-back waits for a cluster barrier so no CTA overwrites values
-// another still reads.  The arithmetic is the same either way.
-template <class T, int KB>
-__device__ __forceinline__ void cluster_reduce(cg::cluster_group& cl, T* sm, int rank, const EOArgs& A,
-                                               float4* __restrict__ xchg) {
-  const T a = A.swap ? coef_r<T>(A) : T(1), b = A.swap ? T(1) : coef_r<T>(A);
-  if constexpr (std::is_same<T, double>::value) {
-    // native FP64: element-wise (the chunk accumulators and FP64 temporaries
-    // together would spill)
-    const int p = A.p, kb = A.n - A.p;
-    T acc[1 << KB];
-#pragma unroll
-    for (int k = 0; k < (1 << KB); ++k) acc[k] = T(0);
-    cl.sync();
-    for (int r = 0; r < (1 << A.c); ++r) {
-      T coef = T(1);
-      for (int bit = 0; bit < A.c; ++bit) coef = coef * ((((r ^ rank) >> bit) & 1) ? b : a);
-      const T* src = (r == rank) ? sm : cl.map_shared_rank(sm, r);
-#pragma unroll
-      for (int k = 0; k < (1 << KB); ++k)
-        if (k < (1 << kb)) acc[k] = acc[k] + coef * src[spad(threadIdx.x + (k << p))];
-    }
-    cl.sync();
-#pragma unroll
-    for (int k = 0; k < (1 << KB); ++k)
-      if (k < (1 << kb)) sm[spad(threadIdx.x + (k << p))] = acc[k];
-    __syncthreads();
-    return;
-  }
-  constexpr int kMaxChunks = ((1 << KB) * 33 * (int)sizeof(T) + 511) / 512;  // ceil(2^KB * 33/32 * sizeof(T) / 16)
+// Butterflies on the top C tile bits, between the cluster's 2^C CTAs.  Each
+// CTA takes 2^-C of the positions: it reads those of every CTA's tile (its
+// partners' through DSMEM), does the C levels in registers and writes the
+// results back to where they came from, so a tile part crosses the cluster
+// once each way, and a level costs one FMA per element.  The positions are
+// raw 16-byte chunks of the padded tiles (equal positions everywhere; the
+// padding slots carry values nobody reads).
+//   With every CTA reading its partners' whole tiles instead (2^C - 1 parts
+// in, 2^C FMAs per element; through L2 for four CTAs) the two passes at
+// L = 32 took 4.24 + 3.38 ms in double-float (four CTAs of 2^14 elements) and
+// 7.18 + 7.18 in FP64; this way 3.73 + 2.84 and 5.92 + 5.89.
+template <class T, int C>
+__device__ __forceinline__ void cluster_bits(cg::cluster_group& cl, T* sm, int rank, const EOArgs& A) {
+  using Chunk = typename std::conditional<std::is_same<T, double>::value, double2, float4>::type;
+  constexpr int NC = 1 << C;
+  constexpr int U = 4 / NC;  // positions in flight per thread
   const int nchunks = (((1 << A.n) + (1 << (A.n - 5))) * (int)sizeof(T)) / 16;
-  const int nc = 1 << A.c;
-  float4* dst = reinterpret_cast<float4*>(sm);
-  float4 acc[kMaxChunks];
-  if (xchg) {
-    const int64_t slot = xchg_slot_chunks(A.n, (int)sizeof(T));
-    const int64_t first = (int64_t)blockIdx.x - rank;  // the cluster's CTAs are consecutive
-    float4* mine = xchg + (int64_t)blockIdx.x * slot;
+  const int share = (nchunks + NC - 1) / NC;
+  const int q1 = min(nchunks, (rank + 1) * share);
+  const T r = coef_r<T>(A);
+  Chunk* tile[NC];
 #pragma unroll
-    for (int k = 0; k < kMaxChunks; ++k) {
-      const int q = (int)threadIdx.x + k * (int)blockDim.x;
-      if (q < nchunks) __stcg(mine + q, dst[q]);
-      acc[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int k = 0; k < NC; ++k) tile[k] = reinterpret_cast<Chunk*>(cl.map_shared_rank(sm, k));
+  cl.sync();
+  for (int q0 = rank * share + (int)threadIdx.x; q0 < q1; q0 += U * (int)blockDim.x) {
+    Chunk v[U][NC];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int q = q0 + u * (int)blockDim.x;
+#pragma unroll
+      for (int k = 0; k < NC; ++k)
+        if (q < q1) v[u][k] = tile[k][q];
     }
-    cl.sync();
-    for (int r = 0; r < nc; ++r) {
-      T coef = T(1);
-      for (int bit = 0; bit < A.c; ++bit) coef = coef * ((((r ^ rank) >> bit) & 1) ? b : a);
-      if (r == rank) {
 #pragma unroll
-        for (int k = 0; k < kMaxChunks; ++k) {
-          const int q = (int)threadIdx.x + k * (int)blockDim.x;
-          if (q < nchunks) axpy16<T>(acc[k], dst[q], coef);
-        }
-      } else {
-        const float4* src = xchg + (first + r) * slot;
+    for (int u = 0; u < U; ++u) {
+      const int q = q0 + u * (int)blockDim.x;
+      if (q < q1) {
 #pragma unroll
-        for (int k = 0; k < kMaxChunks; ++k) {
-          const int q = (int)threadIdx.x + k * (int)blockDim.x;
-          if (q < nchunks) axpy16<T>(acc[k], __ldcg(src + q), coef);
-        }
+        for (int b = 1; b < NC; b <<= 1)
+#pragma unroll
+          for (int k = 0; k < NC; ++k)
+            if (!(k & b)) bfly16(v[u][k], v[u][k | b], r, A.swap);
+#pragma unroll
+        for (int k = 0; k < NC; ++k) tile[k][q] = v[u][k];
       }
     }
-#pragma unroll
-    for (int k = 0; k < kMaxChunks; ++k) {
-      const int q = (int)threadIdx.x + k * (int)blockDim.x;
-      if (q < nchunks) dst[q] = acc[k];
-    }
-    cl.sync();  // the partners' reads of this slot are done (and the tile is complete)
-    for (int64_t line = threadIdx.x; line < slot / 8; line += blockDim.x)
-      asm volatile("discard.global.L2 [%0], 128;\n" ::"l"(mine + line * 8) : "memory");
-    return;
-  }
-#pragma unroll
-  for (int k = 0; k < kMaxChunks; ++k) acc[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-  cl.sync();
-  for (int r = 0; r < nc; ++r) {
-    T coef = T(1);
-    for (int bit = 0; bit < A.c; ++bit) coef = coef * ((((r ^ rank) >> bit) & 1) ? b : a);
-    const float4* src = reinterpret_cast<const float4*>((r == rank) ? sm : cl.map_shared_rank(sm, r));
-#pragma unroll
-    for (int k = 0; k < kMaxChunks; ++k) {
-      const int q = (int)threadIdx.x + k * (int)blockDim.x;
-      if (q < nchunks) axpy16<T>(acc[k], src[q], coef);
-    }
   }
   cl.sync();
-#pragma unroll
-  for (int k = 0; k < kMaxChunks; ++k) {
-    const int q = (int)threadIdx.x + k * (int)blockDim.x;
-    if (q < nchunks) dst[q] = acc[k];
-  }
-  // only this CTA reads its combined tile from here on
-  __syncthreads();
+}
+
+template <class T>
+__device__ __forceinline__ void cluster_combine(cg::cluster_group& cl, T* sm, int rank, const EOArgs& A) {
+  if (A.c == 1)
+    cluster_bits<T, 1>(cl, sm, rank, A);
+  else
+    cluster_bits<T, 2>(cl, sm, rank, A);
 }
 
 // elements per batch of the output loops (independent loads in flight per thread)
@@ -505,8 +447,7 @@ template <class T, int KB, class InT, bool CL>
 __global__ void __launch_bounds__(1024, 1) eo_pass1(EOArgs A, const InT* __restrict__ u,
                                                     const uint32_t* __restrict__ map1,
                                                     const uint16_t* __restrict__ it_e,
-                                                    const uint2* __restrict__ wout, T* __restrict__ w1,
-                                                    float4* __restrict__ xchg) {
+                                                    const uint2* __restrict__ wout, T* __restrict__ w1) {
   static_assert(sizeof(T) == sizeof(InT), "u and the tile share the element size");
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* sm = reinterpret_cast<T*>(smem_raw);
@@ -554,7 +495,7 @@ __global__ void __launch_bounds__(1024, 1) eo_pass1(EOArgs A, const InT* __restr
   }
   __syncthreads();
   smem_rounds<T, KB>(sm, A, n);
-  if constexpr (CL) cluster_reduce<T, KB>(cl, sm, rank, A, xchg);
+  if constexpr (CL) cluster_combine<T>(cl, sm, rank, A);
   // Output.  w1 is class-major: the block of e-class C holds, for each tile,
   // the |C| values of C's members, so a warp writes a few contiguous runs.
   // (the table entries of a whole batch are loaded before any is used, so
@@ -595,7 +536,7 @@ __global__ void __launch_bounds__(1024, 1) eo_pass2(EOArgs A, const T* __restric
                                                     const double* __restrict__ sout64,
                                                     const float* __restrict__ sout32,
                                                     const dfloat* __restrict__ soutdf, ScaleF post,
-                                                    OutT* __restrict__ y, float4* __restrict__ xchg) {
+                                                    OutT* __restrict__ y) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* sm = reinterpret_cast<T*>(smem_raw);
   __shared__ uint32_t he[128];
@@ -636,7 +577,7 @@ __global__ void __launch_bounds__(1024, 1) eo_pass2(EOArgs A, const T* __restric
   }
   __syncthreads();
   smem_rounds<T, KB>(sm, A, n);
-  if constexpr (CL) cluster_reduce<T, KB>(cl, sm, rank, A, xchg);
+  if constexpr (CL) cluster_combine<T>(cl, sm, rank, A);
   // Designated outputs of this tile.  They are ordered like it_o, so the
   // outputs whose o this CTA holds form one contiguous range: groups
   // [rank, rank + 1) * 2^(ct - c) of the tile's 2^ct output groups.
@@ -853,16 +794,6 @@ static int cluster_bits_for(int m, size_t elem) {
   const int cap = g_eo_tile_bits_cap.load();
   if (cap > 0 && m - c > cap) c = m - cap;
   return c;
-}
-
-// Bytes of exchange slots the clustered launches of a plan need (0: none;
-// only clusters of 4 or more CTAs use them).
-size_t eo_xchg_bytes(const EOPlan& P) {
-  size_t b = 0;
-  const size_t nt = (size_t)std::max(P.n_orep, P.n_erep);
-  if (P.c32 >= 2) b = std::max(b, (nt << P.c32) * (size_t)xchg_slot_chunks(P.m - P.c32, 4) * 16);
-  if (P.c64 >= 2) b = std::max(b, (nt << P.c64) * (size_t)xchg_slot_chunks(P.m - P.c64, 8) * 16);
-  return b;
 }
 
 // Orders of the m-bit patterns used by the passes.  cls: H-class index of
@@ -1260,20 +1191,6 @@ struct EoIO<dfloat> {
   using Out = double;
 };
 
-// The exchange buffer for a clustered launch of `ntiles` tiles (one slot per
-// CTA), or null: the cluster combine then reads the partners' tiles through
-// DSMEM.  Clusters of 4 or more CTAs exchange through L2 (at L = 32 the
-// double-float passes take 4.55 + 3.99 ms that way against 5.05 + 4.62 ms
-// over DSMEM); a 2-CTA cluster reads its one partner through DSMEM, which
-// measured 2-3% faster than the round trip through L2.  Native FP64
-// combines element by element through DSMEM.
-template <class T>
-float4* eo_xchg(const EOArgs& A, const EOPlan& P, int ntiles) {
-  if (A.c < 2 || std::is_same<T, double>::value || !P.xchg.p) return nullptr;
-  const size_t need = ((size_t)ntiles << A.c) * (size_t)xchg_slot_chunks(A.n, (int)sizeof(T)) * 16;
-  return need <= P.xchg.bytes ? P.xchg.as<float4>() : nullptr;
-}
-
 template <class T, int KB>
 void launch_pass1(const EOArgs& A, int ntiles, const typename EoIO<T>::In* u, const EOPlan& P, T* w1,
                   cudaStream_t s) {
@@ -1292,8 +1209,7 @@ void launch_pass1(const EOArgs& A, int ntiles, const typename EoIO<T>::In* u, co
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  TM_CK(cudaLaunchKernelEx(&cfg, kfn, A, u, P.map1.as<uint32_t>(), P.it_e.as<uint16_t>(), P.wout.as<uint2>(), w1,
-                           eo_xchg<T>(A, P, ntiles)));
+  TM_CK(cudaLaunchKernelEx(&cfg, kfn, A, u, P.map1.as<uint32_t>(), P.it_e.as<uint16_t>(), P.wout.as<uint2>(), w1));
 }
 
 template <class T, int KB, int OSC, class OutT = typename EoIO<T>::Out>
@@ -1316,8 +1232,7 @@ void launch_pass2(const EOArgs& A, int ntiles, const T* w1, const EOPlan& P, con
   cfg.numAttrs = 1;
   TM_CK(cudaLaunchKernelEx(&cfg, kfn, A, w1, P.t2o.as<uint2>(), P.cf_e.as<uint16_t>(),
                            P.erep.as<uint32_t>(), P.cls_start.as<uint32_t>(), P.cls_size.as<uint32_t>(),
-                           P.out_off.as<uint32_t>(), P.out_o.as<uint16_t>(), sout64, sout32, soutdf, post, y,
-                           eo_xchg<T>(A, P, ntiles)));
+                           P.out_off.as<uint32_t>(), P.out_o.as<uint16_t>(), sout64, sout32, soutdf, post, y));
 }
 
 template <class T>
@@ -1464,7 +1379,7 @@ void eo_dispatch_dd(const Op& op, const EOArgs& A, const dfloat* x, dfloat* y, c
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   TM_CK(cudaLaunchKernelEx(&cfg, k1, A, (const dfloat*)u, P.map1.as<uint32_t>(), P.it_e.as<uint16_t>(),
-                           P.wout.as<uint2>(), w1, eo_xchg<dfloat>(A, P, P.n_orep)));
+                           P.wout.as<uint2>(), w1));
   TM_CKK("eo_pass1_dd");
   launch_pass2<dfloat, KB, kOutDF, dfloat>(A, P.n_erep, w1, P, op.sout64.as<double>(), op.sout32.as<float>(),
                                            op.soutdf.as<dfloat>(), scale_factor(1.0), y, s);
