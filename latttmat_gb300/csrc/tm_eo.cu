@@ -36,8 +36,8 @@
 // The input is scaled by (1 + r)^-L so magnitudes match the normalised
 // operator, and the output factor stays (e^K + e^-K)^L.
 //
-// A tile of 2^m elements is split over a cluster of 2^c CTAs (FP32 m=16: two
-// CTAs x 2^15 elements in 135 KB of shared memory), CTA `rank` holding the
+// A tile of 2^m elements is split over a cluster of 2^c CTAs (FP32 m=16: four
+// CTAs x 2^14 elements in 68 KB of shared memory each), CTA `rank` holding the
 // patterns whose top c bits are `rank`.  The butterflies on those top bits
 // run between the CTAs' tiles through DSMEM once all local rounds are done.
 // Inside a CTA each thread owns 2^KB elements per round: KB butterfly levels
@@ -249,8 +249,8 @@ __device__ __forceinline__ void cp_async_elem<8>(void* dst, const void* src) {
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
-// Tile bits covered by the unrolled butterfly rounds (the largest tile is
-// 2^15 elements in FP32 and 2^14 in 8-byte types).
+// Tile bits covered by the unrolled butterfly rounds (the largest tile part is
+// 2^14 elements).
 constexpr int kMaxTileBits = 16;
 
 // One butterfly round on local bits [G0, G0 + GS) of the shared-memory tile.
@@ -516,7 +516,8 @@ __global__ void __launch_bounds__(1024, 1) eo_pass1(EOArgs A, const InT* __restr
 // (FP64), val * soutdf in double-float (double-float storage), or an FP32
 // val * soutdf * post formed in double-float and rounded once (kOutF32S).
 // Two FP64 multiplies and three conversions per output in place of the last
-// took 0.44 ms of pass 2's 1.22 ms at L = 32; it takes 0.79 ms in all.
+// took 0.44 ms of pass 2's 1.22 ms at L = 32 (0.79 ms in all without them,
+// parts of 2^15 elements).
 enum { kOutF32 = 0, kOutF64 = 1, kOutDF = 2, kOutF32S = 3 };
 
 // pass 2: z[(e_rep, o)] = (Th_O w)[(e_rep, o)]; emit designated outputs.
@@ -787,10 +788,22 @@ int grid_for(int64_t n) {
 static std::atomic<int> g_eo_tile_bits_cap{0};
 void eo_set_tile_bits_cap(int bits) { g_eo_tile_bits_cap.store(bits < 0 ? 0 : bits); }
 
-// Decide cluster bits so a CTA's tile part fits in shared memory.
+// Cluster bits of a tile of 2^m elements.  A pass alternates between waiting
+// for memory (gather, output) and shared memory (rounds), so two or three
+// CTAs per SM overlap where one of 135 KB does not: parts of at most 2^14
+// FP32 elements, and of 2^12 8-byte ones (34 KB; at most four CTAs, so 2^13 at
+// L = 30 and 2^14 at L = 32: eight CTAs there, 3.05 + 2.39 for 3.73 + 2.84 ms,
+// make the orders below so ragged that the FP32 passes lose 10%).
+// Pass 1 + pass 2 in us, one CTA per SM / this split:
+//   FP32  L = 32: 1066 + 705 / 923 + 659;  L = 30 (2^15 elements, c = 0) 220 + 162
+//         with its own order, 258 + 162 with the order of 4-CTA 8-byte parts,
+//         and 239 + 167 split four ways itself
+//   double-float  L = 30: 925 + 711 / 672 + 577;  L = 28: 245 + 180 / 174 + 140;
+//         L = 26: 67 + 52 / 53 + 47 (2^11 elements: 57 + 47)
+//   FP64  L = 30: 1494 + 1485 / 1260 + 1318;  L = 28: 408 + 408 / 334 + 354;
+//         L = 26: 108 + 110 / 92 + 96
 static int cluster_bits_for(int m, size_t elem) {
-  int c = 0;
-  while (((size_t)(1 << (m - c)) * elem * 33 / 32) > 200 * 1024) ++c;
+  int c = (elem == 8) ? std::min(2, std::max(0, m - 12)) : (m >= 15 ? 2 : 0);
   const int cap = g_eo_tile_bits_cap.load();
   if (cap > 0 && m - c > cap) c = m - cap;
   return c;
