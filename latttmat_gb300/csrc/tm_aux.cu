@@ -1124,7 +1124,8 @@ TreeDev tree_dev(const Op& op) {
 }  // namespace
 
 // y = T x (or T^T x for transposed views); scaled: FP32 result divided by the
-// returned factor.
+// returned factor, the step normalisation or, where the rest of the output
+// factor would take FP32 results out of their range (scale_fits), all of it.
 // T: arithmetic and pass-buffer type (float, double, or dfloat: FP64-accurate
 // products on the FP32 pipes); IO: element type of x and y.
 template <class T, class IO = T>
@@ -1151,7 +1152,9 @@ double matvec_aux_dir(const Op& op, const IO* x, IO* y, bool scaled, int dir, cu
   ChainIO<T, IO> io{};
   io.tv = op.tvec.as<double>();
   io.y = y;
-  io.post = scale_factor(((zb || reduced) ? 1.0 : op.normfactor) * sf);
+  const double f = ((zb || reduced) ? 1.0 : op.normfactor) * sf;
+  const bool whole = scaled && !scale_fits(f);
+  io.post = scale_factor(whole ? 1.0 : f);
   if (reduced) {
     U* u = op.ws_c.as<U>();
     chain_scale_in<U, IO><<<grid_for(op.n), 256, 0, s>>>(x, op.tvec.as<double>(), u, op.n);
@@ -1180,7 +1183,7 @@ double matvec_aux_dir(const Op& op, const IO* x, IO* y, bool scaled, int dir, cu
     TM_CKK("aux_chain");
     ++p;
   }
-  return scaled ? gscale : 1.0;
+  return scaled ? (whole ? gscale * f : gscale) : 1.0;
 }
 
 // ------------------------------------------------------------------ batch members

@@ -628,7 +628,9 @@ int64_t kron_power(const Op& op, const double* x, DBuf& part, cudaStream_t s) {
 
 // y = T x on the full space (K_XAT) or on the reduced basis through the full
 // space (reduced kinds whose core is the Kronecker factor).  scaled=true:
-// the result is divided by S = (e^K+e^-K)^L and S is returned.
+// the result is divided by the returned factor, S = (e^K+e^-K)^L or, where
+// what is left of the output factor would take FP32 results out of their
+// range (scale_fits), the whole of it.
 template <class T>
 double matvec_bfly(const Op& op, const T* x, T* y, bool scaled, cudaStream_t s) {
   const KronConst& kc = op.kron;
@@ -638,8 +640,10 @@ double matvec_bfly(const Op& op, const T* x, T* y, bool scaled, cudaStream_t s) 
   if (op.kind == K_XAT) {
     // y = nf * Tv^(1/2) * Th * Tv^(1/2) * x   (TMat/tmat.cpp:71-102)
     const double gin = (sizeof(T) == 8) ? 1.0 : kc.gin;
-    run_sweep<T>(op, x, y, 1, tv, gin, nullptr, 1, tv, op.normfactor * sf * (kc.gin / gin), s);
-    return ret;
+    const double f = op.normfactor * sf * (kc.gin / gin);
+    const bool whole = scaled && !scale_fits(f);
+    run_sweep<T>(op, x, y, 1, tv, gin, nullptr, 1, tv, whole ? 1.0 : f, s);
+    return whole ? ret * f : ret;
   }
   const uint32_t* smap = op.smap.as<uint32_t>();
   const uint32_t* idx = op.idx.as<uint32_t>();

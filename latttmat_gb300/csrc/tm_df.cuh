@@ -122,17 +122,24 @@ __device__ __forceinline__ void df2_mul(float2 xh, float2 xl, float2 wh, float2 
 
 // A constant factor of a result rounded to FP32 once (scale_round): f64, and
 // the same as two * hl with `two` a power of two near its square root, so
-// that partial products stay near the result's exponent range.
+// that partial products stay near the result's exponent range.  A factor that
+// does not fit (zero, negative or not finite ones too) has a NaN for `two`,
+// which no range check passes: every value then takes the FP64 form.
 struct ScaleF {
   double f64;
   float two;
   dfloat hl;
 };
-inline ScaleF scale_factor(double S) {
-  ScaleF p{S, 1.f, dfloat(1.0)};
+inline bool scale_fits(double S) {
   int e = 0;
   std::frexp(S, &e);
-  if (std::isfinite(S) && S > 0 && e > -120 && e < 120) {
+  return std::isfinite(S) && S > 0 && e > -120 && e < 120;
+}
+inline ScaleF scale_factor(double S) {
+  ScaleF p{S, std::nanf(""), dfloat(1.0)};
+  if (scale_fits(S)) {
+    int e = 0;
+    std::frexp(S, &e);
     p.two = std::ldexp(1.f, e / 2);
     p.hl = dfloat(S / (double)p.two);
   }
@@ -161,7 +168,7 @@ __device__ __forceinline__ float lo_of(dfloat v) { return v.lo; }
 __device__ __forceinline__ float scale_round(float v, dfloat sc, const ScaleF& post) {
   const float a = v * post.two;  // exact
   const float p = a * sc.hi;
-  if (v == 0.f) return p;
+  if (v == 0.f && p == 0.f) return p;
   if (!(fabsf(p) > 1e-24f && fabsf(p) < 1e24f)) return scale_round_f64(hi_of(v), lo_of(v), sc.hi, sc.lo, post.f64);
   const float e = fmaf(a, sc.lo, fmaf(a, sc.hi, -p));
   const float q = p * post.hl.hi;
@@ -172,7 +179,7 @@ __device__ __forceinline__ float scale_round(float v, dfloat sc, const ScaleF& p
 __device__ __forceinline__ float scale_round(dfloat v, dfloat sc, const ScaleF& post) {
   const float a = v.hi * post.two;  // exact
   const float p = a * sc.hi;
-  if (v.hi == 0.f) return p;
+  if (v.hi == 0.f && p == 0.f) return p;
   if (!(fabsf(p) > 1e-24f && fabsf(p) < 1e24f)) return scale_round_f64(hi_of(v), lo_of(v), sc.hi, sc.lo, post.f64);
   const float e = fmaf(v.lo * post.two, sc.hi, fmaf(a, sc.lo, fmaf(a, sc.hi, -p)));
   const float q = p * post.hl.hi;
