@@ -160,29 +160,37 @@ __device__ __forceinline__ float hi_of(dfloat v) { return v.hi; }
 __device__ __forceinline__ float lo_of(float) { return 0.f; }
 __device__ __forceinline__ float lo_of(dfloat v) { return v.lo; }
 
+// Whether the two-word products a = v * two, p = a * sc and q = p * post hold
+// all of a result: a has to be exact, the error terms of p representable, and q
+// neither infinite (also: p infinite or NaN) nor where its own error terms
+// would be lost.
+__device__ __forceinline__ bool scale_in_range(float a, float p, float q) {
+  return fabsf(a) > 1e-35f && fabsf(p) > 1e-24f && fabsf(q) > 1e-33f && fabsf(q) < 1e38f;
+}
+
 // (v * sc) * post rounded to FP32 once: the products' rounding errors are
 // carried along (TwoProduct by FMA), so the result is that of FP64 arithmetic
 // to within the last rounding, without the FP64 pipe (two lanes per clock and
 // SM, conversions included).  Infinities, NaN and products near the ends of
-// the exponent range, where the error terms would be lost, take the FP64 form.
+// the exponent range take the FP64 form.
 __device__ __forceinline__ float scale_round(float v, dfloat sc, const ScaleF& post) {
-  const float a = v * post.two;  // exact
+  const float a = v * post.two;
   const float p = a * sc.hi;
   if (v == 0.f && p == 0.f) return p;
-  if (!(fabsf(p) > 1e-24f && fabsf(p) < 1e24f)) return scale_round_f64(hi_of(v), lo_of(v), sc.hi, sc.lo, post.f64);
-  const float e = fmaf(a, sc.lo, fmaf(a, sc.hi, -p));
   const float q = p * post.hl.hi;
+  if (!scale_in_range(a, p, q)) return scale_round_f64(hi_of(v), lo_of(v), sc.hi, sc.lo, post.f64);
+  const float e = fmaf(a, sc.lo, fmaf(a, sc.hi, -p));
   return q + fmaf(e, post.hl.hi, fmaf(p, post.hl.lo, fmaf(p, post.hl.hi, -q)));
 }
 
 // the same for a double-float value
 __device__ __forceinline__ float scale_round(dfloat v, dfloat sc, const ScaleF& post) {
-  const float a = v.hi * post.two;  // exact
+  const float a = v.hi * post.two;
   const float p = a * sc.hi;
   if (v.hi == 0.f && p == 0.f) return p;
-  if (!(fabsf(p) > 1e-24f && fabsf(p) < 1e24f)) return scale_round_f64(hi_of(v), lo_of(v), sc.hi, sc.lo, post.f64);
-  const float e = fmaf(v.lo * post.two, sc.hi, fmaf(a, sc.lo, fmaf(a, sc.hi, -p)));
   const float q = p * post.hl.hi;
+  if (!scale_in_range(a, p, q)) return scale_round_f64(hi_of(v), lo_of(v), sc.hi, sc.lo, post.f64);
+  const float e = fmaf(v.lo * post.two, sc.hi, fmaf(a, sc.lo, fmaf(a, sc.hi, -p)));
   return q + fmaf(e, post.hl.hi, fmaf(p, post.hl.lo, fmaf(p, post.hl.hi, -q)));
 }
 

@@ -71,3 +71,34 @@ def test_factor_range(exe, kind, S):
             y = np.abs((hi.astype(np.float64) + lo) * t * S)
         keep = ~((y > 1e37) & np.isfinite(y) & (2.0 ** -120 < S) & (S < 2.0 ** 120))
         check(*run(exe, kind, hi[keep], lo[keep], t[keep], S))
+
+
+# a factor inside the range whose product with the value leaves it, at both ends: infinities as FP64 rounds them
+@pytest.mark.parametrize("kind", [0, 1])
+@pytest.mark.parametrize("S", [1e30, 1e35, 2.0 ** 118, 1e25, 1.0, 1e-25, 1e-35, 2.0 ** -118])
+def test_results_at_the_ends(exe, kind, S):
+    for seed, end in enumerate((2.0 ** 127, 2.0 ** 128, 2.0 ** 129, 1e45, 2.0 ** -110, 2.0 ** -126, 2.0 ** -140, 1e-50)):
+        r = np.random.default_rng(seed)
+        t = np.ldexp(r.uniform(0.5, 1, 400), r.integers(-30, 31, 400))
+        v = np.clip(end * r.uniform(0.5, 1.5, 400) / (S * t), 1e-36, 3e38) * r.choice([-1.0, 1.0], 400)
+        hi = v.astype(np.float32)
+        lo = (v - hi).astype(np.float32) if kind else np.zeros_like(hi)
+        check(*run(exe, kind, hi, lo, t, S))
+
+
+def test_infinite_and_nan_values(exe):
+    hi = np.array([np.inf, -np.inf, np.nan, 5e8, 1e4], dtype=np.float32)
+    for S in (1.0, 1e30, 1e35, 1e-35, 1e60):
+        check(*run(exe, 0, hi, np.zeros_like(hi), np.ones(5), S))
+
+
+# small values under large weights and small factors: the value times the factor's power of two is subnormal
+@pytest.mark.parametrize("kind", [0, 1])
+def test_subnormal_partial_products(exe, kind):
+    r = np.random.default_rng(0)
+    for S in (2.0 ** -80, 2.0 ** -118, 2.0 ** -40):
+        v = np.ldexp(r.uniform(-1, 1, 400), r.integers(-125, -60, 400))
+        t = np.ldexp(r.uniform(0.5, 1, 400), r.integers(40, 91, 400))
+        hi = v.astype(np.float32)
+        lo = (v - hi).astype(np.float32) if kind else np.zeros_like(hi)
+        check(*run(exe, kind, hi, lo, t, S))
