@@ -71,7 +71,7 @@ __device__ __forceinline__ void to_elem(dfloat u, dfloat& v) { v = u; }
 __device__ __forceinline__ void to_elem(dfloat u, tangent& v) { v = tangent(u, dfloat(0.f, 0.f)); }
 
 // x times its FP64 weight in the chain's arithmetic
-__device__ __forceinline__ void weigh_in(float x, double t, float& v) { v = scale_round(x, t, ScaleF{1.0, 1.f, dfloat(1.f, 0.f)}); }
+__device__ __forceinline__ void weigh_in(float x, double t, float& v) { v = scale_round(x, t); }
 __device__ __forceinline__ void weigh_in(double x, double t, float& v) { v = (float)(x * t); }
 __device__ __forceinline__ void weigh_in(double x, double t, double& v) { v = x * t; }
 __device__ __forceinline__ void weigh_in(double x, double t, dfloat& v) { v = dfloat(x * t); }
@@ -521,6 +521,25 @@ __device__ __forceinline__ void chain_first_two(unsigned char* sm, int plane, co
   }
 }
 
+// The fold of word w in FP64, for sums that leave the FP32 exponent range (two
+// FP32 words make a NaN of an infinite sum).  Not inlined: see scale_round_f64.
+__device__ __forceinline__ double part64(float x) { return x; }
+__device__ __forceinline__ double part64(double x) { return x; }
+__device__ __forceinline__ double part64(dfloat x) { return (double)x; }
+__device__ __forceinline__ double part64(tangent x) { return (double)x.d; }
+template <class T, int S>
+static __device__ __noinline__ double fold_f64(unsigned char* sm, int plane, int slot0, int nlb) {
+  double a = 0.0;
+  for (int t = 0; t < nlb; ++t) {
+    T v[S];
+    slot_ld<T, S>(sm, plane, slot0 | t, v);
+    for (int q = 0; q < S; ++q) a += part64(v[q]);
+  }
+  return a;
+}
+__device__ __forceinline__ bool fold_ok(dfloat a) { return fabsf(a.hi) < 3e38f; }
+__device__ __forceinline__ bool fold_ok(double) { return true; }
+
 // One block of a pass (the tables in sh are loaded and synchronised).
 //   KS = 1: DNNI (permute_mult_T1 / _last, TMat/tmat.cpp:344-376); KS = 2:
 //   diagonal BNNNI (TMat/tmat.cpp:521-588).
@@ -708,7 +727,9 @@ __device__ __forceinline__ void chain_block(const ChainIO<T, IO>& io, ChainShare
       const uint64_t r = out0 + i;
       double t = io.tv[r];
       if (io.dup) t *= (double)io.dup[r];
-      if constexpr (sizeof(IO) == 4)
+      if (!fold_ok(acc))
+        io.y[r] = (IO)(fold_f64<T, S>(sm, plane, w << cp.tb, tmask + 1) * t * io.post.f64);
+      else if constexpr (sizeof(IO) == 4)
         io.y[r] = scale_round(acc, t, io.post);
       else
         io.y[r] = (double)acc * t * io.post.f64;

@@ -194,19 +194,34 @@ __device__ __forceinline__ float scale_round(dfloat v, dfloat sc, const ScaleF& 
   return q + fmaf(e, post.hl.hi, fmaf(p, post.hl.lo, fmaf(p, post.hl.hi, -q)));
 }
 
-// v * t * post for an FP64 weight t: t is split into a double-float by
-// integer operations (the hi word truncated to 24 bits, the lo word the 29
-// bits below), so nothing runs on the FP64 pipe but the rare cases.
-template <class V>
-__device__ __forceinline__ float scale_round(V v, double t, const ScaleF& post) {
+// An FP64 weight as a double-float, by integer operations (the hi word
+// truncated to 24 bits, the lo word the 29 bits below), so that nothing runs
+// on the FP64 pipe but the rare cases; false where it does not fit.
+__device__ __forceinline__ bool weight_df(double t, dfloat& w) {
   const uint32_t up = (uint32_t)__double2hiint(t), dn = (uint32_t)__double2loint(t);
   const int e = (int)((up >> 20) & 0x7ffu) - 1023;
-  if (e < -70 || e > 90) return scale_round_f64(hi_of(v), lo_of(v), t, post.f64);
   const uint32_t sign = up & 0x80000000u;
   const uint32_t m23 = ((up & 0xfffffu) << 3) | (dn >> 29);
-  const float hi = __uint_as_float(sign | ((uint32_t)(e + 127) << 23) | m23);
-  const float lo = __uint2float_rn(dn & 0x1fffffffu) * __uint_as_float(sign | ((uint32_t)(e - 52 + 127) << 23));
-  return scale_round(v, dfloat(hi, lo), post);
+  w.hi = __uint_as_float(sign | ((uint32_t)(e + 127) << 23) | m23);
+  w.lo = __uint2float_rn(dn & 0x1fffffffu) * __uint_as_float(sign | ((uint32_t)(e - 52 + 127) << 23));
+  return e >= -70 && e <= 90;
+}
+
+// v * t * post for an FP64 weight t
+template <class V>
+__device__ __forceinline__ float scale_round(V v, double t, const ScaleF& post) {
+  dfloat w;
+  if (!weight_df(t, w)) return scale_round_f64(hi_of(v), lo_of(v), t, post.f64);
+  return scale_round(v, w, post);
+}
+
+// v * t rounded to FP32 once
+__device__ __forceinline__ float scale_round(float v, double t) {
+  dfloat w;
+  const bool fits = weight_df(t, w);
+  const float p = v * w.hi;
+  if (!fits || !((fabsf(p) > 1e-24f && fabsf(p) < 1e38f) || v == 0.f)) return scale_round_f64(v, 0.f, t, 1.0);
+  return p + fmaf(v, w.lo, fmaf(v, w.hi, -p));
 }
 
 // Forward-mode tangent pair (value, derivative with respect to one

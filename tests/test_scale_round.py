@@ -102,3 +102,11 @@ def test_subnormal_partial_products(exe, kind):
         hi = v.astype(np.float32)
         lo = (v - hi).astype(np.float32) if kind else np.zeros_like(hi)
         check(*run(exe, kind, hi, lo, t, S))
+
+
+@pytest.mark.parametrize("vexp,texp", [(3, 3), (30, 40), (120, 60), (126, 100), (60, 900)])
+def test_without_factor(exe, vexp, texp):
+    hi, lo, t = values(vexp, 0, vexp, texp)
+    hi[5:9] = np.inf, -np.inf, np.nan, 0.0
+    t[8:10] = np.inf, 0.0
+    check(*run(exe, 2, hi, lo, t, 1.0))
