@@ -566,7 +566,11 @@ int64_t kron_power(const Op& op, const double* x, DBuf& part, cudaStream_t s) {
   const uint32_t* smap = op.smap.as<uint32_t>();
   if (reduced && shifts && !op.grp.flip && L > kSmallBits) {
     // (an even/odd operator has no tree of its own; it keeps this one)
-    if (!op.tree.nlev) build_prefix_tree(op, L, tree_steps(L), false, const_cast<Op&>(op).tree);
+    {
+      Op& o = const_cast<Op&>(op);
+      std::lock_guard<std::mutex> lock(o.lazy_mu);
+      if (!o.tree.nlev) build_prefix_tree(op, L, tree_steps(L), false, o.tree);
+    }
     const PrefixTree& t = op.tree;
     for (int k = 0; k <= L; ++k) pw.d[k] = dlam(k);
     int64_t most[2];

@@ -5,6 +5,7 @@
 #include <stdint.h>
 
 #include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -163,6 +164,7 @@ struct Op {
   DBuf smap;       // u32 [nstate]
   KronConst kron;
   PrefixTree tree; // translation groups: output prefixes that lead to a representative
+  std::mutex lazy_mu;  // held while a first gradient adds smap or tree to a finished operator
   // pi order (internal vector order): pi[k] = reference index; identity if empty
   bool has_pi = false;
   DBuf pi, pinv;   // u32 [n]

@@ -282,6 +282,7 @@ void build_orbit_table(Op& op) {
 // its rank structure): rebuild the representative bitset and prefix in
 // temporaries, then map every state.
 void ensure_state_map(Op& op) {
+  std::lock_guard<std::mutex> lock(op.lazy_mu);
   if (op.smap.p) return;
   if (op.L > 30) fail(TM_ERR_LIMIT, "full-space state map limited to L <= 30");
   GroupDev g = to_dev(op.grp);

@@ -143,10 +143,9 @@ void build_prefix_tree(const Op& op, int nbits, const std::vector<int>& steps, b
   TM_CKK("tree_count");
   tree_scan_kernel<<<nlev + 1, kTreeBlock, 0, s>>>(cnt.as<uint32_t>(), nblk, tot);
   TM_CKK("tree_scan");
-  uint32_t h[kTreeMaxLevels + 1];
+  uint32_t h[kTreeMaxLevels + 1] = {0};
   TM_CK(cudaMemcpyAsync(h, tot, (size_t)(nlev + 1) * 4, cudaMemcpyDeviceToHost, s));
   TM_CK(cudaStreamSynchronize(s));
-  out.nlev = nlev;
   int64_t sum = 0;
   for (int i = 0; i <= nlev; ++i) {
     out.b[i] = T.b[i];
@@ -161,6 +160,7 @@ void build_prefix_tree(const Op& op, int nbits, const std::vector<int>& steps, b
   for (int i = 0; words && i <= nlev; ++i) T.words[i] = out.words.as<uint16_t>() + out.off[i];
   tree_fill_kernel<<<(unsigned)nblk, kTreeBlock, 0, s>>>(op.idx.as<uint32_t>(), n, T, cnt.as<uint32_t>());
   TM_CKK("tree_fill");
+  out.nlev = nlev;  // (last: a tree whose tables could not be built is no tree)
   // the counts are released on return: in stream order, or by a synchronising
   // cudaFree outside an allocation scope
 }
