@@ -32,7 +32,6 @@
 #include <algorithm>
 #include <cmath>
 #include <functional>
-#include <mutex>
 #include <type_traits>
 #include <vector>
 
@@ -1039,44 +1038,7 @@ void to_f32_dev(const double* x, float* y, int64_t n, cudaStream_t s) {
   TM_CKK("tune_f32");
 }
 
-// ------------------------------------------------------------------ pass plans and tuning
-// Tile bits and threads per block of the chain passes, per (element size,
-// carried bits, width): 2^13-element tiles and 256 threads for 4-byte
-// elements, 2^12 and 128 for 8-byte ones (32 KB either way; 64 or more groups
-// per warp-round at either size).  Over BNNNI widths 16-24 and DNNI widths
-// 20-26 these are within 10% of the fastest of all tile and block sizes;
-// tm_chain_autotune and tm_chain_set_tuning override entries at run time.
-namespace {
-struct ChainTune {
-  int tile_bits = 0, threads = 0;
-};
-std::mutex g_tune_mu;
-ChainTune g_tune[2][2][33];  // [elem 4/8][zb][L]
-}  // namespace
-
-void chain_tuning(int L, size_t elem, bool zb, int& tile_bits, int& threads) {
-  if (elem >= 16) {  // tangent pairs (adjoint): 32 KB tiles, fewer threads
-    tile_bits = 11;
-    threads = 128;
-    return;
-  }
-  tile_bits = (elem == 8) ? 12 : 13;
-  threads = (elem == 8) ? 128 : 256;
-  if (L < 0 || L > 32) return;
-  std::lock_guard<std::mutex> lock(g_tune_mu);
-  const ChainTune& t = g_tune[elem == 8][zb ? 1 : 0][L];
-  if (t.tile_bits) tile_bits = t.tile_bits;
-  if (t.threads) threads = t.threads;
-}
-
-void chain_set_tuning(int L, size_t elem, bool zb, int tile_bits, int threads) {
-  if (L < 0 || L > 32) fail(TM_ERR_ARG, "width out of range");
-  if (tile_bits && (tile_bits < 10 || tile_bits > (elem == 8 ? 13 : 14))) fail(TM_ERR_ARG, "tile bits out of range");
-  if (threads && threads != 64 && threads != 128 && threads != 256) fail(TM_ERR_ARG, "threads must be 64, 128 or 256");
-  std::lock_guard<std::mutex> lock(g_tune_mu);
-  g_tune[elem == 8][zb ? 1 : 0][L] = ChainTune{tile_bits, threads};
-}
-
+// ------------------------------------------------------------------ pass plans
 // The passes of one product.  A tile of 2^tile_bits elements holds the carried
 // letter, a chunk of the old bits below the pass's letters (at
 // least 128 bytes' worth of slots, for coalescing) and the pass's letters; the
@@ -1312,50 +1274,44 @@ void chain_autotune(const Op& op0, tm_dtype dt, int& best_tb, int& best_th, doub
   y32.alloc((size_t)op.n * 4);
   fill_uniform_dev(x.as<double>(), op.n, 7, s);
   to_f32_dev(x.as<double>(), x32.as<float>(), op.n, s);
-  int tb0 = 0, th0 = 0;
-  chain_tuning(op.L, elem, zb, tb0, th0);
+  chain_tuning(op.L, elem, zb, best_tb, best_th);
   const int tbs[4] = {11, 12, 13, 14};
   const int ths[2] = {128, 256};
-  cudaEvent_t e0, e1;
-  TM_CK(cudaEventCreate(&e0));
-  TM_CK(cudaEventCreate(&e1));
+  ChainTuneKeep tried(op.L, elem, zb);  // the entry as it was, should a step throw
+  struct Events {
+    cudaEvent_t e[2] = {nullptr, nullptr};
+    ~Events() {
+      for (cudaEvent_t v : e)
+        if (v) cudaEventDestroy(v);
+    }
+  } ev;
+  for (cudaEvent_t& v : ev.e) TM_CK(cudaEventCreate(&v));
   best_ms = 1e30;
-  best_tb = tb0;
-  best_th = th0;
-  try {
-    for (int tb : tbs) {
-      if (tb > (elem == 8 ? 13 : 14)) continue;
-      for (int th : ths) {
-        chain_set_tuning(op.L, elem, zb, tb, th);
-        auto run = [&]() {
-          if (elem == 4)
-            matvec_aux_dir<float>(op, x32.as<float>(), y32.as<float>(), true, 0, s);
-          else
-            matvec_aux_dir<dfloat, double>(op, x.as<double>(), y.as<double>(), false, 0, s);
-        };
-        run();
-        TM_CK(cudaEventRecord(e0, s));
-        for (int r = 0; r < 3; ++r) run();
-        TM_CK(cudaEventRecord(e1, s));
-        TM_CK(cudaEventSynchronize(e1));
-        float ms = 0.f;
-        TM_CK(cudaEventElapsedTime(&ms, e0, e1));
-        if (ms / 3.0 < best_ms) {
-          best_ms = ms / 3.0;
-          best_tb = tb;
-          best_th = th;
-        }
+  for (int tb : tbs) {
+    if (tb > (elem == 8 ? 13 : 14)) continue;
+    for (int th : ths) {
+      chain_set_tuning(op.L, elem, zb, tb, th);
+      auto run = [&]() {
+        if (elem == 4)
+          matvec_aux_dir<float>(op, x32.as<float>(), y32.as<float>(), true, 0, s);
+        else
+          matvec_aux_dir<dfloat, double>(op, x.as<double>(), y.as<double>(), false, 0, s);
+      };
+      run();
+      TM_CK(cudaEventRecord(ev.e[0], s));
+      for (int r = 0; r < 3; ++r) run();
+      TM_CK(cudaEventRecord(ev.e[1], s));
+      TM_CK(cudaEventSynchronize(ev.e[1]));
+      float ms = 0.f;
+      TM_CK(cudaEventElapsedTime(&ms, ev.e[0], ev.e[1]));
+      if (ms / 3.0 < best_ms) {
+        best_ms = ms / 3.0;
+        best_tb = tb;
+        best_th = th;
       }
     }
-  } catch (...) {
-    chain_set_tuning(op.L, elem, zb, tb0 == ((elem == 8) ? 12 : 13) ? 0 : tb0, th0 == 256 ? 0 : th0);
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    throw;
   }
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
-  chain_set_tuning(op.L, elem, zb, best_tb, best_th);
+  tried.set(best_tb, best_th);
 }
 
 template <class T>

@@ -151,6 +151,20 @@ inline AuxCoef aux_coef_derivative(double bj, double k, double k2, int t) {
 AuxCoef coef_of(const Op& op);
 void chain_tuning(int L, size_t elem, bool zb, int& tile_bits, int& threads);
 void chain_set_tuning(int L, size_t elem, bool zb, int tile_bits, int threads);
+// Puts a width's table entry (0: the default) back at the end of its scope, or
+// another one if set.
+struct ChainTune {
+  int tile_bits = 0, threads = 0;
+};
+struct ChainTuneKeep {
+  int L;
+  size_t elem;
+  bool zb;
+  ChainTune entry;
+  ChainTuneKeep(int L, size_t elem, bool zb);
+  ~ChainTuneKeep();
+  void set(int tile_bits, int threads) { entry = ChainTune{tile_bits, threads}; }
+};
 std::vector<ChainPass> chain_plan(const Op& op, size_t elem, int tile_bits);
 int64_t chain_pass_blocks(const ChainPass& cp);
 size_t chain_pass_smem(const ChainPass& cp, bool zb, size_t elem);
