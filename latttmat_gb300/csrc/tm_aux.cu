@@ -296,9 +296,9 @@ struct ChainIO {
   const T* src;        // previous pass's output
   T* dst;              // this pass's output
   const typename ChainIn<T>::U* u;  // first pass: input times Tvec, or null:
-  const IO* x;         //   x[r] * pre[r]
+  const IO* x;         //   x * pre
   const double* pre;
-  const uint32_t* smap;  // reduced: state -> row of u
+  const uint32_t* smap;  // reduced: state -> row
   IO* y;               // last pass
   const double* tv;    //   y = sum * tv [* dup] * post
   const uint16_t* dup;
@@ -489,7 +489,8 @@ __device__ __forceinline__ void chain_first_two(unsigned char* sm, int plane, co
 #pragma unroll
       for (int a = 0; a < S; ++a) {
         const uint64_t r = ((uint64_t)lb << (L - KS)) | ((uint64_t)a << (L - 2 * KS)) | below;
-        weigh_in(io.x[r], io.pre[r], x[a]);
+        const uint64_t at = io.smap ? io.smap[r] : r;
+        weigh_in(io.x[at], io.pre[at], x[a]);
       }
     }
     // (a ring of two letters: the bottom letter is the second, the third the first)
@@ -650,7 +651,8 @@ __device__ __forceinline__ void chain_block(const ChainIO<T, IO>& io, ChainShare
             if (e < (1 << fb) && a < na) {
               const int top = bc ? a : (cp.last ? e & tmask : lb_outer);
               const uint64_t r = ((uint64_t)top << (L - KS)) | below[h];
-              weigh_in(io.x[r], io.pre[r], v[h][a]);
+              const uint64_t at = io.smap ? io.smap[r] : r;
+              weigh_in(io.x[at], io.pre[at], v[h][a]);
             }
           }
       }
@@ -770,7 +772,10 @@ __global__ void __launch_bounds__(256, chain_min_blocks<T>())
   chain_block<T, KS, IO>(io, sh, cp, tr, L, bc, blockIdx.x);
 }
 
-// u = x tvec in the product's arithmetic
+// u = x tvec in the product's arithmetic, for reduced operators above
+// kChainFold bits.  Below, the first pass gathers x and the weight of every
+// state itself: the 2^L gathers more cost less than a launch there.
+constexpr int kChainFold = 14;
 template <class U, class IO>
 __global__ void chain_scale_in(const IO* __restrict__ x, const double* __restrict__ tv, U* __restrict__ u, int64_t n) {
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1045,7 +1050,12 @@ void to_f32_dev(const double* x, float* y, int64_t n, cudaStream_t s) {
 // last pass has no bits below, holds the lastbit values instead and takes as
 // many letters as fit; the others share the rest evenly, the first one (whose
 // gathers want long chunks) the fewest.
-std::vector<ChainPass> chain_plan(const Op& op, size_t elem, int tile_bits) {
+//   Small operators would leave most SMs without a block that way (DNNI, full,
+// open, L = 12 in FP64: two blocks of 2^11 slots in the last pass): the last
+// pass then hands letters to the others, down to an even split, and the chunks
+// shrink to two slots, until a pass has `blocks` blocks.  The buffers of such
+// operators stay in L2, where short runs cost little.
+ChainPlan chain_plan(const Op& op, size_t elem, int tile_bits, int blocks) {
   const bool zb = (op.kind == K_ZBT || op.kind == K_ZBM);
   const int KS = zb ? 2 : 1, m = op.L / KS;
   const int bc = zb ? 0 : op.boundary;
@@ -1054,11 +1064,14 @@ std::vector<ChainPass> chain_plan(const Op& op, size_t elem, int tile_bits) {
   const int lbb = (bc == 0) ? KS : 0;
   const int capl = std::min(kChainMaxT, std::max(1, (tile_bits - KS - lbb) / KS));
   const int cap = std::min(kChainMaxT, std::max(1, (tile_bits - KS - cbn) / KS));
-  const int lead = std::max(0, m - capl);  // letters before the last pass
+  int lead = std::max(0, m - capl);  // letters before the last pass
   const int npass = 1 + (lead + cap - 1) / cap;
-  std::vector<ChainPass> out;
-  int t0 = 0;
+  if (npass > kChainMaxPass) fail(TM_ERR_LIMIT, "too many chain passes");
   auto nodes = [&](int t) { return op.tree.nlev ? op.tree.n[t] : (int64_t)1 << (KS * t); };
+  const int even = std::min(cap * (npass - 1), m * (npass - 1) / npass);
+  while (lead < even && nodes(lead) < blocks) ++lead;
+  ChainPlan out;
+  int t0 = 0;
   for (int p = 0; p < npass; ++p) {
     ChainPass cp{};
     cp.t0 = t0;
@@ -1068,10 +1081,11 @@ std::vector<ChainPass> chain_plan(const Op& op, size_t elem, int tile_bits) {
     cp.first = (p == 0);
     cp.last = (p == npass - 1);
     cp.nlb = (bc == 0) ? 1 << KS : 1;
-    cp.tb = cp.last ? lbb : cp.cb;
     cp.nin = nodes(t0);
     cp.nout = nodes(t0 + cp.T);
-    out.push_back(cp);
+    while (cp.cb > 1 && chain_pass_blocks(cp) < blocks) --cp.cb;
+    cp.tb = cp.last ? lbb : cp.cb;
+    out.p[out.n++] = cp;
     t0 += cp.T;
   }
   return out;
@@ -1088,10 +1102,10 @@ size_t chain_pass_smem(const ChainPass& cp, bool zb, size_t elem) {
 }
 // (a full operator's passes write every element where they read it: one
 // buffer, in place)
-void chain_buffer_elems(const Op& op, const std::vector<ChainPass>& plan, int64_t need[2]) {
+void chain_buffer_elems(const Op& op, const ChainPlan& plan, int64_t need[2]) {
   const bool zb = (op.kind == K_ZBT || op.kind == K_ZBM);
   need[0] = need[1] = 0;
-  for (size_t p = 0; p + 1 < plan.size(); ++p)
+  for (int p = 0; p + 1 < plan.n; ++p)
     need[op.tree.nlev ? p & 1 : 0] = std::max(need[op.tree.nlev ? p & 1 : 0], ((int64_t)plan[p].nlb * plan[p].nout) << (plan[p].rest + (zb ? 2 : 1)));
 }
 
@@ -1138,16 +1152,17 @@ double matvec_aux_dir(const Op& op, const IO* x, IO* y, bool scaled, int dir, cu
   const double f = ((zb || reduced) ? 1.0 : op.normfactor) * sf;
   const bool whole = scaled && !scale_fits(f);
   io.post = scale_factor(whole ? 1.0 : f);
+  io.x = x;
+  io.pre = op.tvec.as<double>();
   if (reduced) {
-    U* u = op.ws_c.as<U>();
-    chain_scale_in<U, IO><<<grid_for(op.n), 256, 0, s>>>(x, op.tvec.as<double>(), u, op.n);
-    TM_CKK("chain_scale_in");
-    io.u = u;
     io.smap = op.smap.as<uint32_t>();
     io.dup = op.dup.as<uint16_t>();
-  } else {
-    io.x = x;
-    io.pre = op.tvec.as<double>();
+    if (L > kChainFold) {
+      U* u = op.ws_c.as<U>();
+      chain_scale_in<U, IO><<<grid_for(op.n), 256, 0, s>>>(x, op.tvec.as<double>(), u, op.n);
+      TM_CKK("chain_scale_in");
+      io.u = u;
+    }
   }
   const TreeDev tr = tree_dev(op);
   int p = 0;
@@ -1196,10 +1211,9 @@ void chain_inst_fill(const Op& op, int dir, ChainInst& rec, int tb4, int tb8) {
   if (tb8 <= 0) chain_tuning(L, 8, zb, tb8, th);
   int tb16 = 0;
   chain_tuning(L, 16, zb, tb16, th);
-  const std::vector<ChainPass> p16 = chain_plan(op, 16, tb16);
-  if ((int)p16.size() > kChainMaxPass) fail(TM_ERR_LIMIT, "too many chain passes");
-  rec.np16 = (int)p16.size();
-  for (int q = 0; q < rec.np16; ++q) rec.p16[q] = p16[q];
+  const ChainPlan p16 = chain_plan(op, 16, tb16, 0);
+  rec.np16 = p16.n;
+  std::copy(p16.begin(), p16.end(), rec.p16);
   for (int t = 0; t < 3; ++t) {
     const AuxCoef db = aux_coef_derivative(op.mp.betaJ, op.mp.kappa, op.mp.kappa2, t);
     chain_tab<tangent>(zb, dir, c, &db, true, rec.ctan[t]);  // the normalisation is a constant: no derivative
@@ -1210,12 +1224,11 @@ void chain_inst_fill(const Op& op, int dir, ChainInst& rec, int tb4, int tb8) {
   rec.kap = op.mp.kappa;
   rec.kap2 = op.mp.kappa2;
   rec.h = op.mp.h;
-  const std::vector<ChainPass> p4 = chain_plan(op, 4, tb4), p8 = chain_plan(op, 8, tb8);
-  if ((int)p4.size() > kChainMaxPass || (int)p8.size() > kChainMaxPass) fail(TM_ERR_LIMIT, "too many chain passes");
-  rec.np4 = (int)p4.size();
-  rec.np8 = (int)p8.size();
-  for (int q = 0; q < rec.np4; ++q) rec.p4[q] = p4[q];
-  for (int q = 0; q < rec.np8; ++q) rec.p8[q] = p8[q];
+  const ChainPlan p4 = chain_plan(op, 4, tb4, 0), p8 = chain_plan(op, 8, tb8, 0);
+  rec.np4 = p4.n;
+  rec.np8 = p8.n;
+  std::copy(p4.begin(), p4.end(), rec.p4);
+  std::copy(p8.begin(), p8.end(), rec.p8);
   rec.smap = reduced ? op.smap.as<uint32_t>() : nullptr;
   rec.tvec = op.tvec.as<double>();
   rec.idx = reduced ? op.idx.as<uint32_t>() : nullptr;

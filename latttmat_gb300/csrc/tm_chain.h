@@ -165,11 +165,22 @@ struct ChainTuneKeep {
   ~ChainTuneKeep();
   void set(int tile_bits, int threads) { entry = ChainTune{tile_bits, threads}; }
 };
-std::vector<ChainPass> chain_plan(const Op& op, size_t elem, int tile_bits);
+// The passes of one product, and the least blocks that a pass should have
+// where the operator's size lets it choose (0: a batch fills the launch).
+struct ChainPlan {
+  int n = 0;
+  ChainPass p[kChainMaxPass];
+  int size() const { return n; }
+  const ChainPass* begin() const { return p; }
+  const ChainPass* end() const { return p + n; }
+  const ChainPass& operator[](int i) const { return p[i]; }
+};
+constexpr int kChainBlocks = 256;
+ChainPlan chain_plan(const Op& op, size_t elem, int tile_bits, int blocks = kChainBlocks);
 int64_t chain_pass_blocks(const ChainPass& cp);
 size_t chain_pass_smem(const ChainPass& cp, bool zb, size_t elem);
 // elements of the two pass buffers that a plan writes
-void chain_buffer_elems(const Op& op, const std::vector<ChainPass>& plan, int64_t need[2]);
+void chain_buffer_elems(const Op& op, const ChainPlan& plan, int64_t need[2]);
 
 // Fill the geometry and coefficients of `rec` for operator `op` (an aux-bit
 // operator; dir 1 for its transpose), with tiles of 2^tb4 (4-byte) and 2^tb8

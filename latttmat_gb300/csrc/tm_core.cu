@@ -132,9 +132,10 @@ void launch_tile(int64_t nblocks, int threads, size_t shm, cudaStream_t s, const
   TM_CKK("kron_tile");
 }
 
-// The passes of a full-space product.  Up to 9 bits go in one pass (one
-// block; a second launch would cost more than its 9 levels), else the bits
-// are spread over ceil(L / 9) (FP64) or ceil(L / 10) passes.  A block takes
+// The passes of a full-space product.  Up to 9 bits (FP32: 10) go in one pass
+// (one block; a second launch would cost more than its levels: FP32 at L = 10
+// took 8.2 us in two passes), else the bits are spread over ceil(L / 9) (FP64)
+// or ceil(L / 10) passes.  A block takes
 // up to 16 contiguous positions beside the mixed ones, fewer where that would
 // leave SMs without a block: at small L the FP64 pipe of one SM is the limit
 // (L = 12 in one 4096-element block took 38 us).  Threads: 16 elements each
@@ -147,7 +148,7 @@ struct TilePass {
 };
 int tile_passes(int L, size_t elem) {
   const int most = (elem == 8) ? 9 : 10;
-  return (L <= 9) ? 1 : std::max(2, (L + most - 1) / most);
+  return (L + most - 1) / most;
 }
 // the pass that starts at bit lo, with `left` passes to go
 TilePass tile_pass(int L, int lo, int left, size_t elem) {
@@ -440,24 +441,29 @@ void run_tree(const Op& op, const T* u, T* y, bool fold, double gin, double post
 }
 
 // ------------------------------------------------------------------ small operators
-// A whole reduced product of up to 2^11 states in one block: expand, mix,
-// contract (y may be x: every read of x precedes the first barrier).  Launches are what a small product costs (about 2.5 us each
-// against 1.1 us of FP64 work at L = 9): from L = 12 on one SM's FP64 pipe
-// would take longer than the tree's launches.
-constexpr int kSmallBits = 11;
+// A whole reduced product in one block: expand, mix, contract (y may be x:
+// every read of x precedes the first barrier).  Launches are what a small
+// product costs (about 2.5 us each).  In FP64 one SM's pipe takes 1.1 us at
+// L = 9 and longer than the tree's launches from L = 12 on; FP32 has 64 times
+// the rate and stays in one block up to 12 bits (at 13: 22.6 us, the open
+// boundary's tile passes 16.4, a tree 20.5).
 template <class T>
-__global__ void __launch_bounds__(512) kron_small_kernel(const T* x, const uint32_t* __restrict__ smap,
-                                                         const uint32_t* __restrict__ idx,
-                                                         const uint16_t* __restrict__ dup,
-                                                         const double* __restrict__ tv, int L, Kron<T> c, double gin,
-                                                         double post, T* y, int n) {
-  __shared__ T sm[(1 << kSmallBits) + (1 << kSmallBits) / 32 + 1];
+constexpr int small_bits() {
+  return sizeof(T) == 4 ? 12 : 11;
+}
+template <class T, int KB>
+__global__ void __launch_bounds__(1024) kron_small_kernel(const T* x, const uint32_t* __restrict__ smap,
+                                                          const uint32_t* __restrict__ idx,
+                                                          const uint16_t* __restrict__ dup,
+                                                          const double* __restrict__ tv, int L, Kron<T> c, double gin,
+                                                          double post, T* y, int n) {
+  __shared__ T sm[(1 << small_bits<T>()) + (1 << small_bits<T>()) / 32 + 1];
   for (int i = threadIdx.x; i < (1 << L); i += blockDim.x) {
     const uint32_t q = smap[i];
     sm[spad(i)] = (T)((double)x[q] * tv[q] * gin);
   }
   __syncthreads();
-  tile_rounds<T, 2, Kron<T>>(sm, L, 0, 0, c);
+  tile_rounds<T, KB, Kron<T>>(sm, L, 0, 0, c);
   for (int i = threadIdx.x; i < n; i += blockDim.x)
     y[i] = (T)((double)sm[spad((int)idx[i])] * post * (double)dup[i] * tv[i]);
 }
@@ -519,7 +525,7 @@ void build_bfly(Op& op) {
   kc.out32 = (double)(emax * std::pow((1.0L + rl) / (1.0L + (long double)kron_of<float>(op).r), n));
   if (op.kind == K_XAT) return;
   const bool shifts = (op.kind == K_XAM && op.grp.periodic) || op.kind == K_XAM3;
-  if (op.L <= kSmallBits) return;
+  if (op.L <= small_bits<double>()) return;
   if (!shifts) {
     op.ws_a.alloc((size_t)op.nstate * 8);
     return;
@@ -564,7 +570,7 @@ int64_t kron_power(const Op& op, const double* x, DBuf& part, cudaStream_t s) {
     TM_CKK("scale_in");
   }
   const uint32_t* smap = op.smap.as<uint32_t>();
-  if (reduced && shifts && !op.grp.flip && L > kSmallBits) {
+  if (reduced && shifts && !op.grp.flip && L > small_bits<double>()) {
     // (an even/odd operator has no tree of its own; it keeps this one)
     {
       Op& o = const_cast<Op&>(op);
@@ -653,8 +659,11 @@ double matvec_bfly(const Op& op, const T* x, T* y, bool scaled, cudaStream_t s) 
   const uint32_t* idx = op.idx.as<uint32_t>();
   const uint16_t* dup = op.dup.as<uint16_t>();
   // reduced: u = Tvec .* x ; v = P u ; z = Th v ; y = dup .* Tvec .* z[idx]
-  if (op.L <= kSmallBits) {
-    kron_small_kernel<T><<<1, 512, 0, s>>>(x, smap, idx, dup, tv, op.L, kron_of<T>(op), kc.gin, sf, y, (int)op.n);
+  if (op.L <= small_bits<T>()) {
+    if (op.L <= 11)
+      kron_small_kernel<T, 2><<<1, 512, 0, s>>>(x, smap, idx, dup, tv, op.L, kron_of<T>(op), kc.gin, sf, y, (int)op.n);
+    else
+      kron_small_kernel<T, 3><<<1, 1024, 0, s>>>(x, smap, idx, dup, tv, op.L, kron_of<T>(op), kc.gin, sf, y, (int)op.n);
     TM_CKK("kron_small");
     return ret;
   }

@@ -382,7 +382,7 @@ struct Sweep {
       }
       for (int tb = t0; tb <= t1; ++tb) {
         int64_t need[2];
-        chain_buffer_elems(o, chain_plan(o, e, tb), need);
+        chain_buffer_elems(o, chain_plan(o, e, tb, 0), need);
         for (int k = 0; k < 2; ++k) most[k] = std::max(most[k], (size_t)need[k] * e);
       }
     }
