@@ -893,12 +893,15 @@ struct Dual {
 Dual operator*(Dual a, Dual b) { return Dual(a.v * b.v, a.d * b.v + a.v * b.d); }
 Dual operator/(Dual a, Dual b) { return Dual(a.v / b.v, (a.d - a.v / b.v * b.d) / b.v); }
 
+double value(double x) { return x; }
+double value(Dual x) { return x.v; }
+template <class T>
+T tab_elem(double x) {
+  return (T)x;
+}
 template <class T>
 T tab_elem(Dual x) {
-  if constexpr (std::is_same<T, tangent>::value)
-    return tangent(x.v, x.d);
-  else
-    return (T)x.v;
+  return tangent(x.v, x.d);
 }
 
 // The step tables (see ChainTab) from the factors b1 = e^{+-K}, b2 =
@@ -913,24 +916,31 @@ T tab_elem(Dual x) {
 template <class T>
 double chain_tab(bool zb, int dir, const AuxCoef& c, const AuxCoef* dc, bool norm, ChainTab<T>& tab,
                  double* bias = nullptr) {
-  Dual b1[2], b2[2], b3[2];
+  // (formed for every product: plain values but for tangent pairs)
+  using D = typename std::conditional<std::is_same<T, tangent>::value, Dual, double>::type;
+  D b1[2], b2[2], b3[2];
   for (int k = 0; k < 2; ++k) {
-    b1[k] = Dual(c.b1[k], dc ? dc->b1[k] : 0.0);
-    b2[k] = Dual(c.b2[k], dc ? dc->b2[k] : 0.0);
-    b3[k] = Dual(c.b3[k], dc ? dc->b3[k] : 0.0);
+    b1[k] = D(c.b1[k]);
+    b2[k] = D(c.b2[k]);
+    b3[k] = D(c.b3[k]);
+    if constexpr (std::is_same<T, tangent>::value) {
+      b1[k].d = dc->b1[k];
+      b2[k].d = dc->b2[k];
+      b3[k].d = dc->b3[k];
+    }
   }
   const int S = zb ? 4 : 2;
-  Dual rho1 = b2[1] / b2[0], rho2[4], w1[16], zu[64];
+  D rho1 = b2[1] / b2[0], rho2[4] = {}, w1[16] = {}, zu[64] = {};
   if (!zb) {
     for (int s = 0; s < 2; ++s)
       for (int q = 0; q < 2; ++q) {
-        w1[s * 2 + q] = (s == q) ? Dual(1.0) : rho1;
+        w1[s * 2 + q] = (s == q) ? D(1.0) : rho1;
         for (int k = 0; k < 2; ++k) zu[k * 4 + s * 2 + q] = b2[k ^ s] * b1[s ^ q] * b2[0];  // q is a' here
       }
   } else {
     for (int s = 0; s < 4; ++s) {
       const int sl = s >> 1, sr = s & 1;
-      Dual f = b2[0] * b2[sr];
+      D f = b2[0] * b2[sr];
       rho2[s] = b2[sr ^ 1] / b2[sr];
       if (dir) {
         f = f * b1[sl];
@@ -938,12 +948,12 @@ double chain_tab(bool zb, int dir, const AuxCoef& c, const AuxCoef* dc, bool nor
       }
       for (int q = 0; q < 4; ++q) {
         const int ql = q >> 1, qr = q & 1;
-        w1[s * 4 + q] = (sl == ql ? Dual(1.0) : rho1) * (qr ? rho2[s] : Dual(1.0));
+        w1[s * 4 + q] = (sl == ql ? D(1.0) : rho1) * (qr ? rho2[s] : D(1.0));
         // q as a' = (pl, pr)
-        const Dual u = (dir ? b1[sl ^ qr] : b1[sr ^ ql]) * b3[sr ^ qr] * b3[sl ^ ql];
+        const D u = (dir ? b1[sl ^ qr] : b1[sr ^ ql]) * b3[sr ^ qr] * b3[sl ^ ql];
         for (int k = 0; k < 4; ++k) {
           const int cl = k >> 1, cr = k & 1;
-          const Dual z = dir ? b2[sr ^ cr] * b2[sl ^ cl] : b1[sr ^ cl] * b2[sr ^ cr] * b2[sl ^ cl];
+          const D z = dir ? b2[sr ^ cr] * b2[sl ^ cl] : b1[sr ^ cl] * b2[sr ^ cr] * b2[sl ^ cl];
           zu[k * 16 + q * 4 + s] = z * u * f;
         }
       }
@@ -953,26 +963,26 @@ double chain_tab(bool zb, int dir, const AuxCoef& c, const AuxCoef* dc, bool nor
   for (int k = 0; k < S; ++k)
     for (int s = 0; s < S; ++s) {
       double sum = 0.0;
-      for (int q = 0; q < S; ++q) sum += w1[s * S + q].v;
-      for (int a = 0; a < S; ++a) gb = std::max(gb, zu[k * S * S + (zb ? a * S + s : s * S + a)].v * sum);
+      for (int q = 0; q < S; ++q) sum += value(w1[s * S + q]);
+      for (int a = 0; a < S; ++a) gb = std::max(gb, value(zu[k * S * S + (zb ? a * S + s : s * S + a)]) * sum);
     }
   // What rounding the tables adds to a step, as the ratio of its exact to its
   // rounded sum over all inputs and outputs: every step shares it, so the
   // product's output factor takes it out (FP32: 3e-8 per entry, L of them).
-  const Dual g(norm ? 1.0 / gb : 1.0);
+  const D g(norm ? 1.0 / gb : 1.0);
   if (std::is_same<T, float>::value && bias) {
-    const float r1 = (float)rho1.v;
+    const float r1 = (float)value(rho1);
     double exact = 0.0, rounded = 0.0;
     for (int k = 0; k < S; ++k)
       for (int s = 0; s < S; ++s) {
         double se = 0.0, sr = 0.0;
         for (int q = 0; q < S; ++q) {
-          se += w1[s * S + q].v;
+          se += value(w1[s * S + q]);
           sr += !zb ? (s == q ? 1.0 : (double)r1)
-                    : ((s >> 1) == (q >> 1) ? 1.0 : (double)r1) * ((q & 1) ? (double)(float)rho2[s].v : 1.0);
+                    : ((s >> 1) == (q >> 1) ? 1.0 : (double)r1) * ((q & 1) ? (double)(float)value(rho2[s]) : 1.0);
         }
         for (int a = 0; a < S; ++a) {
-          const double z = zu[k * S * S + (zb ? a * S + s : s * S + a)].v * g.v;
+          const double z = value(zu[k * S * S + (zb ? a * S + s : s * S + a)]) * value(g);
           exact += z * se;
           rounded += (double)(float)z * sr;
         }
@@ -1001,6 +1011,11 @@ void build_aux(Op& op) {
   if (zb && L % 2) fail(TM_ERR_ARG, "diagonal BNNNI operators need an even width");
   if (reduced) build_prefix_tree(op, L, std::vector<int>(zb ? L / 2 : L, zb ? 2 : 1), true, op.tree);
   if (g_batch_member) return;
+  if (!reduced) {  // one buffer, written in place
+    const int nlb = zb ? 4 : (op.boundary == 0 ? 2 : 1);
+    op.ws_a.alloc((size_t)8 * nlb << (L + (zb ? 2 : 1)));
+    return;
+  }
   // the two pass buffers of any plan the tuning table can choose
   int64_t most[2] = {1, 1};
   for (size_t elem : {(size_t)4, (size_t)8})
@@ -1011,7 +1026,7 @@ void build_aux(Op& op) {
     }
   op.ws_a.alloc((size_t)most[0]);
   op.ws_b.alloc((size_t)most[1]);
-  if (reduced) op.ws_c.alloc((size_t)op.n * 8);
+  op.ws_c.alloc((size_t)op.n * 8);
 }
 
 // ------------------------------------------------------------------ autotuner inputs

@@ -137,7 +137,10 @@ void build_prefix_tree(const Op& op, int nbits, const std::vector<int>& steps, b
   if (T.b[nlev] != nbits) fail(TM_ERR_ARG, "prefix tree: steps do not cover the state");
   const int64_t nblk = (n + kTreeBlock - 1) / kTreeBlock;
   DBuf cnt;  // counts per level and block, then the totals per level
-  cnt.alloc((size_t)(nlev + 1) * (nblk + 1) * 4);
+  {
+    AllocStream pool(s);  // (freed in stream order: a cudaFree would wait for the device)
+    cnt.alloc((size_t)(nlev + 1) * (nblk + 1) * 4);
+  }
   uint32_t* tot = cnt.as<uint32_t>() + (size_t)(nlev + 1) * nblk;
   tree_count_kernel<<<(unsigned)nblk, kTreeBlock, 0, s>>>(op.idx.as<uint32_t>(), n, T, cnt.as<uint32_t>());
   TM_CKK("tree_count");
@@ -161,8 +164,6 @@ void build_prefix_tree(const Op& op, int nbits, const std::vector<int>& steps, b
   tree_fill_kernel<<<(unsigned)nblk, kTreeBlock, 0, s>>>(op.idx.as<uint32_t>(), n, T, cnt.as<uint32_t>());
   TM_CKK("tree_fill");
   out.nlev = nlev;  // (last: a tree whose tables could not be built is no tree)
-  // the counts are released on return: in stream order, or by a synchronising
-  // cudaFree outside an allocation scope
 }
 
 }  // namespace ltm

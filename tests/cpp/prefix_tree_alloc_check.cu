@@ -12,6 +12,8 @@ static int g_left = 0;
 void fail(tm_status code, const std::string& msg) { throw Failure{code, msg}; }
 void check_cuda(cudaError_t, const char*, const char*, int) {}
 void note_launch() {}
+AllocStream::AllocStream(cudaStream_t) : prev(nullptr) {}
+AllocStream::~AllocStream() {}
 void DBuf::alloc(size_t b) {
   release();
   if (g_left-- <= 0) fail(TM_ERR_NOMEM, "out of device memory");
