@@ -46,16 +46,28 @@ constexpr int kMaxTileBits = 12;  // 4096 doubles = 32 KB per tile
 // wait until all pairs are done (it is e^{K (L - 2 popc(low ^ high))} then):
 //   out(p) = e1[j] (a(p) + rho_j a(p^1)), rho_j = e1[j^1] e2[1] / e1[j],
 // two FMAs per element and pair where the 4 x 4 matrix takes four.
+//   The L pairs grow the values by up to ((1 + e2) (1 + rho_j))^L before the
+// output factor brings them back.  Where that comes near the end of the FP64
+// range, a ratio above one is turned round, a(p^1) + a(p) / rho_j, and its power
+// goes into the factor of the output state (e2 likewise: a(p) / e2 = in(p) +
+// in(p^2) / e2), so that a pair grows them by four at most.  TURN: bit 0 for e2,
+// bits 1 and 2 for rho_0 and rho_1.  The turned form of rho_1 alone takes 0.93
+// ms at L = 12, the plain one 0.84.
 struct PairCoef {
-  double e2;      // e2[0]
+  double e2;
   double rho[2];
 };
+template <int TURN>
 __device__ __forceinline__ void pair_step(double (&v)[4], const PairCoef& c) {
   double a[4];
 #pragma unroll
-  for (int p = 0; p < 4; ++p) a[p] = fma(c.e2, v[p], v[p ^ 2]);
+  for (int p = 0; p < 4; ++p) a[p] = fma(c.e2, (TURN & 1) ? v[p ^ 2] : v[p], (TURN & 1) ? v[p] : v[p ^ 2]);
 #pragma unroll
-  for (int p = 0; p < 4; ++p) v[p] = fma(c.rho[(p & 1) ^ (p >> 1)], a[p ^ 1], a[p]);
+  for (int p = 0; p < 4; ++p) {
+    const int j = (p & 1) ^ (p >> 1);
+    const bool turned = (TURN >> (j + 1)) & 1;
+    v[p] = fma(c.rho[j], turned ? a[p] : a[p ^ 1], turned ? a[p ^ 1] : a[p]);
+  }
 }
 
 struct PairTab {
@@ -66,6 +78,7 @@ struct PairTab {
 // bits.  Tile index: chunk bits, then the low sites, then the high sites.
 // pre / post_sc: per-state input / output weights (first / last pass).
 // Bound by the FP64 pipe.
+template <int TURN>
 __global__ void __launch_bounds__(512) pair_kernel(const double* x, double* y, int L, int lo, int np, int cb,
                                                    PairCoef c, const double* __restrict__ pre,
                                                    const double* __restrict__ post_sc, PairTab tab) {
@@ -97,7 +110,7 @@ __global__ void __launch_bounds__(512) pair_kernel(const double* x, double* y, i
       int e = ((q >> ba) << (ba + 1)) | (q & (o1 - 1));
       e = ((e >> bb) << (bb + 1)) | (e & (o2 - 1));
       double v[4] = {sm[spad(e)], sm[spad(e | o1)], sm[spad(e | o2)], sm[spad(e | o1 | o2)]};
-      pair_step(v, c);
+      pair_step<TURN>(v, c);
       sm[spad(e)] = v[0];
       sm[spad(e | o1)] = v[1];
       sm[spad(e | o2)] = v[2];
@@ -287,13 +300,25 @@ void matvec_two_layer(const Op& op, const double* x, double* y, cudaStream_t s) 
     kron_swap_product(b, x, y, b.ws_a.as<double>(), tr, s);
   } else if (b.kind == K_Y2AT) {
     // bzwj1 = e^{+-K}, bzwj2 = e^{-+2K kappa} (TMat/tmat.cpp:247-253)
-    const double r1 = std::exp(-2.0 * bj), e21 = std::exp(2.0 * bj * k);  // e1[1] / e1[0], e2[1]
+    // ln e2[0], ln rho_0, ln rho_1
+    const double le2 = -2.0 * bj * k, lr[2] = {-2.0 * bj - le2, 2.0 * bj - le2};
     PairCoef c;
-    c.e2 = std::exp(-2.0 * bj * k);
-    c.rho[0] = r1 * e21;
-    c.rho[1] = e21 / r1;
+    const double growth = L * (std::log1p(std::exp(le2)) + std::log1p(std::exp(std::max(lr[0], lr[1]))));
+    const int turn = growth < 300.0 ? 0 : (le2 > 0.0 ? 1 : 0) | (lr[0] > 0.0 ? 2 : 0) | (lr[1] > 0.0 ? 4 : 0);
+    double lt[3] = {le2, lr[0], lr[1]};  // ln of what was turned round
+    for (int i = 0; i < 3; ++i)
+      if (!((turn >> i) & 1)) lt[i] = 0.0;
+    c.e2 = std::exp(turn & 1 ? -le2 : le2);
+    for (int j = 0; j < 2; ++j) c.rho[j] = std::exp(((turn >> (j + 1)) & 1) ? -lr[j] : lr[j]);
+    decltype(&pair_kernel<0>) const kernels[8] = {pair_kernel<0>, pair_kernel<1>, pair_kernel<2>, pair_kernel<3>,
+                                                  pair_kernel<4>, pair_kernel<5>, pair_kernel<6>, pair_kernel<7>};
     PairTab tab{};
-    for (int q = 0; q <= L; ++q) tab.d[q] = b.normfactor * std::exp(bj * (L - 2.0 * q));
+    for (int q = 0; q <= L; ++q) {
+      const double ln = bj * (L - 2.0 * q) + L * lt[0] + (L - q) * lt[1] + q * lt[2];
+      // (the factor alone may overflow where a tiny normfactor brings it back)
+      tab.d[q] = ln < 700.0 ? b.normfactor * std::exp(ln)
+                            : (b.normfactor > 0.0 ? std::exp(ln + std::log(b.normfactor)) : 0.0);
+    }
     const double* tv = b.tvec.as<double>();
     int lo = 0;
     const double* src = x;
@@ -303,7 +328,7 @@ void matvec_two_layer(const Op& op, const double* x, double* y, cudaStream_t s) 
       const int tile = 1 << (cb + 2 * np);
       const size_t shm = (size_t)(tile + tile / 32 + 1) * sizeof(double);
       const bool last = (lo + np >= L);
-      pair_kernel<<<(unsigned)(1u << (2 * L - cb - 2 * np)), std::min(512, std::max(32, tile / 4)), shm, s>>>(
+      kernels[turn]<<<(unsigned)(1u << (2 * L - cb - 2 * np)), std::min(512, std::max(32, tile / 4)), shm, s>>>(
           src, y, L, lo, np, cb, c, lo == 0 ? tv : nullptr, last ? tv : nullptr, tab);
       TM_CKK("two_layer_pairs");
       src = y;
