@@ -221,7 +221,7 @@ __device__ __forceinline__ void bnnni_step(T (&v)[4][4], const ChainTab<T>& tab,
 template <class T>
 struct ChainSh {
   ChainTab<T> tab;
-  T two[64];  // first pass: zu[c][s', a'] w1[s'][lb] of the second step, [c][s'][a']
+  T two[64];  // first pass: zu[c][s', a'] w2[s'][lb] of the second step, [c][s'][a']
 };
 struct ChainShDF {
   ChainTab<dfloat> tab;
@@ -485,12 +485,18 @@ __device__ __forceinline__ void chain_first_two(unsigned char* sm, int plane, co
       }
 #pragma unroll
       for (int a = 0; a < S; ++a) to_elem(io.u[at[a]], x[a]);
+    } else if (io.smap) {
+      uint32_t at[S];
+#pragma unroll
+      for (int a = 0; a < S; ++a)
+        at[a] = io.smap[((uint64_t)lb << (L - KS)) | ((uint64_t)a << (L - 2 * KS)) | below];
+#pragma unroll
+      for (int a = 0; a < S; ++a) weigh_in(io.x[at[a]], io.pre[at[a]], x[a]);
     } else {
 #pragma unroll
       for (int a = 0; a < S; ++a) {
         const uint64_t r = ((uint64_t)lb << (L - KS)) | ((uint64_t)a << (L - 2 * KS)) | below;
-        const uint64_t at = io.smap ? io.smap[r] : r;
-        weigh_in(io.x[at], io.pre[at], x[a]);
+        weigh_in(io.x[r], io.pre[r], x[a]);
       }
     }
     // (a ring of two letters: the bottom letter is the second, the third the first)
@@ -511,7 +517,7 @@ __device__ __forceinline__ void chain_first_two(unsigned char* sm, int plane, co
 #pragma unroll
         for (int a = 0; a < S; ++a) {
           if (cp.last)
-            o[a] = sh.tab.zu[c * S * S + (KS == 1 ? s1 * S + a : a * S + s1)] * (sh.tab.w1[s1 * S + lb] * xa[a]);
+            o[a] = sh.tab.zu[c * S * S + (KS == 1 ? s1 * S + a : a * S + s1)] * (sh.tab.w2[s1 * S + lb] * xa[a]);
           else
             o[a] = sh.two[c * S * S + s1 * S + a] * xa[a];
         }
@@ -603,7 +609,7 @@ __device__ __forceinline__ void chain_block(const ChainIO<T, IO>& io, ChainShare
     if (!cp.last)
       for (int k = threadIdx.x; k < S * S * S; k += blockDim.x) {
         const int c = k / (S * S), s1 = (k / S) % S, a = k % S;
-        sh.two[k] = sh.tab.zu[c * S * S + (KS == 1 ? s1 * S + a : a * S + s1)] * sh.tab.w1[s1 * S + lb_outer];
+        sh.two[k] = sh.tab.zu[c * S * S + (KS == 1 ? s1 * S + a : a * S + s1)] * sh.tab.w2[s1 * S + lb_outer];
       }
     __syncthreads();
     chain_first_two<T, KS, IO>(sm, plane, io, sh, cp, L, lb_outer, low0, allowed);
@@ -904,18 +910,31 @@ T tab_elem(Dual x) {
   return tangent(x.v, x.d);
 }
 
+// A bound on ln of the operator's Tvec entries (aux_tvec_grad's terms, with the
+// normfactor that the BNNNI and reduced forms hold) and of the factors that an
+// open boundary adds at both ends.
+double weight_bound(const Op& op) {
+  const bool zb = (op.kind == K_ZBT || op.kind == K_ZBM);
+  const double aK = std::fabs(op.mp.betaJ);
+  double b = 0.5 * aK * (op.L + 1) * (1.0 + std::fabs(op.mp.h) + (zb ? std::fabs(op.mp.kappa2) : 0.0));
+  if (op.kind != K_XDT) b += 0.5 * op.mp.betaJ * op.nfexp;
+  if (!zb && op.boundary) b += 2.0 * aK * std::fabs(op.mp.kappa);
+  return b;
+}
+
 // The step tables (see ChainTab) from the factors b1 = e^{+-K}, b2 =
 // e^{-+K kappa}, b3 = e^{-+K kappa2} (TMat/tmat.cpp:344-376, 521-588) and
 // their derivatives; returns the largest row sum of a step, whose inverse
-// normalises the FP32 and double-float steps.  The ring is walked from the
+// normalises the FP32 and double-float steps.  lnmax: ln of the largest input
+// weight (up: 1 / the power of two in w1, see ChainTab).  The ring is walked from the
 // top, so the carried letter q is the neighbour above and the control c the
 // one below: the reference's factors of the lower neighbour (dir 0: b1[sr^al]
 // b2[sr^ar] b2[sl^al]; dir 1: b2[sr^ar] b2[sl^al]) belong to c, those of the
 // upper one (dir 0: b2[sr^fr] b2[sl^fl]; dir 1: b1[sl^fr] b2[sr^fr]
 // b2[sl^fl]) to q.
 template <class T>
-double chain_tab(bool zb, int dir, const AuxCoef& c, const AuxCoef* dc, bool norm, ChainTab<T>& tab,
-                 double* bias = nullptr) {
+double chain_tab(bool zb, int dir, const AuxCoef& c, const AuxCoef* dc, bool norm, ChainTab<T>& tab, double lnmax,
+                 double* up, double* bias = nullptr) {
   // (formed for every product: plain values but for tangent pairs)
   using D = typename std::conditional<std::is_same<T, tangent>::value, Dual, double>::type;
   D b1[2], b2[2], b3[2];
@@ -989,10 +1008,20 @@ double chain_tab(bool zb, int dir, const AuxCoef& c, const AuxCoef* dc, bool nor
       }
     *bias = exact / rounded;
   }
+  // (e^80 of e^88.7: vectors of unit norm leave room)
+  double top = 0.0;
+  for (int s = 0; zb && s < 4; ++s) top = std::max(top, value(rho2[s]));
+  const double grow = std::log((1.0 + value(rho1)) * (1.0 + top));
+  const double over = std::min(grow, lnmax + grow - 80.0);
+  const int k = (norm && over > 0.0) ? (int)std::ceil(std::min(over, 80.0) / std::log(2.0)) : 0;
+  *up = std::ldexp(1.0, k);
   tab.rho1 = tab_elem<T>(rho1);
   for (int k = 0; k < 4; ++k) tab.rho2[k] = tab_elem<T>(rho2[k]);
   for (int k = 0; k < 2; ++k) tab.b2[k] = tab_elem<T>(b2[k]);
-  for (int k = 0; k < 16; ++k) tab.w1[k] = tab_elem<T>(w1[k]);
+  for (int k = 0; k < 16; ++k) {
+    tab.w1[k] = tab_elem<T>(w1[k] * D(1.0 / *up));
+    tab.w2[k] = tab_elem<T>(w1[k]);
+  }
   for (int k = 0; k < 64; ++k) tab.zu[k] = tab_elem<T>(zu[k] * g);
   return gb;
 }
@@ -1151,10 +1180,10 @@ double matvec_aux_dir(const Op& op, const IO* x, IO* y, bool scaled, int dir, cu
   // (FP32 exponent range)
   const bool norm = !std::is_same<T, double>::value;
   ChainTab<T> tab;
-  double bias = 1.0;
-  const double gb = chain_tab<T>(zb, dir, coef_of(op), dcoef, norm, tab, &bias);
+  double bias = 1.0, up = 1.0;
+  const double gb = chain_tab<T>(zb, dir, coef_of(op), dcoef, norm, tab, weight_bound(op), &up, &bias);
   const int nsteps = zb ? L / 2 : L;
-  const double gscale = norm ? std::pow(gb, (double)nsteps) : 1.0;
+  const double gscale = norm ? std::pow(gb, (double)nsteps) * up : 1.0;
   const double sf = (scaled ? 1.0 : gscale) * std::pow(bias, (double)nsteps);
   const int bc = zb ? 0 : op.boundary;
   int tile_bits = 0, threads = 0;
@@ -1213,12 +1242,13 @@ void chain_inst_fill(const Op& op, int dir, ChainInst& rec, int tb4, int tb8) {
   // full DNNI applies the normfactor at the output; the BNNNI Tvec holds it
   rec.nf = (reduced || zb) ? 1.0 : op.normfactor;
   const AuxCoef c = coef_of(op);
-  double bias = 1.0;
-  const double gb = chain_tab<float>(zb, dir, c, nullptr, true, rec.c32, &bias);
-  chain_tab<dfloat>(zb, dir, c, nullptr, true, rec.cdf);
-  chain_tab<double>(zb, dir, c, nullptr, false, rec.c64);
+  double bias = 1.0, up = 1.0, none = 1.0;
+  const double lnmax = weight_bound(op);
+  const double gb = chain_tab<float>(zb, dir, c, nullptr, true, rec.c32, lnmax, &up, &bias);
+  chain_tab<dfloat>(zb, dir, c, nullptr, true, rec.cdf, lnmax, &up);
+  chain_tab<double>(zb, dir, c, nullptr, false, rec.c64, lnmax, &none);
   const int nsteps = zb ? L / 2 : L;
-  rec.gsdf = std::pow(gb, (double)nsteps);
+  rec.gsdf = std::pow(gb, (double)nsteps) * up;
   rec.gs32 = rec.gsdf * std::pow(bias, (double)nsteps);
   rec.gs64 = 1.0;
   int th = 0;
@@ -1231,7 +1261,7 @@ void chain_inst_fill(const Op& op, int dir, ChainInst& rec, int tb4, int tb8) {
   std::copy(p16.begin(), p16.end(), rec.p16);
   for (int t = 0; t < 3; ++t) {
     const AuxCoef db = aux_coef_derivative(op.mp.betaJ, op.mp.kappa, op.mp.kappa2, t);
-    chain_tab<tangent>(zb, dir, c, &db, true, rec.ctan[t]);  // the normalisation is a constant: no derivative
+    chain_tab<tangent>(zb, dir, c, &db, true, rec.ctan[t], lnmax, &up);  // the normalisation is a constant: no derivative
   }
   rec.tree = tree_dev(op);
   rec.kind = op.kind;

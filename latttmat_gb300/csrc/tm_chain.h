@@ -26,12 +26,17 @@ struct AuxCoef {
 //          d(sl, sr) = t(sl, 0) + rho2[s'] t(sl, 1)
 // zu: DNNI [c][s'][a'], BNNNI [c][a'][s'].  w1[s'][q]: the same sum's
 // coefficients, for the first step (one q only).  b2: open-boundary factors.
+//   The sums can exceed the values they are formed from (rho > 1) before zu
+// brings them back.  Where the weights come so near the end of the FP32
+// exponent range that a sum could leave it while its values do not, w1 holds a
+// negative power of two that the product's output factor undoes.  w2: the
+// coefficients without it, where two steps are applied at once.
 template <class T>
 struct ChainTab {
   T rho1;
   T rho2[4];
   T b2[2];
-  T w1[16];
+  T w1[16], w2[16];
   T zu[64];
 };
 
