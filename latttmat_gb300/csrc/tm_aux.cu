@@ -499,15 +499,13 @@ __device__ __forceinline__ void chain_first_two(unsigned char* sm, int plane, co
         weigh_in(io.x[r], io.pre[r], x[a]);
       }
     }
-    // (a ring of two letters: the bottom letter is the second, the third the first)
-    const bool two = L == 2 * KS;
-    const int c = two ? lb : (int)(below >> (L - 3 * KS)) & (S - 1);
+    const int c = (int)(below >> (L - 3 * KS)) & (S - 1);  // (three letters at least: the caller)
     for (int s0 = split ? item >> fb : 0; s0 < (split ? (item >> fb) + 1 : S); ++s0) {
       if (!((allowed >> (s0 * S)) & ((1u << S) - 1u))) continue;
       T xa[S];
 #pragma unroll
       for (int a = 0; a < S; ++a) {
-        const int q = two ? a : (int)below & (S - 1);
+        const int q = (int)below & (S - 1);
         xa[a] = sh.tab.zu[a * S * S + (KS == 1 ? s0 * S + lb : lb * S + s0)] * (sh.tab.w1[s0 * S + q] * x[a]);
       }
 #pragma unroll
