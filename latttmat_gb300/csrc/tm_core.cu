@@ -23,6 +23,7 @@
 
 #include "tm_bfly.cuh"
 #include "tm_internal.h"
+#include "tm_power.h"
 
 namespace ltm {
 
@@ -560,13 +561,8 @@ void build_bfly(Op& op) {
 // takes 0.39 ms, its copies included.
 int64_t kron_power(const Op& op, const double* x, DBuf& part, cudaStream_t s) {
   const int L = op.L;
-  const double c2 = 2.0 * std::cosh(op.mp.betaJ), s2 = 2.0 * std::sinh(op.mp.betaJ);
-  auto dlam = [&](int k) {  // (s^(L-k) d^k)' with s' = d, d' = s
-    double r = 0.0;
-    if (k < L) r += (L - k) * std::pow(c2, L - k - 1) * std::pow(s2, k + 1);
-    if (k > 0) r += k * std::pow(c2, L - k + 1) * std::pow(s2, k - 1);
-    return r * std::ldexp(1.0, -L);
-  };
+  double dlam[33];
+  power_weights(op.mp.betaJ, L, dlam);
   const double* tv = op.tvec.as<double>();
   const bool reduced = op.kind != K_XAT;
   const bool shifts = (op.kind == K_XAM && op.grp.periodic) || op.kind == K_XAM3;
@@ -586,7 +582,7 @@ int64_t kron_power(const Op& op, const double* x, DBuf& part, cudaStream_t s) {
       if (!o.tree.nlev) build_prefix_tree(op, L, tree_steps(L), false, o.tree);
     }
     const PrefixTree& t = op.tree;
-    for (int k = 0; k <= L; ++k) pw.d[k] = dlam(k);
+    for (int k = 0; k <= L; ++k) pw.d[k] = dlam[k];
     int64_t most[2];
     tree_buffer_elems(op, most);
     a.alloc((size_t)most[0] * 8);
@@ -613,7 +609,7 @@ int64_t kron_power(const Op& op, const double* x, DBuf& part, cudaStream_t s) {
   }
   const bool half = reduced && op.grp.flip;
   const int n = half ? L - 1 : L;
-  for (int k = 0; k <= n; ++k) pw.d[k] = half ? 4.0 * dlam(k + (k & 1)) : dlam(k);
+  for (int k = 0; k <= n; ++k) pw.d[k] = half ? 4.0 * dlam[k + (k & 1)] : dlam[k];
   a.alloc(((size_t)1 << n) * 8);
   int lo = 0;
   const int npass = tile_passes(n, 8);
