@@ -947,7 +947,7 @@ double chain_tab(bool zb, int dir, const AuxCoef& c, const AuxCoef* dc, bool nor
     }
   }
   const int S = zb ? 4 : 2;
-  D rho1 = b2[1] / b2[0], rho2[4] = {}, w1[16] = {}, zu[64] = {};
+  D rho1 = b2[1] / b2[0], rho2[4] = {}, w1[16], zu[64];
   if (!zb) {
     for (int s = 0; s < 2; ++s)
       for (int q = 0; q < 2; ++q) {
@@ -1009,18 +1009,21 @@ double chain_tab(bool zb, int dir, const AuxCoef& c, const AuxCoef* dc, bool nor
   // (e^80 of e^88.7: vectors of unit norm leave room)
   double top = 0.0;
   for (int s = 0; zb && s < 4; ++s) top = std::max(top, value(rho2[s]));
-  const double grow = std::log((1.0 + value(rho1)) * (1.0 + top));
-  const double over = std::min(grow, lnmax + grow - 80.0);
-  const int k = (norm && over > 0.0) ? (int)std::ceil(std::min(over, 80.0) / std::log(2.0)) : 0;
+  const double sums = (1.0 + value(rho1)) * (1.0 + top);
+  int k = 0;
+  if (norm && !(sums < 1e4 && lnmax < 70.0)) {
+    const double grow = std::log(sums), over = std::min(grow, lnmax + grow - 80.0);
+    if (over > 0.0) k = (int)std::ceil(std::min(over, 80.0) / std::log(2.0));
+  }
   *up = std::ldexp(1.0, k);
   tab.rho1 = tab_elem<T>(rho1);
   for (int k = 0; k < 4; ++k) tab.rho2[k] = tab_elem<T>(rho2[k]);
   for (int k = 0; k < 2; ++k) tab.b2[k] = tab_elem<T>(b2[k]);
-  for (int k = 0; k < 16; ++k) {
+  for (int k = 0; k < S * S; ++k) {
     tab.w1[k] = tab_elem<T>(w1[k] * D(1.0 / *up));
     tab.w2[k] = tab_elem<T>(w1[k]);
   }
-  for (int k = 0; k < 64; ++k) tab.zu[k] = tab_elem<T>(zu[k] * g);
+  for (int k = 0; k < S * S * S; ++k) tab.zu[k] = tab_elem<T>(zu[k] * g);
   return gb;
 }
 
@@ -1177,7 +1180,7 @@ double matvec_aux_dir(const Op& op, const IO* x, IO* y, bool scaled, int dir, cu
   // FP32 and double-float steps (tangent pairs included) are normalised
   // (FP32 exponent range)
   const bool norm = !std::is_same<T, double>::value;
-  ChainTab<T> tab;
+  ChainTab<T> tab;  // (DNNI leaves the end of its arrays as it is)
   double bias = 1.0, up = 1.0;
   const double gb = chain_tab<T>(zb, dir, coef_of(op), dcoef, norm, tab, weight_bound(op), &up, &bias);
   const int nsteps = zb ? L / 2 : L;

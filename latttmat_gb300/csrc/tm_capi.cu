@@ -37,8 +37,10 @@ void note_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
 void note_launches(int64_t n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 
 // The attribute belongs to the current device, so the cache is kept per
-// (device, kernel).
+// (device, kernel).  (Below 40 KB the default of 48 KB, static shared memory
+// included, is enough: no look-up in the small calls.)
 void raise_smem_limit(const void* kernel, size_t bytes) {
+  if (bytes <= 40 * 1024) return;
   static std::mutex mu;
   static std::unordered_map<const void*, size_t> cur[64];
   int dev = 0;

@@ -31,7 +31,7 @@ namespace {
 
 template <class T>
 Kron<T> kron_of(const Op& op) {
-  return Kron<T>{(T)std::exp(-2.0 * std::fabs(op.mp.betaJ)), op.mp.betaJ < 0 ? 1 : 0};
+  return Kron<T>{(T)op.kron.r, op.mp.betaJ < 0 ? 1 : 0};
 }
 
 // Weights of the squared Hadamard coefficients by bit count (adjoint), and
@@ -133,10 +133,10 @@ void launch_tile(int64_t nblocks, int threads, size_t shm, cudaStream_t s, const
   TM_CKK("kron_tile");
 }
 
-// The passes of a full-space product.  Up to 9 bits (FP32: 10) go in one pass
-// (one block; a second launch would cost more than its levels: FP32 at L = 10
-// took 8.2 us in two passes), else the bits are spread over ceil(L / 9) (FP64)
-// or ceil(L / 10) passes.  A block takes
+// The passes of a full-space product.  Up to 10 bits (FP32: 11) go in one pass
+// (one block; a second launch costs more than its levels, in time alone and in
+// host time where several operators' products overlap), else the bits are spread
+// over ceil(L / 9) (FP64) or ceil(L / 10) passes.  A block takes
 // up to 16 contiguous positions beside the mixed ones, fewer where that would
 // leave SMs without a block: at small L the FP64 pipe of one SM is the limit
 // (L = 12 in one 4096-element block took 38 us).  Threads: 16 elements each
@@ -148,6 +148,7 @@ struct TilePass {
   int64_t nblocks;
 };
 int tile_passes(int L, size_t elem) {
+  if (L <= (elem == 8 ? 10 : 11)) return 1;
   const int most = (elem == 8) ? 9 : 10;
   return (L + most - 1) / most;
 }
@@ -157,7 +158,7 @@ TilePass tile_pass(int L, int lo, int left, size_t elem) {
   t.nb = (L - lo + left - 1) / left;
   t.cb = std::min(std::min(4, lo), std::max(0, L - t.nb - 7));
   const int tb = t.nb + t.cb;
-  t.kb = (tb >= 11) ? 4 : (tb >= 9 ? 2 : 1);
+  t.kb = (tb >= 11 && t.nb < L) ? 4 : (tb >= 9 ? 2 : 1);  // (a block alone: more threads)
   t.threads = std::min(512, std::max(32, (1 << tb) >> t.kb));
   t.shm = ((size_t)(((1 << t.nb) + (1 << t.nb) / 32) | 1) << t.cb) * elem;
   t.nblocks = (int64_t)1 << (L - tb);
@@ -169,7 +170,10 @@ void run_sweep(const Op& op, const T* x, T* out, int load_mode, const double* pr
   const int L = op.L;
   const Kron<T> c = kron_of<T>(op);
   const int npass = tile_passes(L, sizeof(T));
-  const ScaleF fi = scale_factor(fin), fo = scale_factor(fout);
+  // (FP64 takes the plain factors)
+  const bool f64 = sizeof(T) == 8;
+  const ScaleF fi = f64 ? ScaleF{fin, 1.f, dfloat(0)} : scale_factor(fin);
+  const ScaleF fo = f64 ? ScaleF{fout, 1.f, dfloat(0)} : scale_factor(fout);
   int lo = 0;
   const T* src = x;
   for (int p = 0; p < npass; ++p) {
@@ -347,7 +351,7 @@ __global__ void __launch_bounds__(256) kron_tree_kernel(const T* __restrict__ sr
                                                         const uint2* __restrict__ nodes, int64_t nnode, int rest,
                                                         C c, T* __restrict__ dst,
                                                         const uint16_t* __restrict__ dup,
-                                                        const double* __restrict__ tv, double post,
+                                                        const double* __restrict__ tv, ScaleF post,
                                                         const uint32_t* __restrict__ idx, PowerTab pw) {
   constexpr bool kPower = LAST && std::is_same<C, Had>::value;
   double acc = 0.0;
@@ -370,7 +374,7 @@ __global__ void __launch_bounds__(256) kron_tree_kernel(const T* __restrict__ sr
       for (int j = 0; j < (1 << KB); ++j) v[j] = __ldg(src + at[j]);
       if (tv) {
 #pragma unroll
-        for (int j = 0; j < (1 << KB); ++j) v[j] = (T)((double)v[j] * tv[at[j]] * post);
+        for (int j = 0; j < (1 << KB); ++j) v[j] = weigh(v[j], tv[at[j]], post);
       }
     } else {
       const T* p = src + (node << (rest + KB)) + low;
@@ -385,7 +389,7 @@ __global__ void __launch_bounds__(256) kron_tree_kernel(const T* __restrict__ sr
         if constexpr (kPower)
           acc = fma((double)dup[child] * pw.d[__popc(idx[child])], (double)v[j] * (double)v[j], acc);
         else if constexpr (LAST)
-          dst[child] = (T)((double)v[j] * post * (double)dup[child] * tv[child]);
+          dst[child] = (T)((double)v[j] * post.f64 * (double)dup[child] * tv[child]);
         else
           dst[(child << rest) | low] = v[j];
         ++child;
@@ -401,21 +405,27 @@ int grid_for(int64_t n, int threads = 256) {
   return (int)std::max<int64_t>(1, std::min(b, cap));
 }
 
+// (small levels in blocks of two warps, so that more than a few SMs' FP64 pipes
+// have work)
+int tree_threads(int64_t nnode, int rest) { return (nnode << rest) < (int64_t)num_sms() * 256 ? 64 : 256; }
 int tree_grid(int64_t nnode, int rest) {
-  return (int)std::min<int64_t>(((nnode << rest) + 255) / 256, (int64_t)num_sms() * 64);
+  const int th = tree_threads(nnode, rest);
+  return (int)std::min<int64_t>(((nnode << rest) + th - 1) / th, (int64_t)num_sms() * 64);
 }
 
 template <class T, bool FIRST, bool LAST, class C>
 void launch_tree(int kb, const T* src, const uint32_t* smap, const uint2* nodes, int64_t nnode, int rest, const C& c,
                  T* dst, const uint16_t* dup, const double* tv, double post, cudaStream_t s,
                  const uint32_t* idx = nullptr, const PowerTab* pw = nullptr) {
-  const int grid = tree_grid(nnode, rest);
+  const int grid = tree_grid(nnode, rest), threads = tree_threads(nnode, rest);
   const PowerTab tab = pw ? *pw : PowerTab{};
+  const ScaleF pf = scale_factor(post);
   auto go = [&](auto k) {
-    kron_tree_kernel<T, decltype(k)::value, FIRST, LAST, C><<<grid, 256, 0, s>>>(src, smap, nodes, nnode, rest, c, dst,
-                                                                                 dup, tv, post, idx, tab);
+    kron_tree_kernel<T, decltype(k)::value, FIRST, LAST, C><<<grid, threads, 0, s>>>(src, smap, nodes, nnode, rest, c,
+                                                                                     dst, dup, tv, pf, idx, tab);
   };
   switch (kb) {
+    case 5: go(std::integral_constant<int, 5>()); break;
     case 4: go(std::integral_constant<int, 4>()); break;
     case 3: go(std::integral_constant<int, 3>()); break;
     case 2: go(std::integral_constant<int, 2>()); break;
@@ -498,10 +508,12 @@ __global__ void contract_kernel(const T* __restrict__ z, const uint32_t* __restr
 
 }  // namespace
 
-// four bits per level, the odd ones out in threes at the end
+// Four bits per level, the odd ones out in threes at the end.  Up to 20 bits,
+// where launches are what a product costs, a single bit left over joins the
+// first level (L = 13, 17; all levels of five bits were slower at L = 15 and 20).
 static std::vector<int> tree_steps(int L) {
   std::vector<int> steps;
-  const int nlev = (L + 3) / 4;
+  const int nlev = (L + 3) / 4 - (L <= 20 && L % 4 == 1 ? 1 : 0);
   for (int i = 0, b = 0; i < nlev; ++i) {
     steps.push_back((L - b + nlev - i - 1) / (nlev - i));
     b += steps.back();
@@ -521,6 +533,7 @@ static void tree_buffer_elems(const Op& op, int64_t most[2]) {
 void build_bfly(Op& op) {
   const double K = op.mp.betaJ, aK = std::fabs(K);
   KronConst& kc = op.kron;
+  kc.r = std::exp(-2.0 * aK);
   kc.S = std::pow(std::exp(K) + std::exp(-K), (double)op.L);
   // gin keeps the magnitudes of the unnormalised butterflies those of the
   // normalised factor, (max(a, b) / (a + b))^L = (1 + r)^-L; out undoes it
@@ -671,7 +684,7 @@ double matvec_bfly(const Op& op, const T* x, T* y, bool scaled, cudaStream_t s) 
     TM_CKK("kron_small");
     return ret;
   }
-  const bool fold = op.tree.nlev && op.L <= 16;
+  const bool fold = op.tree.nlev && op.L <= (sizeof(T) == 4 ? 20 : 16);
   T* u = static_cast<T*>(op.ws_c.p);
   if (!fold) {
     scale_in_kernel<T><<<grid_for(op.n), 256, 0, s>>>(x, tv, kc.gin, u, op.n);

@@ -128,6 +128,7 @@ struct PrefixTree {
 
 // Host constants of the Kronecker-core products (set once per operator).
 struct KronConst {
+  double r = 0.0;               // e^{-2|K|}
   double S = 1.0;               // (e^K + e^-K)^L
   double gin = 1.0;             // input factor (1 + r)^-L
   double out64 = 1.0, out32 = 1.0;  // output factors of the FP64 / FP32 butterflies
