@@ -350,9 +350,10 @@ int64_t tm_alloc_count(void);
 
 /* Caps the tile size of the even/odd x-ANNNI passes at 2^bits elements for
  * operators created afterwards (0 removes the cap).  Operators whose tiles
- * exceed the cap split them over thread-block clusters, as those with
- * L >= 30 always do; the cap makes those code paths reachable at small L,
- * for tests.  Results are the same up to rounding. */
+ * exceed the cap split them over thread-block clusters of up to four CTAs
+ * (more are refused at creation, TM_ERR_LIMIT), as 8-byte products do from
+ * L = 26 on and FP32 ones from L = 30; the cap makes those code paths reachable
+ * at small L, for tests.  Results are the same up to rounding. */
 void tm_debug_set_eo_tile_bits(int bits);
 
 /* ---- misc -------------------------------------------------------------- */

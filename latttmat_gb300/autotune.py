@@ -3,8 +3,8 @@
 For each width it builds one operator of the family, times its FP32 and
 double-float products over the candidate tile sizes (2^11..2^14 elements)
 and block sizes (128, 256 threads) with tm_chain_autotune, and prints the
-fastest per width and element size -- the table the library carries as its
-built-in choices (kTunedBNNNI in csrc/tm_aux.cu) -- optionally as JSON.
+fastest per width and element size, optionally as JSON.  They override the
+library's defaults (csrc/tm_tune.cu) until the process ends.
 
   python -m latttmat_gb300.autotune [--model B] [--axialdir 7] [--widths 16 18 20 22 24] [--json out.json]
 """

@@ -161,7 +161,7 @@ int64_t kron_power(const Op& op, const double* x, DBuf& part, cudaStream_t s);
 // the chain C of local step gates built from b1 = e^{+-bJ}, b2 = e^{-+bJ k},
 // b3 = e^{-+bJ k2}.  d ln(lambda) = 2 <g>_{lr} + <l, D_out (dC) D_in r> /
 // (lambda <l, r>); the second term is a tangent product of the chain
-// (matvec_aux_tangent) per parameter the gates depend on.
+// (matvec_aux_tangents) per parameter the gates depend on.
 // (the partial sums of every term come back in one copy)
 void adjoint_grad(const Op& op, const double* qr_h, const double* ql_h, double lam, double grad[4]) {
   const bool aux = (op.kind == K_ZBT || op.kind == K_ZBM || op.kind == K_XDT || op.kind == K_XDM);

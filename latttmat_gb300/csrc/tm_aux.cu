@@ -95,8 +95,7 @@ __device__ __forceinline__ dfloat fold_add(dfloat a, tangent x) { return a + x.d
 // A slot holds the S values of the carried letter.  It is kept as 16-byte (8
 // for DNNI in FP32) vectors, each in a plane of its own: neighbouring slots
 // are then neighbouring vectors, where whole 32-byte slots would use half the
-// banks per access (the first BNNNI pass's shared-memory pipe was 73% busy
-// that way, its FP32 pipe 45%).  Vector i of a plane sits at i + i / 8 (8-byte
+// banks per access.  Vector i of a plane sits at i + i / 8 (8-byte
 // vectors: i + i / 16), one pad per 128 bytes, so that strided letters spread
 // over the banks, and planes are 64 bytes apart modulo 128.  Double-float
 // slots are planar (hi words, then lo words), the order the packed FP32 lanes
@@ -757,10 +756,11 @@ __device__ __forceinline__ void chain_block(const ChainIO<T, IO>& io, ChainShare
 // Measured at the sizes of the sweep and the full operators, against in-place
 // passes of all 2^L states with four multiply-adds and one multiply per
 // output: BNNNI (reduced) at L = 24 in double-float 10.1 -> 1.47 ms, DNNI
-// (full) at L = 26 in FP32 5.18 -> 2.03 ms.  What is left: the FP32 pipes
-// (45% busy in the first double-float pass) and, in FP32, memory (4.3 GB of
-// pass buffers at L = 26, 0.65 ms at the copy rate) behind shared-memory
-// round trips of three letters each.
+// (full) at L = 26 in FP32 5.18 -> 2.04 ms.  No unit is at its peak: the three
+// double-float passes issue in 48, 47 and 42% of all cycles (FP32 pipe 36, 52
+// and 47%, shared memory 52, 47 and 53%, 24% of the warps resident at 124
+// registers), the FP32 ones in 68, 72 and 71% (shared memory 38, 47 and 61%,
+// memory 33, 50 and 28%).
 template <class T>
 constexpr int chain_min_blocks() {
   return sizeof(T) == 4 ? 4 : 2;

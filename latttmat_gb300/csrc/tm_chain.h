@@ -229,7 +229,7 @@ struct BatchMemberScope {
 };
 
 // Measure the operator's product over the chain kernels' tile and block sizes
-// and keep the fastest in the tuning table (tm_aux.cu).
+// and keep the fastest in the tuning table (tm_tune.cu).
 void chain_autotune(const Op& op, tm_dtype dt, int& tile_bits, int& threads, double& ms);
 
 // Operator construction as tm_create does it (throws Failure).

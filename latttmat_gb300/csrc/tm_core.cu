@@ -7,7 +7,7 @@
 // bound by the FP64 pipe (two lanes per clock and SM on sm_103a: every FMA
 // and conversion counts, memory does not), FP32 products by memory.
 //
-// Full operators: shared-memory tile passes of up to 10 bits
+// Full operators: shared-memory tile passes of up to 11 bits
 // (kron_tile_kernel), Tv^(1/2) fused into the first load and nf Tv^(1/2) into
 // the last store.
 //
@@ -342,8 +342,8 @@ __device__ __forceinline__ void tree_bfly(T (&v)[1 << KB], uint32_t mask, const 
 //   LAST:  the children are the representatives: y = post dup tvec value; of
 //          the Hadamard transform (C = Had) the sum over the block's
 //          representatives of dup d[bit count] value^2.
-// Bound by the FP64 pipe in FP64 (78% busy in the first level at L = 25), by
-// the map gather in FP32.  FP64 products against three full-space tile passes
+// Bound by the FP64 pipe in FP64 (busy 81, 78, 72 and 67% in the first four
+// levels at L = 25, 58 to 66% in the short last ones), by the map gather in FP32.  FP64 products against three full-space tile passes
 // with two FP64 operations per element and bit: x-ANNNI at L = 25 without
 // flip 3.17 -> 0.465 ms, the 5x5 layer with flip 3.16 -> 0.142 ms.
 template <class T, int KB, bool FIRST, bool LAST, class C>

@@ -90,7 +90,7 @@ __device__ __forceinline__ dfloat& operator*=(dfloat& a, dfloat b) {
 }
 
 // Double-float values two to a lane pair: hi words in one float2, lo words in
-// another.  df2_fma_unnorm is df_fma_unnorm (tm_df.cuh) on both lanes with the
+// another.  df2_fma_unnorm is df_fma_unnorm on both lanes with the
 // same operation sequence (so the same results), on the packed FP32 pipes;
 // differences are taken as fma(b, -1, a), and -p comes from -r.hi, so no
 // operand needs a separate negation.
@@ -147,8 +147,7 @@ inline ScaleF scale_factor(double S) {
 }
 
 // The FP64 form of scale_round.  Not inlined: as part of the caller it would be
-// predicated, and a predicated FP64 instruction takes its slot on the pipe
-// (73% busy in the first DNNI pass that way).
+// predicated, and a predicated FP64 instruction takes its slot on the pipe.
 static __device__ __noinline__ float scale_round_f64(float vh, float vl, double t, double f) {
   return (float)(((double)vh + (double)vl) * t * f);
 }

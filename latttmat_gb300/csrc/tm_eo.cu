@@ -784,7 +784,7 @@ int grid_for(int64_t n) {
 
 // Cap on the tile bits of the passes for operators created from now on
 // (0: none).  A diagnostic: it lets small operators run the clustered code
-// paths that otherwise only L >= 30 reaches.
+// paths that the 8-byte types reach from L = 26 on and FP32 from L = 30.
 static std::atomic<int> g_eo_tile_bits_cap{0};
 void eo_set_tile_bits_cap(int bits) { g_eo_tile_bits_cap.store(bits < 0 ? 0 : bits); }
 
