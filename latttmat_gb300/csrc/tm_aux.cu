@@ -778,8 +778,10 @@ __global__ void __launch_bounds__(256, chain_min_blocks<T>())
 
 // u = x tvec in the product's arithmetic, for reduced operators above
 // kChainFold bits.  Below, the first pass gathers x and the weight of every
-// state itself: the 2^L gathers more cost less than a launch there.
-constexpr int kChainFold = 14;
+// state itself: the 2^L gathers more cost less than a launch there (with a
+// scaling launch / without, us: DNNI L = 15 FP32 20.5 / 16.4, L = 17 FP64 43.0 /
+// 39.0, BNNNI L = 16 double-float 26.7 / 24.6, L = 18 49.2 / 53.3).
+constexpr int kChainFold = 17;
 template <class U, class IO>
 __global__ void chain_scale_in(const IO* __restrict__ x, const double* __restrict__ tv, U* __restrict__ u, int64_t n) {
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1099,7 +1101,10 @@ void to_f32_dev(const double* x, float* y, int64_t n, cudaStream_t s) {
 // open, L = 12 in FP64: two blocks of 2^11 slots in the last pass): the last
 // pass then hands letters to the others, down to an even split, and the chunks
 // shrink to two slots, until a pass has `blocks` blocks.  The buffers of such
-// operators stay in L2, where short runs cost little.
+// operators stay in L2, where short runs cost little.  With the greedy split /
+// 128 / 256 / 512 blocks, us: full DNNI L = 12 FP64 43.0 / 17.4 / 17.4 / 17.4,
+// L = 17 FP64 - / 57.4 / 51.2 / 50.7, L = 18 FP32 - / 22.5 / 18.5 / 18.5, reduced
+// BNNNI L = 18 FP32 - / 29.7 / 29.9 / 36.9.
 ChainPlan chain_plan(const Op& op, size_t elem, int tile_bits, int blocks) {
   const bool zb = (op.kind == K_ZBT || op.kind == K_ZBM);
   const int KS = zb ? 2 : 1, m = op.L / KS;
